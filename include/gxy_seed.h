@@ -144,7 +144,8 @@ typedef struct {
     uint32_t gapped_pool_blocks;  /* gapped extension: traceback blocks the first pass may use at most
                                      (0 = no limit: sized by the library); sides that do not fit run
                                      again in an exactly sized second pass */
-    uint32_t gapped_cells;        /* gapped extension: cells of a DP row per thread, 4 (the default) or 8 */
+    uint32_t gapped_cells;        /* gapped extension: 4 (the default): chunks of a DP row sized by the band;
+                                     8: chunks of 256 columns, 8 a lane */
 } gxy_tuning;
 gxy_status gxy_ctx_set_tuning(gxy_ctx* ctx, const gxy_tuning* t);
 gxy_status gxy_ctx_get_tuning(gxy_ctx* ctx, gxy_tuning* t);
@@ -418,10 +419,10 @@ typedef struct {
     uint64_t cells;                /* DP cells of all sides (the band's width summed over the rows) */
     double device_ms;              /* CUDA-event time of the DP kernel (last run) */
     uint32_t reruns;               /* first passes repeated after the run buffer had to grow */
-    uint32_t warps_per_side;       /* warps of the block that runs one side (8 cells of a row a thread) */
+    uint32_t warps_per_side;       /* warps that run one side */
     uint64_t max_side_rows;        /* rows of the longest side (sides run in parallel; rows are sequential) */
     uint64_t second_pass_sides;    /* sides run again with exactly sized traceback storage */
-    uint32_t cells_per_thread;     /* cells of a DP row one thread holds (4 or 8) */
+    uint32_t cells_per_thread;     /* gapped_cells of the call (4 or 8) */
     uint32_t pad_;
     uint64_t second_pass_cells;    /* DP cells computed again by the second pass (not in cells) */
 } gxy_gapped_stats;

@@ -276,3 +276,40 @@ def test_gapped_plain_workload_full_size(gxy, ctx):
                                 threads=max(1, min(16, os.cpu_count() or 1)))
     assert [gpu_result(x) for x in got] == [orc_result(x) for x in want]
     assert st["max_side_rows"] > 50_000
+
+
+@pytest.mark.parametrize("go,ge,ydrop,scale", [(400, 30, 9400, 1), (400, 30, 6000, 1), (400, 30, 3000, 1),
+                                               (400, 30, 900, 1), (0, 10, 200, 1), (1200, 90, 28200, 3),
+                                               (6000, 140, 70000, 1)])
+def test_gapped_row_chunks(gxy, ctx, go, ge, ydrop, scale):
+    # A row is worked in chunks of 128, 256 or 512 columns by its band, over as
+    # many as its survivors touch: tandem repeats keep many diagonals alive (rows
+    # of several chunks, bands cut by their cap), insertions and deletions of up
+    # to 330 columns move the cells across chunk edges, and scores of more than
+    # a byte and a y_drop of more than 16 bits take the other forms of a row.
+    rng = np.random.default_rng(4000 + go + ge + ydrop)
+    m = gxy.ScoringMatrix.hoxd70()
+    m.sub = [[scale * x for x in row] for row in m.sub]
+    m.ambig_score *= scale
+    m.gap_open, m.gap_extend = go, ge
+    flat = [x for row in m.sub for x in row]
+    gp = O.gapped_params(go, ge, ydrop, -10 ** 6)
+    for case in range(6):
+        unit = rand_ascii(rng, int(rng.integers(2, 40)), b"ACGT")
+        t = rand_ascii(rng, 500, b"ACGTN", p=[.245, .245, .245, .245, .02]) + unit * (900 // len(unit)) + \
+            rand_ascii(rng, int(rng.integers(300, 1500)), b"ACGT")
+        q = bytearray(_mutate(rng, t, 25))
+        for k in (int(rng.integers(1, 40)), int(rng.integers(100, 330))):
+            at = int(rng.integers(200, len(q) - 400))
+            if rng.random() < 0.5:
+                del q[at:at + k]
+            else:
+                q[at:at] = rand_ascii(rng, k, b"ACGT")
+        q = bytes(q)
+        a = np.stack([rng.integers(0, len(t), 10), rng.integers(0, len(q), 10)], 1)
+        a[:6, 1] = np.minimum(a[:6, 0], len(q) - 1)
+        got = gxy.gapped_extend(gxy.DeviceSeq.from_ascii(t, ctx), gxy.DeviceSeq.from_ascii(q, ctx), a, m,
+                                gxy.GappedParams(ydrop, -10 ** 6), ctx=ctx)
+        want = O.gapped_extend_many(O.pack_ascii(t), O.pack_ascii(q), O.params(sub=flat, ambig=m.ambig_score), gp,
+                                    a[:, 0], a[:, 1], threads=8)
+        assert [gpu_result(x) for x in got] == [orc_result(x) for x in want], case
