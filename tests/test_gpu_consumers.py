@@ -131,3 +131,18 @@ def test_chain_groups_rejects_bad_offsets(gxy, ctx):
         o = np.array(off, np.uint64)
         assert lib().gxy_best_chain_groups(ctx.h, h.ctypes.data, o.ctypes.data, 2, out.ctypes.data,
                                            ln.ctypes.data) != 0
+
+
+@pytest.mark.parametrize("scale", [1, 2_000_000])
+def test_chain_groups_tile_edges(gxy, ctx, scale):
+    # Groups about the tile of 512 HSPs, the warp of 32 and the 8,192 whose parents
+    # sit in shared memory; with the large scores a chain's sum leaves 32 bits.
+    rng = np.random.default_rng(73)
+    groups = [_random_group(rng, gxy, n, max(64, n * 8), ties=i % 2 == 0)
+              for i, n in enumerate([1, 31, 32, 33, 511, 512, 513, 544, 1023, 1025, 8192, 8193])]
+    for g in groups:
+        g["score"] = np.clip(g["score"].astype(np.int64) * scale, -2 ** 31, 2 ** 31 - 1).astype(np.int32)
+    groups.append(np.array([(5, 5, 3, -2 ** 31), (9, 9, 3, -2 ** 31)], gxy.HSP_DTYPE))
+    got = gxy.best_chain_groups(groups, ctx)
+    for g, arr in zip(got, groups):
+        assert g.tobytes() == O.best_chain_c(arr).tobytes(), len(arr)
