@@ -294,6 +294,7 @@ gxy_status gxy_ctx_create(int device, gxy_ctx** out) {
     API_CK(cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &thr));
     prims_init();
     filter_init();
+    epilogue_init();
     table_init();
     gxy_ctx* c = new gxy_ctx();
     c->device = device;

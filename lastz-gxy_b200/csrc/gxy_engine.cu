@@ -483,8 +483,18 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
     // holds runs as several passes, each taking tiles until the buffer is
     // full and handing the tile that did not fit to the next pass, all on
     // the device.
-    double est = 1 << 20;
-    for (const UnitPlan& u : units) est += 1.5 * (double)u.nwin * sa.n_var * u.avg_bucket;
+    double est = 1 << 20, exp_random = 0, exp_windows = 0;
+    for (const UnitPlan& u : units) {
+        exp_random += (double)u.nwin * sa.n_var * u.avg_bucket;
+        exp_windows += (double)u.nwin;
+    }
+    est += 1.5 * exp_random;
+    // What the grids are sized for (every kernel takes any count): raw hits, the
+    // filter's survivors and the candidates, each with a share of the windows for
+    // what is homologous.
+    const uint64_t exp_raw = (uint64_t)(exp_random + exp_windows / 4) + 1;
+    const uint64_t exp_surv = use_filter ? (uint64_t)(exp_random / 16 + exp_windows / 4) + 1 : exp_raw;
+    const uint64_t exp_cands = (uint64_t)(exp_random / 32 + exp_windows / 8) + 1;
     {
         if (use_filter) {
             const uint64_t want_s = (uint64_t)std::min<double>((double)kMaxHitCap, (1 << 20) + est / kRawPerSurvivorSlot);
@@ -503,8 +513,11 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
             W->hit_cap = want_hits;
         }
     }
-    const int blocks_screen = ctx->sm_count * (int)std::max<uint32_t>(1, ctx->tuning.screen_blocks_per_sm);
+    const int screen_per_sm = (int)std::max<uint32_t>(1, ctx->tuning.screen_blocks_per_sm);
+    const int blocks_screen = (int)std::min<uint64_t>((uint64_t)ctx->sm_count * screen_per_sm,
+                                                      exp_surv / (32 * std::max<uint32_t>(1, ctx->tuning.screen_warps)) + 8);
     const int blocks_misc = ctx->sm_count * 4;
+    const int blocks_walk = (int)std::min<uint64_t>((uint64_t)blocks_misc, exp_cands / 32 + 8);
     const int walk_warps = ctx->tuning.walk_warps == 4 ? 4 : 8;
     GXY_CK(W->redo.ensure((size_t)2 * kRedoCap * 4));
 
@@ -523,12 +536,12 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
             sv.hit_cap = W->surv_cap;
             sv.hit_count = survc;
             FilterIO io{sa.hits, hitc, sa.hit_cap, cnt + kCFiltNext};
-            launch_filter_hits(sv, io, ctx->sm_count, st);
+            launch_filter_hits(sv, io, exp_raw, ctx->sm_count, st);
             if (timing) cudaEventRecord(W->ev[3], st);
-            launch_screen(sv, (int)ctx->tuning.screen_warps, blocks_screen, st);
+            launch_screen(sv, (int)ctx->tuning.screen_warps, screen_per_sm, blocks_screen, st);
         } else {
             if (timing) cudaEventRecord(W->ev[3], st);
-            launch_screen(sa, (int)ctx->tuning.screen_warps, blocks_screen, st);
+            launch_screen(sa, (int)ctx->tuning.screen_warps, screen_per_sm, blocks_screen, st);
         }
         if (timing) cudaEventRecord(W->ev[1], st);
     };
@@ -540,11 +553,22 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
     uint32_t* fin_unit = nullptr;
     uint32_t cap = W->cand_cap;
     auto epilogue = [&]() -> gxy_status {
-        const int which = radix_sort_u64(W->ck0.as<uint64_t>(), W->cv0.as<uint32_t>(), W->ck1.as<uint64_t>(),
-                                             W->cv1.as<uint32_t>(), cnt + kCCand, 0, cap, passes, npass, W->ps, st);
-            const uint64_t* skeys = which ? W->ck1.as<uint64_t>() : W->ck0.as<uint64_t>();
-            const uint32_t* sidx = which ? W->cv1.as<uint32_t>() : W->cv0.as<uint32_t>();
-            GXY_CK(cudaMemsetAsync(W->flags.p, 0, cap, st));
+        EpiSort es;
+        es.k0 = W->ck0.as<uint64_t>();
+        es.k1 = W->ck1.as<uint64_t>();
+        es.v0 = W->cv0.as<uint32_t>();
+        es.v1 = W->cv1.as<uint32_t>();
+        es.n_dev = cnt + kCCand;
+        es.n_cap = cap;
+        es.clear = W->flags.as<uint8_t>();
+        std::copy(passes, passes + npass, es.passes);
+        es.npass = npass;
+        es.hist = W->ps.hist;
+        es.bar = cnt + kCBar;
+        GXY_CK(cudaMemsetAsync(cnt + kCWalk, 0, 64, st));   // the walk's cursor and the barriers
+        GXY_CK(launch_sort_candidates(es, exp_cands, ctx->sm_count, st));
+        const uint64_t* skeys = (npass & 1) ? es.k1 : es.k0;
+        const uint32_t* sidx = (npass & 1) ? es.v1 : es.v0;
             WalkArgs wa;
             memset(&wa, 0, sizeof(wa));
             wa.keys = skeys;
@@ -563,29 +587,37 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
             wa.out_hsp = W->ohsp.as<Hsp>();
             wa.chunk_next = cnt + kCWalk;
             wa.n_units = nu;
-            GXY_CK(cudaMemsetAsync(cnt + kCWalk, 0, 4, st));
-            launch_walk(wa, walk_warps, blocks_misc, st);
-            scan_u8(W->flags.as<uint8_t>(), W->offsets.as<uint32_t>(), cnt + kCCand, 0, cap, false, cnt + kCHsps, W->ps,
-                    st);
-            launch_compact(W->flags.as<uint8_t>(), W->offsets.as<uint32_t>(), W->ohsp.as<Hsp>(), sidx,
-                           W->cands.as<Cand>(), cnt + kCCand, cap, W->rhsp.as<Hsp>(), W->runit.as<uint32_t>(), blocks_misc, st);
-            fin = W->rhsp.as<Hsp>();
-            fin_unit = W->runit.as<uint32_t>();
+            launch_walk(wa, walk_warps, blocks_walk, st);
+            EpiFinish ef;
+            memset(&ef, 0, sizeof(ef));
+            ef.flag = W->flags.as<uint8_t>();
+            ef.ohsp = W->ohsp.as<Hsp>();
+            ef.idx = sidx;
+            ef.cands = W->cands.as<Cand>();
+            ef.n_dev = cnt + kCCand;
+            ef.n_cap = cap;
+            ef.n_units = nu;
+            ef.hsp0 = W->rhsp.as<Hsp>();
+            ef.unit0 = W->runit.as<uint32_t>();
+            ef.head = W->flags.as<uint8_t>();
+            ef.n_hsps = cnt + kCHsps;
+            ef.hist = W->ps.hist;
+            ef.bar = cnt + kCBar + 2;
+            fin = ef.hsp0;
+            fin_unit = ef.unit0;
             if (nu > 1) {
-                // Group by unit, keeping each unit's (diagonal, t) order: stable sort.
-                RadixPass up[4];
-                const int nup = plan_radix(0, bits_for(nu - 1), 0, 0, up, 4);
-                launch_iota(W->perm.as<uint32_t>(), cnt + kCHsps, cap, blocks_misc, st);
-                GXY_CK(cudaMemcpyAsync(W->runit2.p, W->runit.p, (size_t)cap * 4, cudaMemcpyDeviceToDevice, st));
-                const int w2 = radix_sort_u32(W->runit2.as<uint32_t>(), W->perm.as<uint32_t>(), W->offsets.as<uint32_t>(),
-                                              W->perm2.as<uint32_t>(), cnt + kCHsps, 0, cap, up, nup, W->ps, st);
-                const uint32_t* perm = w2 ? W->perm2.as<uint32_t>() : W->perm.as<uint32_t>();
-                launch_gather_hsp(W->rhsp.as<Hsp>(), W->runit.as<uint32_t>(), perm, cnt + kCHsps, cap, W->rhsp2.as<Hsp>(),
-                                  W->runit2.as<uint32_t>(), blocks_misc, st);
-                fin = W->rhsp2.as<Hsp>();
-                fin_unit = W->runit2.as<uint32_t>();
+                // Grouped by unit, each unit's (diagonal, t) order kept.
+                ef.npass = plan_radix(0, bits_for(nu - 1), 0, 0, ef.passes, 4);
+                ef.key0 = W->runit2.as<uint32_t>();   // (unit1 as well: the sorted keys are the units)
+                ef.perm0 = W->perm.as<uint32_t>();
+                ef.key1 = W->offsets.as<uint32_t>();
+                ef.perm1 = W->perm2.as<uint32_t>();
+                ef.hsp1 = W->rhsp2.as<Hsp>();
+                ef.unit1 = W->runit2.as<uint32_t>();
+                fin = ef.hsp1;
+                fin_unit = ef.unit1;
             }
-            launch_fixup(fin, fin_unit, cnt + kCHsps, cap, W->flags.as<uint8_t>(), blocks_misc, st);
+            GXY_CK(launch_finish_hsps(ef, exp_cands, ctx->sm_count, st));
             if (records) {
                 // Driver records (src/driver.rs:371-391): stable LSD sort by
                 // (group, global t, q, span) over the unit-major HSP order, then
@@ -709,6 +741,10 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
             }
             const uint32_t np = hc[kCPass];
             const uint64_t tile_at = hc[kCTile], redo_left = hc[kCRedoN + (np & 1u)];
+            if (hc[kCBar + 1] || hc[kCBar + 3]) {
+                set_error("a grid barrier of the epilogue ran out of time");
+                return GXY_ETIMEDOUT;
+            }
             if (hc[kCRedoOver]) {
                 set_error("more tiles than the hit buffer's passes can carry over");
                 return GXY_ENOMEM;

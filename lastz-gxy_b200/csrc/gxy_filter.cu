@@ -273,7 +273,7 @@ __global__ __launch_bounds__(NW * 32, 2) void k_filter_hits(const __grid_constan
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) n_cols += __shfl_xor_sync(kFull, n_cols, o);
-    if (lane == 0) atomicAdd(&a.stats[3], n_cols);
+    if (lane == 0 && n_cols) atomicAdd(&a.stats[3], n_cols);
 }
 
 __global__ void k_occupancy(const uint32_t* __restrict__ starts, uint64_t nw, uint32_t* __restrict__ occ) {
@@ -330,9 +330,13 @@ void filter_init() {
     cudaFuncSetAttribute(k_filter_hits<kFilterWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLutBytes);
 }
 
-void launch_filter_hits(const ScreenArgs& a, const FilterIO& io, int sm_count, cudaStream_t st) {
+void launch_filter_hits(const ScreenArgs& a, const FilterIO& io, uint64_t expected, int sm_count, cudaStream_t st) {
     count_launch();
-    k_filter_hits<kFilterWarps><<<sm_count * 2, kFilterWarps * 32, kLutBytes, st>>>(a, io);
+    // A hit a lane at most: small launches leave the rest of the GPU alone (each
+    // block fills its 64 KB table, each warp claims from the cursor).
+    const uint64_t want = (expected + kFilterWarps * 32 - 1) / (kFilterWarps * 32);
+    const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sm_count * 2));
+    k_filter_hits<kFilterWarps><<<blocks, kFilterWarps * 32, kLutBytes, st>>>(a, io);
 }
 
 void launch_occupancy(const uint32_t* starts, uint64_t num_words, uint32_t* occ, cudaStream_t st) {

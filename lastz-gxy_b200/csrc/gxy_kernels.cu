@@ -342,6 +342,9 @@ __device__ __forceinline__ Hit load_hit(const Hit* p) { return *p; }
 // one transition, else 16.
 template <uint32_t kRegVar>
 __global__ __launch_bounds__(256, 4) void k_enumerate(const __grid_constant__ ScreenArgs a) {
+    __shared__ unsigned long long s_stats[2];   // windows, raw hits
+    if (threadIdx.x < 2) s_stats[threadIdx.x] = 0;
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     const uint32_t ntile = a.tile_hi - a.tile_lo;
     unsigned long long n_windows = 0, n_raw = 0;
@@ -529,10 +532,12 @@ __global__ __launch_bounds__(256, 4) void k_enumerate(const __grid_constant__ Sc
         for (uint32_t tl = next; tl < min(ntile, next + kClaim); tl++) defer(tl, 0);
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) n_windows += __shfl_xor_sync(kFull, n_windows, o);
-    if (lane == 0) {
-        atomicAdd(&a.stats[0], n_windows);
-        atomicAdd(&a.stats[1], n_raw);
-    }
+    // One pair of global atomics a block: every warp's own took longer than the
+    // work of a small launch.
+    if (lane == 0 && n_windows) atomicAdd(&s_stats[0], n_windows);
+    if (lane == 0 && n_raw) atomicAdd(&s_stats[1], n_raw);
+    __syncthreads();
+    if (threadIdx.x < 2 && s_stats[threadIdx.x]) atomicAdd(&a.stats[threadIdx.x], s_stats[threadIdx.x]);
 }
 
 __global__ void k_pass_reset(uint32_t* ctl, uint64_t surv_cap) {
@@ -560,9 +565,12 @@ void launch_pass_reset(uint32_t* ctl, uint64_t surv_cap, cudaStream_t st) {
 
 void launch_enumerate(const ScreenArgs& a, int sm_count, cudaStream_t st) {
     count_launch();
-    if (a.n_var == 1) k_enumerate<1><<<sm_count * 8, 256, 0, st>>>(a);
-    else if (a.n_var == 13) k_enumerate<13><<<sm_count * 8, 256, 0, st>>>(a);
-    else k_enumerate<16><<<sm_count * 8, 256, 0, st>>>(a);
+    // A warp per tile at most: the idle warps of a full grid took 30 us to claim
+    // nothing on a 30 kbp query (938 tiles).
+    const int blocks = (int)std::max<uint64_t>(1, umin64(((uint64_t)(a.tile_hi - a.tile_lo) + 7) / 8, (uint64_t)sm_count * 8));
+    if (a.n_var == 1) k_enumerate<1><<<blocks, 256, 0, st>>>(a);
+    else if (a.n_var == 13) k_enumerate<13><<<blocks, 256, 0, st>>>(a);
+    else k_enumerate<16><<<blocks, 256, 0, st>>>(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -1122,10 +1130,9 @@ static bool packed_ok(const ScreenArgs& a) {
     return a.cap <= 192 && m <= 16383 && a.sc.xdrop >= 0 && a.sc.xdrop <= (1 << 22);
 }
 
-void launch_screen(const ScreenArgs& a, int warps, int blocks, cudaStream_t st) {
-    // blocks = SMs x blocks-per-SM; for 8-warp blocks the register budget
-    // follows the requested blocks per SM (2: 128, 3: 85, 4: 64 registers).
-    const int per_sm = blocks / 148 > 0 ? blocks / 148 : 1;
+void launch_screen(const ScreenArgs& a, int warps, int per_sm, int blocks, cudaStream_t st) {
+    // For 8-warp blocks the register budget follows the requested blocks per SM
+    // (2: 128, 3: 85, 4: 64 registers).
     count_launch();
     if (packed_ok(a)) {
         switch (warps) {
@@ -1340,99 +1347,6 @@ void launch_walk(const WalkArgs& a, int warps, int blocks, cudaStream_t st) {
         case 4: count_launch(); k_walk<4><<<blocks, 128, 0, st>>>(a); break;
         default: count_launch(); k_walk<8><<<blocks, 256, 0, st>>>(a); break;
     }
-}
-
-__global__ void k_compact(const uint8_t* flag, const uint32_t* off, const Hsp* hsp, const uint32_t* idx,
-                          const Cand* cands, const uint32_t* n_dev, uint32_t n_cap, Hsp* out, uint32_t* out_unit) {
-    const uint32_t n = min(*n_dev, n_cap);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (!flag[i]) continue;
-        const uint32_t o = off[i];
-        out[o] = hsp[i];
-        out_unit[o] = cands[idx[i]].unit;
-    }
-}
-
-void launch_compact(const uint8_t* flag, const uint32_t* offsets, const Hsp* hsp, const uint32_t* idx,
-                    const Cand* cands, const uint32_t* n_dev, uint32_t n_cap, Hsp* out, uint32_t* out_unit,
-                    int blocks, cudaStream_t st) {
-    count_launch();
-    k_compact<<<blocks, 256, 0, st>>>(flag, offsets, hsp, idx, cands, n_dev, n_cap, out, out_unit);
-}
-
-__device__ __forceinline__ int64_t diag_of(const Hsp& h) { return (int64_t)h.t_start - (int64_t)h.q_start; }
-__device__ __forceinline__ bool hsp_less(const Hsp& x, const Hsp& y) {
-    if (x.t_start != y.t_start) return x.t_start < y.t_start;
-    if (x.length != y.length) return x.length < y.length;
-    return x.score < y.score;
-}
-
-// Each (unit, diagonal) run arrives in hit order; the canonical order within
-// a run is (t_start, length, score).  Run heads are marked first (from the
-// unmodified array), then one thread per run insertion-sorts it; runs are
-// short and almost always already ordered.
-__global__ void k_mark_runs(const Hsp* hsp, const uint32_t* unit, const uint32_t* n_dev, uint32_t n_cap,
-                            uint8_t* head) {
-    const uint32_t n = min(*n_dev, n_cap);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
-        head[i] = (i == 0 || unit[i - 1] != unit[i] || diag_of(hsp[i - 1]) != diag_of(hsp[i])) ? 1 : 0;
-}
-
-__global__ void k_fixup(Hsp* hsp, const uint8_t* head, const uint32_t* n_dev, uint32_t n_cap) {
-    const uint32_t n = min(*n_dev, n_cap);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        if (!head[i]) continue;
-        uint32_t e = i + 1;
-        bool sorted = true;
-        while (e < n && !head[e]) {
-            if (hsp_less(hsp[e], hsp[e - 1])) sorted = false;
-            e++;
-        }
-        if (sorted) continue;
-        for (uint32_t x = i + 1; x < e; x++) {
-            const Hsp key = hsp[x];
-            uint32_t y = x;
-            while (y > i && hsp_less(key, hsp[y - 1])) {
-                hsp[y] = hsp[y - 1];
-                y--;
-            }
-            hsp[y] = key;
-        }
-    }
-}
-
-void launch_fixup(Hsp* hsp, const uint32_t* unit, const uint32_t* n_dev, uint32_t n_cap, uint8_t* head_scratch,
-                  int blocks, cudaStream_t st) {
-    count_launch();
-    k_mark_runs<<<blocks, 256, 0, st>>>(hsp, unit, n_dev, n_cap, head_scratch);
-    count_launch();
-    k_fixup<<<blocks, 256, 0, st>>>(hsp, head_scratch, n_dev, n_cap);
-}
-
-__global__ void k_gather_hsp(const Hsp* in, const uint32_t* in_unit, const uint32_t* perm, const uint32_t* n_dev,
-                             uint32_t n_cap, Hsp* out, uint32_t* out_unit) {
-    const uint32_t n = min(*n_dev, n_cap);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t p = perm[i];
-        out[i] = in[p];
-        out_unit[i] = in_unit[p];
-    }
-}
-
-void launch_gather_hsp(const Hsp* in, const uint32_t* in_unit, const uint32_t* perm, const uint32_t* n_dev,
-                       uint32_t n_cap, Hsp* out, uint32_t* out_unit, int blocks, cudaStream_t st) {
-    count_launch();
-    k_gather_hsp<<<blocks, 256, 0, st>>>(in, in_unit, perm, n_dev, n_cap, out, out_unit);
-}
-
-__global__ void k_iota(uint32_t* v, const uint32_t* n_dev, uint32_t n_cap) {
-    const uint32_t n = min(*n_dev, n_cap);
-    for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) v[i] = i;
-}
-
-void launch_iota(uint32_t* v, const uint32_t* n_dev, uint32_t n_cap, int blocks, cudaStream_t st) {
-    count_launch();
-    k_iota<<<blocks, 256, 0, st>>>(v, n_dev, n_cap);
 }
 
 // ---------------------------------------------------------------------------

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 
 #include "gxy_device.cuh"
+#include "gxy_prims.cuh"
 
 namespace gxy {
 
@@ -74,14 +75,15 @@ constexpr uint32_t kNoUnit = 0xffffffffu;
 //    candidates, [kCHsps] HSPs, [kCRecs] records, u64 [kCStats] statistics,
 //    [kCRedoN + 0/1] redo-list lengths, u64 [kCMaxFail] largest tile that
 //    did not fit the hit buffer, flags [kCSurvOver] and [kCRedoOver],
-//    [kCWorkPasses] passes that found raw hits, [kCWalk] walk cursor;
+//    [kCWorkPasses] passes that found raw hits, [kCWalk] walk cursor, then the
+//    epilogue's barriers [kCBar + 0, 2, 4] and their error flags [kCBar + 1, 3, 5];
 //  - per pass (reset by k_pass_reset): u64 [kCHits] raw hits, u64 [kCSurv]
 //    survivors, [kCHitNext] screen cursor, [kCFiltNext] filter cursor,
 //    [kCRedoTake] redo-list cursor, [kCStop] the hit buffer is full.
 constexpr uint32_t kCTile = 0, kCHsps = 2, kCRecs = 4, kCStats = 8, kCPass = 128, kCStop = 160, kCRedoN = 192,
                    kCMaxFail = 224, kCSurvOver = 256, kCRedoOver = 288, kCWorkPasses = 320, kCCand = 1024,
                    kCHitNext = 2048, kCRedoTake = 2560, kCHits = 3072, kCSurv = 3328, kCWalk = 3584,
-                   kCFiltNext = 3840;
+                   kCFiltNext = 3840, kCBar = kCWalk + 8;
 constexpr uint32_t kCounterWords = 4096;
 // Tiles a pass can hand to the next one (two lists of this many).
 constexpr uint32_t kRedoCap = 1u << 16;
@@ -132,8 +134,9 @@ void launch_enumerate(const ScreenArgs& a, int sm_count, cudaStream_t st);
 // Starts a pass: flags survivor overflow of the previous pass (its count above
 // surv_cap), advances the pass counter and resets the per-pass counters.
 void launch_pass_reset(uint32_t* ctl, uint64_t surv_cap, cudaStream_t st);
-// Capped lane-per-hit x-drop over a.hits; keeps the candidates.  grid = persistent.
-void launch_screen(const ScreenArgs& a, int warps_per_block, int blocks, cudaStream_t st);
+// Capped lane-per-hit x-drop over a.hits; keeps the candidates.  per_sm: the
+// resident blocks per SM its registers are limited for.
+void launch_screen(const ScreenArgs& a, int warps_per_block, int per_sm, int blocks, cudaStream_t st);
 // The upper-bound x-drop filter between enumeration and the exact screen
 // (gxy_filter.cu).  filter_bounds fills a's fub/f_inv/f_end/f_seed_max from
 // a.sc and a.pat and returns false when the scoring admits no such bound
@@ -148,7 +151,8 @@ struct FilterIO {
     uint64_t raw_cap;
     uint32_t* cursor;      // zeroed by the caller
 };
-void launch_filter_hits(const ScreenArgs& a, const FilterIO& io, int sm_count, cudaStream_t st);
+// expected: raw hits the grid is sized for (the kernel takes any number).
+void launch_filter_hits(const ScreenArgs& a, const FilterIO& io, uint64_t expected, int sm_count, cudaStream_t st);
 // Per-device kernel attributes of the filter (its shared-memory table); call
 // once with the device current, before any stream capture.
 void filter_init();
@@ -179,17 +183,48 @@ struct WalkArgs {
 // one warp per diagonal segment.
 void launch_walk(const WalkArgs& a, int warps_per_block, int blocks, cudaStream_t st);
 
-// Gathers the kept HSPs: out[offsets[i]] = hsp[i], out_unit likewise.
-void launch_compact(const uint8_t* flag, const uint32_t* offsets, const Hsp* hsp, const uint32_t* idx,
-                    const Cand* cands, const uint32_t* n_dev, uint32_t n_cap, Hsp* out, uint32_t* out_unit,
-                    int blocks, cudaStream_t st);
-// Orders each (unit, diagonal) run by (t_start, length, score).
-void launch_fixup(Hsp* hsp, const uint32_t* unit, const uint32_t* n_dev, uint32_t n_cap, uint8_t* head_scratch,
-                  int blocks, cudaStream_t st);
-// Gathers records by a permutation.
-void launch_gather_hsp(const Hsp* in, const uint32_t* in_unit, const uint32_t* perm, const uint32_t* n_dev,
-                       uint32_t n_cap, Hsp* out, uint32_t* out_unit, int blocks, cudaStream_t st);
-void launch_iota(uint32_t* v, const uint32_t* n_dev, uint32_t n_cap, int blocks, cudaStream_t st);
+// The launch's epilogue kernels (gxy_epilogue.cu): cooperative launches that
+// use as many of their blocks as the device-side count needs.  bar: two words,
+// zero before the launch; bar[1] is set when a grid barrier gave up.
+struct EpiSort {
+    uint64_t *k0, *k1;         // keys and values, ping-ponged: the result is in 0 when npass is even
+    uint32_t *v0, *v1;
+    const uint32_t* n_dev;     // count (clamped to n_cap)
+    uint32_t n_cap;
+    uint8_t* clear;            // optional: [0, n) zeroed (the walk's flags)
+    RadixPass passes[16];
+    int npass;
+    uint32_t* hist;            // 256 words per block
+    uint32_t* bar;
+};
+// Stable sort of (key, value) pairs; expected: the count the grid is sized for.
+cudaError_t launch_sort_candidates(const EpiSort& a, uint64_t expected, int sm_count, cudaStream_t st);
+
+struct EpiFinish {
+    const uint8_t* flag;       // the walk's output, per sorted position
+    const Hsp* ohsp;
+    const uint32_t* idx;
+    const Cand* cands;
+    const uint32_t* n_dev;
+    uint32_t n_cap;
+    uint32_t n_units;
+    Hsp* hsp0;                 // the kept HSPs in sorted order (the result for one unit)
+    uint32_t* unit0;
+    uint32_t *key0, *perm0, *key1, *perm1;   // several units: the sort by unit
+    Hsp* hsp1;                 // and its result
+    uint32_t* unit1;
+    RadixPass passes[4];
+    int npass;
+    uint8_t* head;             // scratch, may be `flag`
+    uint32_t* n_hsps;
+    uint32_t* hist;
+    uint32_t* bar;
+};
+// The flagged HSPs, grouped by unit, each (unit, diagonal) run ordered by
+// (t_start, length, score).
+cudaError_t launch_finish_hsps(const EpiFinish& a, uint64_t expected, int sm_count, cudaStream_t st);
+// Kernel attributes of the epilogue; once per device, before any capture.
+void epilogue_init();
 
 // --- driver records (src/driver.rs:371-391, :437-468) --------------------------
 // Where a unit's HSPs go: the output group (the driver's (target, query,

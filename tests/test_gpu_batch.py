@@ -230,3 +230,24 @@ def test_objects_freed_after_their_context(gxy, ctx):
     h = gxy.search(tab2, T, T, gxy.ScoringMatrix.hoxd70(), gxy.SearchParams())
     assert len(h) > 0
     tab2.free()
+
+
+@pytest.mark.parametrize("n_units,lo,hi,thresh", [(1, 3000, 3001, 3000), (2, 20_000, 20_001, 1500), (256, 400, 1200, 2000),
+                                                  (257, 400, 1200, 2000), (700, 1500, 4000, 1500)])
+def test_epilogue_sizes(gxy, ctx, n_units, lo, hi, thresh):
+    # The candidate sort and the HSPs' grouping by unit run in one block up to
+    # 4,096 items and in as many as they need above; units take one digit up to
+    # 256 and two above.  From none to some 20,000 candidates, against the oracle's
+    # search of each unit.
+    rng = np.random.default_rng(900 + n_units)
+    target = rand_ascii(rng, 60_000, b"ACGTACGTacgtN")
+    queries = make_queries(rng, target, n_units, lo, hi)
+    tab = gxy.PosTable.build(gxy.PackedSeq.from_ascii(target), P12, 1, ctx=ctx)
+    dq = [gxy.DeviceSeq.from_ascii(q, ctx) for q in queries]
+    units = [(0, i, i & 1) for i in range(n_units)]
+    sp = gxy.SearchParams(1, gxy.HspParams(910, thresh), 1)
+    got = gxy.batch_search([tab], dq, units, gxy.ScoringMatrix.hoxd70(), sp, ctx=ctx)
+    want = oracle_units(target, queries, units, sp=O.params(hspthresh=thresh))
+    assert n_units == 1 or sum(len(w) for w in want) > 0   # (the single unit finds nothing: an empty sort)
+    for u, (g, w) in enumerate(zip(got, want)):
+        assert g.tobytes() == w.tobytes(), u
