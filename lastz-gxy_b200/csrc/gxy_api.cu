@@ -107,7 +107,7 @@ TableMem::~TableMem() {
     dev_free(starts);
     dev_free(positions);
     dev_free(occ);
-    dev_free(ilv);
+    dev_free(rec);
 }
 
 namespace {
@@ -136,24 +136,22 @@ gxy_status build_tables(gxy_ctx* ctx, const gxy_dseq* seq, uint32_t n, const uin
         set_error(std::string("table allocation: ") + cudaGetErrorString(e));
         return GXY_ENOMEM;
     }
-    // The interleaved copy of the sequence words the views cover (with two
-    // words of margin each side: the filter's windows reach 32 positions
-    // left of a view and one word past its end).
+    // The window records of the sequence words the views cover.
     {
         uint64_t lo_min = UINT64_MAX, hi_max = 0;
         for (uint32_t v = 0; v < n; v++) {
             lo_min = std::min(lo_min, lo[v]);
             hi_max = std::max(hi_max, hi[v]);
         }
-        const uint64_t w0 = (kPad + lo_min) / 32, w1 = (kPad + hi_max) / 32;
-        mem->ilv_first = w0 >= 2 ? w0 - 2 : 0;
-        const uint64_t last = std::min<uint64_t>(seq->nwords - 1, w1 + 2);
-        e = dev_alloc((void**)&mem->ilv, (size_t)(last + 1 - mem->ilv_first) * 16, st);
+        // (One word of margin: the filter's left windows start up to 32 before a view.)
+        mem->rec_first = (kPad + lo_min) / 32 - 1;
+        const uint64_t n_rec = (kPad + hi_max) / 32 + 1 - mem->rec_first;
+        e = dev_alloc((void**)&mem->rec, (size_t)n_rec * 32, st);
         if (e != cudaSuccess) {
             set_error(std::string("table allocation: ") + cudaGetErrorString(e));
             return GXY_ENOMEM;
         }
-        launch_interleave(seq->codes, seq->valid, seq->mask, mem->ilv_first, last + 1 - mem->ilv_first, mem->ilv, st);
+        launch_window_records(seq->codes, seq->valid, mem->rec_first, n_rec, mem->rec, st);
     }
     std::vector<uint32_t> first((size_t)n + 1);
     API_TRY(atomic_build_views(seq, n, lo, hi, pat, step, mem->starts, mem->positions, mem->occ, first.data(), W));

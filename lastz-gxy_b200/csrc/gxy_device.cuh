@@ -33,29 +33,22 @@ struct SeqView {
     uint64_t base;
     uint32_t len;
     uint32_t key_base;
-    // Optional interleaved copy (a table's target): the 32-position word i's
-    // codes, valid and mask bits as one 16-byte record ilv[i - ilv_first], so
-    // that a random 32-position window takes two loads instead of four.
-    const uint4* ilv = nullptr;
-    uint64_t ilv_first = 0;
+    // Optional window records (a table's target): record i - rec_first holds the
+    // codes of the 32-position words i - 1 .. i + 2 in 32 bytes, so that the
+    // surroundings of a position in word i (32 positions before it to 32 after a
+    // seed of up to 32) take one sector.  The last of its 128 positions is never
+    // among them: its two bits are set when any of the 128 is invalid, else clear.
+    const uint32_t* rec = nullptr;
+    uint64_t rec_first = 0;
 };
 
-// Codes and valid bits of the 32 positions from global position gp, from the
-// interleaved copy when the view has one.
+// Codes and valid bits of the 32 positions from global position gp.
 __device__ __forceinline__ void load_window32(const SeqView& S, uint64_t gp, uint64_t& codes, uint32_t& valid) {
     const uint64_t i = gp >> 5;
     const uint32_t s = (uint32_t)(gp & 31);
-    if (S.ilv) {
-        const uint4 a = __ldg(S.ilv + (i - S.ilv_first));
-        const uint4 b = __ldg(S.ilv + (i + 1 - S.ilv_first));
-        const uint64_t lo = ((uint64_t)a.y << 32) | a.x, hi = ((uint64_t)b.y << 32) | b.x;
-        codes = s ? ((lo >> (2 * s)) | (hi << (64 - 2 * s))) : lo;
-        valid = __funnelshift_r(a.z, b.z, s);
-    } else {
-        const uint64_t lo = __ldg(S.codes + i), hi = __ldg(S.codes + i + 1);
-        codes = s ? ((lo >> (2 * s)) | (hi << (64 - 2 * s))) : lo;
-        valid = __funnelshift_r(__ldg(S.valid + i), __ldg(S.valid + i + 1), s);
-    }
+    const uint64_t lo = __ldg(S.codes + i), hi = __ldg(S.codes + i + 1);
+    codes = s ? ((lo >> (2 * s)) | (hi << (64 - 2 * s))) : lo;
+    valid = __funnelshift_r(__ldg(S.valid + i), __ldg(S.valid + i + 1), s);
 }
 
 // One reference search() call: a (target segment, query segment) pair with

@@ -121,9 +121,9 @@ SeqView view_of(const gxy_dseq* s, uint64_t lo, uint64_t hi) {
 
 SeqView table_view(const gxy_table* t) {
     SeqView v = view_of(t->seq, t->lo, t->hi);
-    if (t->mem && t->mem->ilv) {
-        v.ilv = t->mem->ilv;
-        v.ilv_first = t->mem->ilv_first;
+    if (t->mem && t->mem->rec) {
+        v.rec = t->mem->rec;
+        v.rec_first = t->mem->rec_first;
     }
     return v;
 }
@@ -272,7 +272,7 @@ gxy_status reserve_worker(gxy_ctx* ctx, Worker* W, uint64_t est_hits, uint64_t c
         W->surv.release();
         W->surv_cap = want_s;
     }
-    GXY_CK(W->surv.ensure((size_t)W->surv_cap * sizeof(Hit)));
+    GXY_CK(W->surv.ensure((size_t)W->surv_cap * kHitBytes));
     GXY_CK(W->redo.ensure((size_t)2 * kRedoCap * 4));
     const size_t mu = std::max<uint32_t>(max_units, 1);
     GXY_CK(W->d_units.ensure(mu * sizeof(UnitDev)));
@@ -285,7 +285,7 @@ gxy_status reserve_worker(gxy_ctx* ctx, Worker* W, uint64_t est_hits, uint64_t c
     }
     if (candidates > W->cand_cap) W->cand_cap = (uint32_t)candidates;
     const size_t cap = W->cand_cap;
-    GXY_CK(W->hits.ensure((size_t)W->hit_cap * sizeof(Hit)));
+    GXY_CK(W->hits.ensure((size_t)W->hit_cap * kHitBytes));
     DevBuf* by8[] = {&W->ck0, &W->ck1};
     for (DevBuf* b : by8) GXY_CK(b->ensure(cap * 8));
     DevBuf* by4[] = {&W->cv0, &W->cv1, &W->runit, &W->runit2, &W->perm, &W->perm2};
@@ -459,7 +459,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
     // The upper-bound filter runs between enumeration and the exact screen
     // when the scores admit class bounds (every matrix with a class whose
     // scores are all <= 0); otherwise the exact screen takes every raw hit.
-    sa.f_cap = std::max<uint32_t>(32, ctx->tuning.filter_cap);
+    sa.f_cap = std::min<uint32_t>(1u << 29, std::max<uint32_t>(32, ctx->tuning.filter_cap));   // (counted in 30 bits)
     sa.f_claim = ctx->tuning.filter_claim > 1 ? ctx->tuning.filter_claim : 0u;
     const bool use_filter = filter_bounds(sa);
 
@@ -532,7 +532,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
         if (use_filter) {
             // Raw hits -> the bounded filter -> survivors -> the exact screen.
             ScreenArgs sv = sa;
-            sv.hits = W->surv.as<Hit>();
+            sv.hits = W->surv.as<uint32_t>();
             sv.hit_cap = W->surv_cap;
             sv.hit_count = survc;
             FilterIO io{sa.hits, hitc, sa.hit_cap, cnt + kCFiltNext};
@@ -671,8 +671,8 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
     uint32_t rounds = 0;
     for (int attempt = 0; attempt < 16; attempt++) {
         cap = W->cand_cap;
-        GXY_CK(W->hits.ensure((size_t)W->hit_cap * sizeof(Hit)));
-        if (use_filter) GXY_CK(W->surv.ensure((size_t)W->surv_cap * sizeof(Hit)));
+        GXY_CK(W->hits.ensure((size_t)W->hit_cap * kHitBytes));
+        if (use_filter) GXY_CK(W->surv.ensure((size_t)W->surv_cap * kHitBytes));
         GXY_CK(W->ck0.ensure((size_t)cap * 8));
         GXY_CK(W->ck1.ensure((size_t)cap * 8));
         GXY_CK(W->cv0.ensure((size_t)cap * 4));
@@ -698,7 +698,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
         sa.cand_count = cnt + kCCand;
         sa.hit_next = cnt + kCHitNext;
         sa.hit_count = hitc;
-        sa.hits = W->hits.as<Hit>();
+        sa.hits = W->hits.as<uint32_t>();
         sa.hit_cap = W->hit_cap;
         sa.stats = st64;
         sa.cand_keys = W->ck0.as<uint64_t>();

@@ -23,10 +23,11 @@
 //    columns, against five operations per column in the exact screen;
 //  - a hit survives when the bounded seed footprint + both sides' bests reach
 //    hspthresh, or when a side is still running after f_cap columns;
-//  - target windows come from the table's interleaved copy of its target
-//    (two 16-byte loads per 32-position window): the lanes' target positions
-//    are random, and these gathers are what bounds the kernel, while a warp's
-//    query positions come from one tile of windows.
+//  - nearly every hit is decided by the first 32 columns of both sides, so
+//    these are scored for 32 hits at a time from one 32-byte record of the
+//    target (SeqView::rec) and the query's words around the window; the few
+//    hits that run on, or whose columns hold an invalid base or a sequence end,
+//    go through a queue of the warp's own, 32 at a time.
 //
 // Survivors (about 1 % of the raw hits on chromosome-scale inputs) go to a
 // second hit array, where the exact screen (k_screen) takes them.  The
@@ -40,8 +41,10 @@ namespace gxy {
 
 namespace {
 
-constexpr int kLutBytes = 256 * 32 * 8;         // (sum, max prefix) x 32 lane copies
-constexpr int kFilterWarps = 16;                // warps per block, two blocks per SM
+constexpr int kLutBytes = 256 * 32 * 8;         // (sum, max prefix) x 32 lane copies; one table a direction
+constexpr int kFilterWarps = 32;                // warps per block, one block per SM (the tables fill it)
+constexpr uint32_t kQueue = 64;                 // hits a warp's queue holds, eight words each
+constexpr int kFilterSmem = 2 * kLutBytes + kFilterWarps * kQueue * 32;
 
 // Columns whose bit in `keep` is clear take the classes of `pat`.
 __device__ __forceinline__ uint64_t fold_cols(uint64_t x, uint32_t keep, uint64_t pat) {
@@ -65,46 +68,39 @@ __device__ __forceinline__ void f_group(FSide& S, uint32_t w, uint32_t lane8, in
     S.run += e.x;
 }
 
-// 32 columns of two independent sides, interleaved so that the two serial
-// chains issue side by side.
-__device__ __forceinline__ void f_scan2(FSide& A, uint64_t xa, FSide& B, uint64_t xb, uint32_t lane8,
-                                        const unsigned char* lut) {
-    const uint32_t a0 = (uint32_t)xa, a1 = (uint32_t)(xa >> 32);
-    const uint32_t b0 = (uint32_t)xb, b1 = (uint32_t)(xb >> 32);
+// 32 columns of each side, interleaved so that the two serial chains issue
+// side by side.  R runs up from column 0 of (r0, r1); L runs down from column
+// 31 of (l0, l1), through the table of prefix sums taken from a byte's high end.
+__device__ __forceinline__ void f_scan2(FSide& R, uint32_t r0, uint32_t r1, FSide& Lf, uint32_t l0, uint32_t l1,
+                                        uint32_t lane8, const unsigned char* lut) {
 #pragma unroll
     for (int g = 0; g < 4; g++) {
-        f_group(A, a0, lane8, g, lut);
-        f_group(B, b0, lane8, g, lut);
+        f_group(R, r0, lane8, g, lut);
+        f_group(Lf, l1, lane8, 3 - g, lut + kLutBytes);
     }
 #pragma unroll
     for (int g = 0; g < 4; g++) {
-        f_group(A, a1, lane8, g, lut);
-        f_group(B, b1, lane8, g, lut);
+        f_group(R, r1, lane8, g, lut);
+        f_group(Lf, l0, lane8, 3 - g, lut + kLutBytes);
     }
 }
 
 __device__ __forceinline__ void lut_fill(unsigned char* lut, const int32_t* fub) {
-    for (uint32_t i = threadIdx.x; i < 256u * 32u; i += blockDim.x) {
-        const uint32_t b = i >> 5;
+    for (uint32_t i = threadIdx.x; i < 2u * 256u * 32u; i += blockDim.x) {
+        const uint32_t b = (i >> 5) & 255u;
+        const bool down = i >> 13;
         int32_t p = 0, mp = INT32_MIN;
 #pragma unroll
         for (int c = 0; c < 4; c++) {
-            p += fub[(b >> (2 * c)) & 3u];
+            p += fub[(b >> (2 * (down ? 3 - c : c))) & 3u];
             mp = max(mp, p);
         }
         reinterpret_cast<int2*>(lut)[i] = make_int2(p, mp);
     }
 }
 
-// The seed footprint's bound: all L columns at (t, q) (src/hsp.rs:119-123).
-__device__ __forceinline__ int32_t seed_bound(const SeqView& T, const SeqView& Q, uint32_t t, uint32_t q,
-                                              uint32_t L, uint64_t f_inv, int32_t ub0, uint32_t lane8,
-                                              const unsigned char* lut) {
-    const uint64_t tg = T.base + t, qg = Q.base + q;
-    uint64_t tc;
-    uint32_t tv;
-    load_window32(T, tg, tc, tv);
-    const uint64_t x = fold_cols(tc ^ load_codes32(Q.codes, qg), tv & load_bits32(Q.valid, qg), f_inv);
+// The seed footprint's bound: all L columns from column 0 of x (src/hsp.rs:119-123).
+__device__ __forceinline__ int32_t seed_sum(uint64_t x, uint32_t L, int32_t ub0, uint32_t lane8, const unsigned char* lut) {
     int32_t sd = 0;
 #pragma unroll
     for (int g = 0; g < 8; g++) {
@@ -119,13 +115,37 @@ __device__ __forceinline__ int32_t seed_bound(const SeqView& T, const SeqView& Q
     return sd;
 }
 
-// The bounded x-drop over the raw-hit array written by k_enumerate: one lane
-// per hit, hits claimed by the warp in chunks from a global cursor and dealt
-// to its idle lanes (as in k_screen).  A side still running after a chunk
-// continues while the idle lanes take new hits.  Survivors go to a.hits.
-template <int NW>
-__global__ __launch_bounds__(NW * 32, 2) void k_filter_hits(const __grid_constant__ ScreenArgs a,
-                                                             const __grid_constant__ FilterIO io) {
+// 256 bits from a 32-byte boundary.
+__device__ __forceinline__ void load_rec(const uint32_t* p, uint32_t (&w)[8]) {
+    asm("ld.global.nc.v8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+        : "=r"(w[0]), "=r"(w[1]), "=r"(w[2]), "=r"(w[3]), "=r"(w[4]), "=r"(w[5]), "=r"(w[6]), "=r"(w[7])
+        : "l"(p));
+}
+
+// The 96 positions from position s (0 .. 31) of 128: 16 a word.
+__device__ __forceinline__ void align96(const uint32_t (&w)[8], uint32_t s, uint32_t (&o)[6]) {
+    const bool up = s & 16;
+    const uint32_t sh = 2 * (s & 15);
+    uint32_t v[7];
+#pragma unroll
+    for (int i = 0; i < 7; i++) v[i] = up ? w[i + 1] : w[i];
+#pragma unroll
+    for (int i = 0; i < 6; i++) o[i] = __funnelshift_r(v[i], v[i + 1], sh);
+}
+
+// The bounded x-drop over the raw-hit array written by k_enumerate.  Warps
+// claim hits in chunks from a cursor and take 32 at a time, one a lane: both
+// sides' first 32 columns, from which nearly every hit is dropped.  The rest is
+// queued and taken 32 at a time, a further 32 columns a step.  Survivors go to
+// a.hits.
+//
+// What bounds it: the integer pipe and the L1's one tag a cycle.  A form with a
+// persistent hit a lane, a window of its own for each side (two 16-byte records
+// and four query words) and a reversal of the left one took 601 instructions
+// and 6.6 sectors a hit, 0.70 ms for 26.1 M hits (10 Mbp x 10 Mbp); this one
+// 404 and 2.2, 0.48 ms.
+__global__ __launch_bounds__(kFilterWarps * 32, 1) void k_filter_hits(const __grid_constant__ ScreenArgs a,
+                                                                       const __grid_constant__ FilterIO io) {
     extern __shared__ __align__(16) unsigned char smem[];
     unsigned char* lut = smem;
     lut_fill(lut, a.fub);
@@ -134,142 +154,219 @@ __global__ __launch_bounds__(NW * 32, 2) void k_filter_hits(const __grid_constan
     // next pass).
     const uint32_t n_hits = (uint32_t)min(*io.raw_count, (unsigned long long)io.raw_cap);
     const int lane = threadIdx.x & 31;
+    // Word k of queued hit s at k * kQueue + s: t, q, unit, the right run and best,
+    // the left ones, and the columns scanned << 2 | the sides that run (whose columns
+    // scanned are the same number).
+    uint32_t* const queue = reinterpret_cast<uint32_t*>(smem + 2 * kLutBytes) + (threadIdx.x >> 5) * (kQueue * 8);
     const uint32_t lane8 = (uint32_t)lane * 8u, lt = lanemask_lt();
     const uint32_t L = a.pat.len;
     const int32_t X = a.sc.xdrop, thresh = a.sc.hspthresh;
     const int32_t need = thresh - a.f_seed_max;
     const int32_t ub0 = a.fub[0];
-    const uint32_t n_warps = gridDim.x * NW;
-    const uint32_t chunk = a.f_claim ? a.f_claim : max(32u, min(512u, n_hits / max(1u, n_warps * 8u)));
-    uint32_t wcur = 0, wend = 0;
+    const uint32_t n_warps = gridDim.x * kFilterWarps;
+    const uint32_t chunk = a.f_claim ? a.f_claim : max(32u, min(512u, n_hits / max(1u, n_warps * 8u)) & ~31u);
+    uint32_t wcur = 0, wend = 0, qn = 0;
     bool exhausted = false;
     unsigned long long n_cols = 0;
-
-    bool busy = false, ralive = false, lalive = false;
-    uint32_t ht = 0, hq = 0, hu = 0xffffffffu, cur_unit = 0xffffffffu;
-    uint32_t rext = 0, lext = 0, rrem = 0, lrem = 0;
-    int32_t rrun = 0, rbest = 0, lrun = 0, lbest = 0;
-    SeqView T{}, Q{};
+    uint32_t cur_unit = kNoUnit;
+    // The current unit's target records and query.
+    const uint32_t* rec = nullptr;
+    uint64_t t_base = 0, q_base = 0;   // t_base counts from the first record
+    uint32_t t_len = 0, q_len = 0;
+    const uint64_t* qc = nullptr;
+    const uint32_t* qv = nullptr;
+    auto take_unit = [&](uint32_t u) {
+        cur_unit = u;
+        const UnitDev U = a.units[u];
+        const SeqView& T = a.tsegs[U.tseg];
+        const SeqView& Q = a.qsegs[U.qseg];
+        rec = T.rec;
+        t_base = T.base - 32 * T.rec_first;
+        t_len = T.len;
+        qc = Q.codes;
+        qv = Q.valid;
+        q_base = Q.base;
+        q_len = Q.len;
+    };
+    auto emit = [&](bool surv, uint32_t t, uint32_t q, uint32_t u) {
+        const uint32_t sm = __ballot_sync(kFull, surv);
+        if (!sm) return;
+        unsigned long long base = 0;
+        if (lane == 0) base = atomicAdd(a.hit_count, (unsigned long long)__popc(sm));
+        base = __shfl_sync(kFull, base, 0);
+        const unsigned long long slot = base + __popc(sm & lt);
+        if (surv && slot < a.hit_cap) {
+            a.hits[slot] = t;
+            a.hits[a.hit_cap + slot] = q;
+            a.hits[2 * a.hit_cap + slot] = u;
+        }
+    };
+    auto enqueue = [&](bool on, uint32_t t, uint32_t q, uint32_t u, const FSide& R, const FSide& Lf, uint32_t state) {
+        const uint32_t m = __ballot_sync(kFull, on);
+        if (on) {
+            uint32_t* e = queue + qn + __popc(m & lt);
+            e[0] = t;
+            e[kQueue] = q;
+            e[2 * kQueue] = u;
+            e[3 * kQueue] = (uint32_t)R.run;
+            e[4 * kQueue] = (uint32_t)R.best;
+            e[5 * kQueue] = (uint32_t)Lf.run;
+            e[6 * kQueue] = (uint32_t)Lf.best;
+            e[7 * kQueue] = state;
+        }
+        qn += __popc(m);
+        __syncwarp();
+    };
     for (;;) {
-        const uint32_t im = __ballot_sync(kFull, !busy);
-        const uint32_t need_n = __popc(im);
-        const uint32_t avail = wend - wcur;
-        uint32_t nb = 0, ncount = 0;
-        if (need_n > avail && !exhausted) {
+        if (wcur == wend && !exhausted) {
+            uint32_t nb = 0;
             if (lane == 0) nb = atomicAdd(io.cursor, chunk);
             nb = __shfl_sync(kFull, nb, 0);
-            ncount = nb < n_hits ? min(chunk, n_hits - nb) : 0u;
-            if (nb + chunk >= n_hits) exhausted = true;
+            wcur = min(nb, n_hits);
+            wend = min(nb + chunk, n_hits);
+            exhausted = nb + chunk >= n_hits;
         }
-        if (!busy) {
-            const uint32_t rk = __popc(im & lt);
-            uint32_t hidx = 0xffffffffu;
-            if (rk < avail) hidx = wcur + rk;
-            else if (rk - avail < ncount) hidx = nb + (rk - avail);
-            if (hidx != 0xffffffffu) {
-                const Hit h = io.raw[hidx];
-                ht = h.t;
-                hq = h.q;
-                hu = h.unit;
-                if (hu != kNoUnit && hu != cur_unit) {
-                    cur_unit = hu;
-                    const UnitDev U = a.units[hu];
-                    T = a.tsegs[U.tseg];
-                    Q = a.qsegs[U.qseg];
-                }
-                busy = hu != kNoUnit;   // else an unused slot of a failed reservation
-                if (busy) {
-                    rrem = min(T.len - ht - L, Q.len - hq - L);
-                    lrem = min(ht, hq);
-                    rrun = rbest = lrun = lbest = 0;
-                    rext = lext = 0;
-                    ralive = rrem > 0;
-                    lalive = lrem > 0;
-                }
+        if (qn < 32 && wcur < wend) {
+            // ---- 32 new hits: both sides' first 32 columns.
+            const uint32_t idx = wcur + lane;
+            wcur = min(wcur + 32, wend);
+            uint32_t t = 0, q = 0, u = kNoUnit;
+            if (idx < wend) {
+                t = __ldg(io.raw + idx);
+                q = __ldg(io.raw + io.raw_cap + idx);
+                u = __ldg(io.raw + 2 * io.raw_cap + idx);
             }
-        }
-        {
-            const uint32_t from_old = min(need_n, avail);
-            if (ncount) {
-                wcur = nb + min(need_n - from_old, ncount);
-                wend = nb + ncount;
-            } else {
-                wcur += from_old;
+            const bool on = u != kNoUnit;   // else an unused slot of a failed reservation
+            if (on && u != cur_unit) take_unit(u);
+            const uint32_t rrem = on ? min(t_len - t - L, q_len - q - L) : 0u, lrem = on ? min(t, q) : 0u;
+            bool plain = on && rec && rrem >= 32 && lrem >= 32;
+            uint32_t x[6] = {0, 0, 0, 0, 0, 0};
+            if (plain) {
+                const uint64_t gt = t_base + t, gq = q_base + q;
+                uint32_t w[8], o[6];
+                load_rec(rec + (gt >> 5) * 8, w);
+                const uint64_t* c = qc + (gq >> 5) - 1;
+                const uint32_t* v = qv + (gq >> 5) - 1;
+                uint32_t y[8];
+#pragma unroll
+                for (int k = 0; k < 4; k++) {
+                    const uint64_t z = __ldg(c + k);
+                    y[2 * k] = (uint32_t)z;
+                    y[2 * k + 1] = (uint32_t)(z >> 32);
+                }
+                const uint32_t ok = __ldg(v) & __ldg(v + 1) & __ldg(v + 2) & __ldg(v + 3);
+                plain = ok == kFull && !(w[7] >> 31);
+                align96(w, (uint32_t)gt & 31, x);
+                align96(y, (uint32_t)gq & 31, o);
+#pragma unroll
+                for (int k = 0; k < 6; k++) x[k] ^= o[k];
             }
-        }
-        if (!__any_sync(kFull, busy)) {
-            if (exhausted && wcur == wend) break;
+            // Classes: the 32 columns left of the seed in x[0..1], 32 from its start
+            // in x[2..3], the next 32 in x[4..5]; the right side starts L further.
+            const uint32_t s = 2 * (L & 15);
+            const uint32_t a0 = L >= 32 ? x[4] : (L >= 16 ? x[3] : x[2]), a1 = L >= 32 ? x[5] : (L >= 16 ? x[4] : x[3]),
+                           a2 = L >= 16 ? x[5] : x[4];
+            FSide R{0, 0}, Lf{0, 0};
+            f_scan2(R, __funnelshift_r(a0, a1, s), __funnelshift_r(a1, a2, s), Lf, x[0], x[1], lane8, lut);
+            const bool ra = plain && rrem > 32 && R.best - R.run <= X, la = plain && lrem > 32 && Lf.best - Lf.run <= X;
+            bool surv = plain && !ra && !la && R.best + Lf.best >= need;
+            if (__any_sync(kFull, surv)) {
+                if (surv)
+                    surv = seed_sum(((uint64_t)x[3] << 32) | x[2], L, ub0, lane8, lut) + R.best + Lf.best >= thresh;
+                emit(surv, t, q, u);
+            }
+            if (plain) n_cols += 64;
+            if (on && !plain) R = Lf = FSide{0, 0};
+            const bool more = ra || la || (on && !plain);
+            if (__any_sync(kFull, more))
+                enqueue(more, t, q, u, R, Lf,
+                        plain ? (32u << 2) | (ra ? 1u : 0u) | (la ? 2u : 0u) : (rrem ? 1u : 0u) | (lrem ? 2u : 0u));
             continue;
         }
-        const uint32_t nr = ralive ? min(32u, rrem) : 0u, nl = lalive ? min(32u, lrem) : 0u;
+        if (qn == 0) {
+            if (exhausted) break;
+            continue;
+        }
+        // ---- up to 32 queued hits: 32 more columns of each side that runs.
+        const uint32_t take = min(qn, 32u);
+        qn -= take;
+        const bool on = (uint32_t)lane < take;
+        uint32_t t = 0, q = 0, u = kNoUnit, state = 0;
+        FSide R{0, 0}, Lf{0, 0};
+        if (on) {
+            const uint32_t* e = queue + qn + lane;
+            t = e[0];
+            q = e[kQueue];
+            u = e[2 * kQueue];
+            R.run = (int32_t)e[3 * kQueue];
+            R.best = (int32_t)e[4 * kQueue];
+            Lf.run = (int32_t)e[5 * kQueue];
+            Lf.best = (int32_t)e[6 * kQueue];
+            state = e[7 * kQueue];
+            if (u != cur_unit) take_unit(u);
+        }
+        __syncwarp();
+        const uint32_t ext = state >> 2;
+        const uint32_t rrem = on ? min(t_len - t - L, q_len - q - L) - ext : 0u, lrem = on ? min(t, q) - ext : 0u;
+        const uint32_t nr = (state & 1u) ? min(32u, rrem) : 0u, nl = (state & 2u) ? min(32u, lrem) : 0u;
+        // The classes of the 32 columns from target position tp and query position
+        // qp (tp may lie up to 32 before the view); n columns count, from the low
+        // end or (top) the high one.
+        auto classes = [&](int64_t tp, int64_t qp, uint32_t n, bool top) {
+            const uint64_t gq = (uint64_t)((int64_t)q_base + qp);
+            uint64_t tcod, qcod;
+            uint32_t ok, w[8];
+            qcod = load_codes32(qc, gq);
+            ok = load_bits32(qv, gq);
+            bool exact = true;   // the record tells that all is valid
+            if (rec) {
+                const uint64_t gt = (uint64_t)((int64_t)t_base + tp);
+                load_rec(rec + (gt >> 5) * 8, w);
+                const bool up = gt & 16;
+                const uint32_t sh = 2 * ((uint32_t)gt & 15);
+                const uint32_t v0 = up ? w[3] : w[2], v1 = up ? w[4] : w[3], v2 = up ? w[5] : w[4];
+                tcod = ((uint64_t)__funnelshift_r(v1, v2, sh) << 32) | __funnelshift_r(v0, v1, sh);
+                exact = !(w[7] >> 31);
+            }
+            if (!rec || !exact) {
+                const SeqView& T = a.tsegs[a.units[u].tseg];
+                uint32_t tv;
+                load_window32(T, (uint64_t)((int64_t)T.base + tp), tcod, tv);
+                ok &= tv;
+            }
+            uint64_t x = tcod ^ qcod;
+            if (n < 32 || ok != kFull)
+                x = fold_cols(fold_cols(x, ok, a.f_inv), n >= 32 ? kFull : (top ? kFull << (32 - n) : (1u << n) - 1u), a.f_end);
+            return x;
+        };
         uint64_t xr = 0, xl = 0;
-        uint32_t vr = kFull, vl = kFull;
-        if (nr) {
-            const uint64_t tg = T.base + ht + L + rext, qg = Q.base + hq + L + rext;
-            uint64_t tc;
-            uint32_t tv;
-            load_window32(T, tg, tc, tv);
-            xr = tc ^ load_codes32(Q.codes, qg);
-            vr = tv & load_bits32(Q.valid, qg);
-        }
-        if (nl) {
-            const uint64_t tg = T.base + ht - lext - 32, qg = Q.base + hq - lext - 32;
-            uint64_t tc;
-            uint32_t tv;
-            load_window32(T, tg, tc, tv);
-            xl = rev_pairs64(tc ^ load_codes32(Q.codes, qg));
-            vl = __brev(tv & load_bits32(Q.valid, qg));
-        }
-        const bool slow = (nr && (nr < 32 || vr != kFull)) || (nl && (nl < 32 || vl != kFull));
-        if (__any_sync(kFull, slow)) {
-            const uint32_t er = nr >= 32 ? kFull : ((1u << nr) - 1u);
-            const uint32_t el = nl >= 32 ? kFull : ((1u << nl) - 1u);
-            xr = fold_cols(fold_cols(xr, vr, a.f_inv), er, a.f_end);
-            xl = fold_cols(fold_cols(xl, vl, a.f_inv), el, a.f_end);
-        }
-        FSide R{rrun, rbest}, Lf{lrun, lbest};
-        f_scan2(R, xr, Lf, xl, lane8, lut);
+        if (nr) xr = classes((int64_t)t + L + ext, (int64_t)q + L + ext, nr, false);
+        if (nl) xl = classes((int64_t)t - ext - 32, (int64_t)q - ext - 32, nl, true);
+        const FSide R0 = R, L0 = Lf;
+        f_scan2(R, (uint32_t)xr, (uint32_t)(xr >> 32), Lf, (uint32_t)xl, (uint32_t)(xl >> 32), lane8, lut);
         n_cols += nr + nl;
+        bool ra = false, la = false;
         if (nr) {
-            rrun = R.run;
-            rbest = R.best;
-            rext += nr;
-            rrem -= nr;
-            ralive = rrem > 0 && rbest - rrun <= X;
+            ra = rrem > nr && R.best - R.run <= X;
+        } else {
+            R = R0;
         }
         if (nl) {
-            lrun = Lf.run;
-            lbest = Lf.best;
-            lext += nl;
-            lrem -= nl;
-            lalive = lrem > 0 && lbest - lrun <= X;
+            la = lrem > nl && Lf.best - Lf.run <= X;
+        } else {
+            Lf = L0;
         }
-        const bool capped = busy && ((ralive && rext >= a.f_cap) || (lalive && lext >= a.f_cap));
-        const bool done = busy && (capped || (!ralive && !lalive));
-        bool surv = done && (capped || rbest + lbest >= need);
+        const bool capped = on && (ra || la) && ext + 32 >= a.f_cap;
+        const bool done = on && (capped || (!ra && !la));
+        bool surv = done && (capped || R.best + Lf.best >= need);
         if (__any_sync(kFull, surv && !capped)) {
-            if (surv && !capped) surv = seed_bound(T, Q, ht, hq, L, a.f_inv, ub0, lane8, lut) + rbest + lbest >= thresh;
-        }
-        const uint32_t sm = __ballot_sync(kFull, surv);
-        if (sm) {
-            unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(a.hit_count, (unsigned long long)__popc(sm));
-            base = __shfl_sync(kFull, base, 0);
-            if (surv) {
-                const unsigned long long slot = base + __popc(sm & lt);
-                if (slot < a.hit_cap) {
-                    Hit h;
-                    h.t = ht;
-                    h.q = hq;
-                    h.unit = hu;
-                    a.hits[slot] = h;
-                }
+            if (surv && !capped) {
+                surv = seed_sum(classes(t, q, 32, false), L, ub0, lane8, lut) + R.best + Lf.best >= thresh;
             }
         }
-        if (done) {
-            busy = false;
-            ralive = lalive = false;
-        }
+        emit(surv, t, q, u);
+        if (__any_sync(kFull, on && !done))
+            enqueue(on && !done, t, q, u, R, Lf, (ext + 32) << 2 | (ra ? 1u : 0u) | (la ? 2u : 0u));
     }
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) n_cols += __shfl_xor_sync(kFull, n_cols, o);
@@ -327,16 +424,16 @@ bool filter_bounds(ScreenArgs& a) {
 }
 
 void filter_init() {
-    cudaFuncSetAttribute(k_filter_hits<kFilterWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, kLutBytes);
+    cudaFuncSetAttribute(k_filter_hits, cudaFuncAttributeMaxDynamicSharedMemorySize, kFilterSmem);
 }
 
 void launch_filter_hits(const ScreenArgs& a, const FilterIO& io, uint64_t expected, int sm_count, cudaStream_t st) {
     count_launch();
     // A hit a lane at most: small launches leave the rest of the GPU alone (each
-    // block fills its 64 KB table, each warp claims from the cursor).
+    // block fills its two 64 KB tables, each warp claims from the cursor).
     const uint64_t want = (expected + kFilterWarps * 32 - 1) / (kFilterWarps * 32);
-    const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sm_count * 2));
-    k_filter_hits<kFilterWarps><<<blocks, kFilterWarps * 32, kLutBytes, st>>>(a, io);
+    const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sm_count));
+    k_filter_hits<<<blocks, kFilterWarps * 32, kFilterSmem, st>>>(a, io);
 }
 
 void launch_occupancy(const uint32_t* starts, uint64_t num_words, uint32_t* occ, cudaStream_t st) {

@@ -330,12 +330,11 @@ __device__ __forceinline__ void scan_pair_any(SideScan& A, SideScan& B, uint32_t
 // variant's bucket (src/pos_table.rs:102-108).  Large buckets are copied by
 // the whole warp.
 // ---------------------------------------------------------------------------
-__device__ __forceinline__ void store_hit(Hit* p, uint32_t t, uint32_t q, uint32_t u) {
-    p->t = t;
-    p->q = q;
-    p->unit = u;
+__device__ __forceinline__ void store_hit(const ScreenArgs& a, uint64_t i, uint32_t t, uint32_t q, uint32_t u) {
+    a.hits[i] = t;
+    a.hits[a.hit_cap + i] = q;
+    a.hits[2 * a.hit_cap + i] = u;
 }
-__device__ __forceinline__ Hit load_hit(const Hit* p) { return *p; }
 
 // kRegVar: variants whose bucket bounds stay in registers between the two
 // passes (the rest are re-read): 1 without transitions, 13 for weight 12 with
@@ -475,7 +474,7 @@ __global__ __launch_bounds__(256, 4) void k_enumerate(const __grid_constant__ Sc
             // part of its reservation inside the buffer is marked unused.
             if (lane == 0) defer(tl, wtot);
             for (uint64_t j = base + lane; j < min((unsigned long long)a.hit_cap, base + wtot); j += 32)
-                a.hits[j].unit = kNoUnit;
+                a.hits[2 * a.hit_cap + j] = kNoUnit;
             continue;
         }
         n_windows += wv ? 1 : 0;
@@ -492,7 +491,7 @@ __global__ __launch_bounds__(256, 4) void k_enumerate(const __grid_constant__ Sc
 #pragma unroll
             for (uint32_t i = 0; i < 8; i++)
                 if (v0 + i < kRegVar && rc[v0 + i] != 0 && rc[v0 + i] <= 16)
-                    store_hit(a.hits + dst++, first[i], q, u);
+                    store_hit(a, dst++, first[i], q, u);
         }
         for (uint32_t v = 0; v < a.n_var; v++) {
             uint32_t b = 0, c = 0;
@@ -512,7 +511,7 @@ __global__ __launch_bounds__(256, 4) void k_enumerate(const __grid_constant__ Sc
             // Small buckets of the first kRegVar variants wrote their first position above.
             const uint32_t j0 = (v < kRegVar && !big) ? 1u : 0u;
             if (!big) {
-                for (uint32_t j = j0; j < c; j++) store_hit(a.hits + dst++, __ldg(U.positions + b + j), q, u);
+                for (uint32_t j = j0; j < c; j++) store_hit(a, dst++, __ldg(U.positions + b + j), q, u);
             }
             uint32_t bm = __ballot_sync(kFull, big);
             while (bm) {
@@ -521,7 +520,7 @@ __global__ __launch_bounds__(256, 4) void k_enumerate(const __grid_constant__ Sc
                 const uint32_t bb = __shfl_sync(kFull, b, src), cc = __shfl_sync(kFull, c, src);
                 const uint32_t qq = __shfl_sync(kFull, q, src);
                 const uint64_t dd = __shfl_sync(kFull, dst, src);
-                for (uint32_t j = lane; j < cc; j += 32) store_hit(a.hits + dd + j, __ldg(U.positions + bb + j), qq, u);
+                for (uint32_t j = lane; j < cc; j += 32) store_hit(a, dd + j, __ldg(U.positions + bb + j), qq, u);
             }
             if (big) dst += c;
         }
@@ -626,10 +625,9 @@ __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen_wide(const __grid_c
         if (!busy) {
             const uint32_t rk = __popc(im & lt);
             if (rk < take) {
-                const Hit h = load_hit(a.hits + base + rk);
-                ht = h.t;
-                hq = h.q;
-                hu = h.unit;
+                ht = a.hits[base + rk];
+                hq = a.hits[a.hit_cap + base + rk];
+                hu = a.hits[2 * a.hit_cap + base + rk];
                 if (hu != kNoUnit && hu != cur_unit) {
                     cur_unit = hu;
                     const UnitDev U = a.units[hu];
@@ -975,10 +973,9 @@ __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen(const __grid_consta
             if (rk < avail) hidx = wcur + rk;
             else if (rk - avail < ncount) hidx = nb + (rk - avail);
             if (hidx != 0xffffffffu) {
-                const Hit h = load_hit(a.hits + hidx);
-                ht = h.t;
-                hq = h.q;
-                hu = h.unit;
+                ht = a.hits[hidx];
+                hq = a.hits[a.hit_cap + hidx];
+                hu = a.hits[2 * a.hit_cap + hidx];
                 if (hu != kNoUnit && hu != cur_unit) {
                     cur_unit = hu;
                     const UnitDev U = a.units[hu];

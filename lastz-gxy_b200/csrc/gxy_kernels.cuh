@@ -59,13 +59,10 @@ void launch_prune_copy(const uint32_t* positions, const uint32_t* starts, uint64
                        const uint32_t* new_starts, uint32_t limit, uint32_t* new_positions, cudaStream_t st);
 
 // --- search ------------------------------------------------------------------
-// A raw seed hit: target position t, query window q, unit.  unit kNoUnit
+// Seed hits: target position t, query window q, unit, in three arrays of the
+// buffer's capacity (hits[i], hits[cap + i], hits[2 cap + i]).  unit kNoUnit
 // marks a slot of a hit-buffer reservation that failed (skipped by readers).
-struct Hit {
-    uint32_t t;
-    uint32_t q;
-    uint32_t unit;
-};
+constexpr size_t kHitBytes = 12;
 constexpr uint32_t kNoUnit = 0xffffffffu;
 
 // Layout of a worker's device counters (u32 indices).  The ones every warp
@@ -103,7 +100,7 @@ struct ScreenArgs {
     Score sc;
     uint32_t cap;          // columns per side before a hit is deferred
     uint32_t qkey_total;   // size of the query key axis
-    Hit* hits;             // raw hits of this pass
+    uint32_t* hits;        // raw hits of this pass
     uint64_t hit_cap;
     unsigned long long* hit_count;   // hits enumerated (may exceed hit_cap: then the pass is redone smaller)
     uint32_t* hit_next;    // x-drop work counter
@@ -146,7 +143,7 @@ bool filter_bounds(ScreenArgs& a);
 // io.raw[0, *io.raw_count) (nothing when that count exceeds io.raw_cap) and
 // writes the survivors to a.hits / a.hit_count / a.hit_cap.
 struct FilterIO {
-    const Hit* raw;
+    const uint32_t* raw;
     const unsigned long long* raw_count;
     uint64_t raw_cap;
     uint32_t* cursor;      // zeroed by the caller

@@ -220,12 +220,17 @@ __global__ void k_view_firsts(const uint32_t* __restrict__ starts, uint64_t nw, 
     for (uint32_t v = threadIdx.x; v <= n_views; v += blockDim.x) first[v] = starts[(uint64_t)v * nw];
 }
 
-// ilv[j] = word first + j's codes (low, high half), valid and mask bits.
-__global__ void k_interleave(const uint64_t* __restrict__ codes, const uint32_t* __restrict__ valid,
-                             const uint32_t* __restrict__ mask, uint64_t first, uint64_t n, uint4* __restrict__ ilv) {
+// rec[8 j ..]: the codes of words first + j - 1 .. first + j + 2; the last
+// position's two bits set when any of the 128 positions is invalid, else clear.
+__global__ void k_window_records(const uint64_t* __restrict__ codes, const uint32_t* __restrict__ valid, uint64_t first,
+                                 uint64_t n, uint4* __restrict__ rec) {
     for (uint64_t j = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; j < n; j += (uint64_t)gridDim.x * blockDim.x) {
-        const uint64_t c = codes[first + j];
-        ilv[j] = make_uint4((uint32_t)c, (uint32_t)(c >> 32), valid[first + j], mask[first + j]);
+        const uint64_t w = first + j - 1;
+        const uint64_t a = codes[w], b = codes[w + 1], c = codes[w + 2], d = codes[w + 3];
+        const bool ok = (valid[w] & valid[w + 1] & valid[w + 2] & valid[w + 3]) == 0xffffffffu;
+        rec[2 * j] = make_uint4((uint32_t)a, (uint32_t)(a >> 32), (uint32_t)b, (uint32_t)(b >> 32));
+        rec[2 * j + 1] = make_uint4((uint32_t)c, (uint32_t)(c >> 32), (uint32_t)d,
+                                    ((uint32_t)(d >> 32) & 0x3fffffffu) | (ok ? 0u : 0xc0000000u));
     }
 }
 
@@ -233,11 +238,12 @@ __global__ void k_interleave(const uint64_t* __restrict__ codes, const uint32_t*
 
 void table_init() {}
 
-void launch_interleave(const uint64_t* codes, const uint32_t* valid, const uint32_t* mask, uint64_t first, uint64_t n,
-                       uint4* ilv, cudaStream_t st) {
+void launch_window_records(const uint64_t* codes, const uint32_t* valid, uint64_t first, uint64_t n, uint32_t* rec,
+                           cudaStream_t st) {
     if (!n) return;
     count_launch();
-    k_interleave<<<(int)std::min<uint64_t>((n + 255) / 256, 148 * 16), 256, 0, st>>>(codes, valid, mask, first, n, ilv);
+    k_window_records<<<(int)std::min<uint64_t>((n + 255) / 256, 148 * 16), 256, 0, st>>>(codes, valid, first, n,
+                                                                                         reinterpret_cast<uint4*>(rec));
 }
 
 gxy_status atomic_build_views(const gxy_dseq* seq, uint32_t n_views, const uint64_t* lo, const uint64_t* hi,

@@ -475,3 +475,26 @@ def test_filter_bounds_cases(gxy, ctx, case):
     g, o = both(gxy, ctx, t, q, P12, sp, matrix=m)
     assert g == o
     assert len(o) > 0
+
+
+@pytest.mark.parametrize("pattern", ["1" * 11, "111011011101111", "1110110111011110" + "1", "11" * 6 + "0001",
+                                     "1" + "0" * 20 + "1" * 10 + "1", "1010100010010001" * 2])
+@pytest.mark.parametrize("n", [63, 65, 97, 200])
+def test_filter_windows(gxy, ctx, pattern, n):
+    # The filter scores a hit's first 32 columns of both sides from one record when
+    # both sequences reach that far and all is valid, and queues it otherwise: queries
+    # of n bases around that reach, with an N beside every fourth one's middle, cut
+    # from the target's ends and from its inside; patterns of 11 to 32 columns.
+    rng = np.random.default_rng(77 * n + len(pattern))
+    target = rand_ascii(rng, 3 * n, b"ACGT")
+    pieces = [target[:n], target[-n:], target[n + 7:2 * n + 7], target[n - 5:2 * n - 5]]
+    for i, p in enumerate(pieces):
+        q = bytearray(p)
+        for k in rng.integers(0, n, 2):
+            q[k] = b"ACGT"[rng.integers(4)]
+        if i == 3:
+            q[n // 2 + int(rng.integers(-8, 9))] = ord("N")
+        for t in (target, target[:n + 20] + b"N" + target[n + 21:]):
+            sp = gxy.SearchParams(1, gxy.HspParams(400, 900), 1)
+            g, o = both(gxy, ctx, t, bytes(q), pattern, sp)
+            assert g == o, (i, t is target)
