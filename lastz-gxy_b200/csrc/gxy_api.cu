@@ -90,7 +90,8 @@ gxy_status prune_table(gxy_table* t, uint32_t limit, Worker* W) {
     t->own_arrays = true;
     t->npos = total2;
     // Pruned buckets are empty now: their occupancy bits go.
-    launch_occupancy(t->starts, nw, t->occ, st);
+    launch_occupancy(t->starts, nw, t->occ, t->packed, st);
+    if (t->nbr) launch_neighbours(t->occ, 1, t->pat.weight, t->nbr, st);
     e = cudaStreamSynchronize(st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
@@ -107,10 +108,17 @@ TableMem::~TableMem() {
     dev_free(starts);
     dev_free(positions);
     dev_free(occ);
+    dev_free(nbr);
+    dev_free(packed);
     dev_free(rec);
 }
 
 namespace {
+
+// Tables of at least this many windows (a view, on average) carry neighbour
+// masks and packed bounds: writing 4^weight of them (48 MB, some 15 us, at weight
+// 12) then costs less than the searches of a query of that size save.
+constexpr uint64_t kNbrMinWindows = 1u << 19;
 
 // PosTable::build for n views [lo[v], hi[v]) of seq, as one sort; out[v] is
 // view v's table.  The tables share one TableMem.
@@ -154,7 +162,17 @@ gxy_status build_tables(gxy_ctx* ctx, const gxy_dseq* seq, uint32_t n, const uin
         launch_window_records(seq->codes, seq->valid, mem->rec_first, n_rec, mem->rec, st);
     }
     std::vector<uint32_t> first((size_t)n + 1);
-    API_TRY(atomic_build_views(seq, n, lo, hi, pat, step, mem->starts, mem->positions, mem->occ, first.data(), W));
+    const bool masks = total >= kNbrMinWindows * n && pat.weight >= kNbrMinWeight && pat.weight <= kNbrMaxWeight;
+    if (masks) {
+        e = dev_alloc((void**)&mem->nbr, (size_t)G * 2, st);
+        if (e == cudaSuccess) e = dev_alloc((void**)&mem->packed, (size_t)G, st);
+        if (e != cudaSuccess) {
+            set_error(std::string("table allocation: ") + cudaGetErrorString(e));
+            return GXY_ENOMEM;
+        }
+    }
+    API_TRY(atomic_build_views(seq, n, lo, hi, pat, step, mem->starts, mem->positions, mem->occ, mem->packed, first.data(), W));
+    if (masks) launch_neighbours(mem->occ, n, pat.weight, mem->nbr, st);
     std::vector<gxy_table*> made;
     auto fail = [&](gxy_status s) {
         for (gxy_table* t : made) {
@@ -182,6 +200,8 @@ gxy_status build_tables(gxy_ctx* ctx, const gxy_dseq* seq, uint32_t n, const uin
         t->positions = mem->positions;
         t->pos_base = first[v];
         t->occ = mem->occ + (size_t)v * nw / 32;
+        t->nbr = mem->nbr ? mem->nbr + (size_t)v * nw : nullptr;
+        t->packed = mem->packed ? mem->packed + (size_t)v * nw / 8 : nullptr;
         t->npos = first[v + 1] - first[v];
         if (mwc > 0) {
             const gxy_status ps = prune_table(t, mwc, W);
@@ -233,6 +253,8 @@ gxy_status search_impl(gxy_ctx* ctx, Worker* W, const gxy_table* table, const Se
     units[0].starts = table->starts;
     units[0].positions = table->positions;
     units[0].occ = table->occ;
+    units[0].nbr = table->nbr;
+    units[0].packed = table->packed;
     units[0].nwin = n_windows(Q.len, table->pat.len, p->step);
     units[0].primary_lo = units[0].primary_hi = 0;
     units[0].avg_bucket = table->num_words ? (double)table->npos / (double)table->num_words : 0.0;
@@ -708,6 +730,8 @@ static gxy_status batch_run(gxy_ctx* ctx, uint32_t n_tables, const gxy_table* co
         plan[i].starts = t->starts;
         plan[i].positions = t->positions;
         plan[i].occ = t->occ;
+        plan[i].nbr = t->nbr;
+        plan[i].packed = t->packed;
         plan[i].nwin = n_windows(queries[u.query]->len, pat.len, params->step);
         plan[i].primary_lo = u.primary_lo;
         plan[i].primary_hi = u.primary_hi;

@@ -16,7 +16,6 @@ namespace gxy {
 constexpr uint32_t kPad = 64;         // leading pad (positions)
 constexpr uint32_t kTailPad = 1536;   // trailing pad (positions); covers one warp stage
 constexpr int kMaxWeight = 15;        // 4^15 buckets; starts[] is u32 x (2^30 + 1)
-constexpr int kMaxVariants = 1 + 15 + 105;
 constexpr uint32_t kFull = 0xffffffffu;
 
 // Process-wide count of kernels this library launched (gxy_kernel_launches).
@@ -59,6 +58,8 @@ struct UnitDev {
     const uint32_t* starts;
     const uint32_t* positions;
     const uint32_t* occ;  // bucket occupancy bitmap (bit w & 31 of occ[w >> 5])
+    const uint16_t* nbr;  // neighbour masks, or null (see launch_neighbours)
+    const uint2* packed;  // bounds of eight buckets each (see pack_buckets), with nbr
     uint32_t nwin;        // query windows 0, step, ... <= len - L
     uint32_t tile_base;   // first screen tile of this unit
     uint32_t primary_lo;  // driver primary-region filter, src/driver.rs:250-256

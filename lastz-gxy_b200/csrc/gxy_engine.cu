@@ -249,18 +249,11 @@ static int bits_for(uint64_t x) {
     return b;   // smallest b with x < 2^b
 }
 
-static void build_variants(const Pattern& pat, uint32_t transitions, uint32_t* vx, uint32_t& nv) {
-    // src/seed_search.rs:63, :303-316.
+// Words a window looks up (src/seed_search.rs:63, :303-316): its own, those
+// with one care position's transition, those with two.
+static uint32_t count_variants(const Pattern& pat, uint32_t transitions) {
     const uint32_t w = pat.weight;
-    uint32_t shifts[16];
-    for (uint32_t i = 0; i < w; i++) shifts[i] = 2 * (w - 1 - i);
-    nv = 0;
-    vx[nv++] = 0;
-    if (transitions >= 1)
-        for (uint32_t i = 0; i < w; i++) vx[nv++] = 2u << shifts[i];
-    if (transitions >= 2)
-        for (uint32_t i = 0; i < w; i++)
-            for (uint32_t j = i + 1; j < w; j++) vx[nv++] = (2u << shifts[i]) ^ (2u << shifts[j]);
+    return 1 + (transitions >= 1 ? w : 0) + (transitions >= 2 ? w * (w ? w - 1 : 0) / 2 : 0);
 }
 
 gxy_status reserve_worker(gxy_ctx* ctx, Worker* W, uint64_t est_hits, uint64_t candidates, uint32_t max_units) {
@@ -273,7 +266,7 @@ gxy_status reserve_worker(gxy_ctx* ctx, Worker* W, uint64_t est_hits, uint64_t c
         W->surv_cap = want_s;
     }
     GXY_CK(W->surv.ensure((size_t)W->surv_cap * kHitBytes));
-    GXY_CK(W->redo.ensure((size_t)2 * kRedoCap * 4));
+    GXY_CK(W->redo.ensure((size_t)2 * kRedoCap * sizeof(uint2)));
     const size_t mu = std::max<uint32_t>(max_units, 1);
     GXY_CK(W->d_units.ensure(mu * sizeof(UnitDev)));
     GXY_CK(W->d_tsegs.ensure(mu * sizeof(SeqView)));
@@ -374,6 +367,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
     }
     std::vector<UnitDev> ud(nu);
     uint64_t tiles = 0;
+    bool masks = true;   // every table has neighbour masks
     for (uint32_t i = 0; i < nu; i++) {
         const UnitPlan& u = units[i];
         ud[i].tseg = u.tseg;
@@ -381,6 +375,9 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
         ud[i].starts = u.starts;
         ud[i].positions = u.positions;
         ud[i].occ = u.occ;
+        ud[i].nbr = u.nbr;
+        ud[i].packed = u.packed;
+        masks = masks && u.nbr;
         ud[i].nwin = u.nwin;
         ud[i].tile_base = (uint32_t)tiles;
         ud[i].primary_lo = u.primary_lo;
@@ -445,11 +442,17 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
     sa.tsegs = W->d_tsegs.as<SeqView>();
     sa.qsegs = W->d_qsegs.as<SeqView>();
     sa.n_units = nu;
-    sa.tile_lo = 0;
-    sa.tile_hi = (uint32_t)tiles;
+    // With two transitions, group 0 takes the words with at most one, group g > 0
+    // those with care position g - 1's and a later one's.
+    sa.n_groups = p.transitions >= 2 ? std::max<uint32_t>(1, pat.weight) : 1;
+    // The cursor may run some claims past the end.
+    sa.n_split = tiles * sa.n_groups < (1ull << 32) - (1u << 20) ? sa.n_groups : 1;
+    const uint64_t items = tiles * sa.n_split;
+    sa.n_items = (uint32_t)items;
+    sa.enum_mode = p.transitions == 0 ? 0 : (masks ? 1 : 2);
     sa.pat = pat;
     sa.step = p.step;
-    build_variants(pat, p.transitions, sa.var_xor, sa.n_var);
+    const uint32_t n_var = count_variants(pat, p.transitions);
     memcpy(sa.sc.sub, p.sub, sizeof(p.sub));
     sa.sc.ambig = p.ambig;
     sa.sc.xdrop = p.xdrop;
@@ -485,7 +488,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
     // the device.
     double est = 1 << 20, exp_random = 0, exp_windows = 0;
     for (const UnitPlan& u : units) {
-        exp_random += (double)u.nwin * sa.n_var * u.avg_bucket;
+        exp_random += (double)u.nwin * n_var * u.avg_bucket;
         exp_windows += (double)u.nwin;
     }
     est += 1.5 * exp_random;
@@ -519,7 +522,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
     const int blocks_misc = ctx->sm_count * 4;
     const int blocks_walk = (int)std::min<uint64_t>((uint64_t)blocks_misc, exp_cands / 32 + 8);
     const int walk_warps = ctx->tuning.walk_warps == 4 ? 4 : 8;
-    GXY_CK(W->redo.ensure((size_t)2 * kRedoCap * 4));
+    GXY_CK(W->redo.ensure((size_t)2 * kRedoCap * sizeof(uint2)));
 
     // One pass: start it (k_pass_reset), enumerate into the hit buffer, filter
     // and screen.  With timing (a one-pass launch outside a graph) the kernels
@@ -706,7 +709,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
         sa.cands = W->cands.as<Cand>();
         sa.cand_cap = cap;
         sa.ctl = cnt;
-        sa.redo = W->redo.as<uint32_t>();
+        sa.redo = W->redo.as<uint2>();
 
         // Round one: counters cleared, the passes, the epilogue and the
         // counters' copy back -- one CUDA graph (kept across calls and
@@ -749,7 +752,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
                 set_error("more tiles than the hit buffer's passes can carry over");
                 return GXY_ENOMEM;
             }
-            if (tile_at < tiles || redo_left) {
+            if (tile_at < items || redo_left) {
                 if (tile_at == last_tile && redo_left == last_redo) {
                     const unsigned long long mf = *reinterpret_cast<const unsigned long long*>(hc + kCMaxFail);
                     if (mf > W->hit_cap) {
@@ -761,7 +764,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
                 last_redo = redo_left;
                 multi = true;
                 const uint64_t more = std::min<uint64_t>(
-                    256, (uint64_t)((double)(tiles - std::min<uint64_t>(tile_at, tiles)) / tiles * first_round) + 2);
+                    256, (uint64_t)((double)(items - std::min<uint64_t>(tile_at, items)) / items * first_round) + 2);
                 for (uint64_t i = 0; i < more; i++) pass(false);
                 API_TRY_ENGINE(epilogue());
                 rounds++;

@@ -75,6 +75,8 @@ struct UnitPlan {
     const uint32_t* starts;
     const uint32_t* positions;
     const uint32_t* occ;   // the table's bucket occupancy bitmap
+    const uint16_t* nbr;   // its neighbour masks, or null
+    const uint2* packed;   // and its packed bounds, with nbr
     uint32_t nwin;
     uint32_t primary_lo;
     uint32_t primary_hi;
@@ -130,6 +132,8 @@ struct TableMem {
     uint32_t* starts = nullptr;      // tables x num_words + 1 global bucket starts
     uint32_t* positions = nullptr;   // the tables' positions, one after the other
     uint32_t* occ = nullptr;         // occupancy bits of all tables' buckets
+    uint16_t* nbr = nullptr;         // their neighbour masks, or null (see kNbrMinWindows)
+    uint2* packed = nullptr;         // bounds of eight buckets each, with nbr
     uint32_t* rec = nullptr;         // window records of the sequence words the views cover (SeqView::rec)
     uint64_t rec_first = 0;          // the first of those words
     ~TableMem();
@@ -146,6 +150,8 @@ struct gxy_table {
     uint32_t* positions = nullptr;   // likewise
     bool own_arrays = false;         // starts and positions are this table's own (after a prune)
     uint32_t* occ = nullptr;   // bit (w & 31) of occ[w >> 5]: bucket w is non-empty (in mem)
+    uint16_t* nbr = nullptr;   // neighbour masks (in mem), or null
+    uint2* packed = nullptr;   // packed bounds (in mem), with nbr
     // starts[w] index the shared positions array (positions points at its
     // start); this table's positions begin at pos_base (0 after a prune).
     uint32_t pos_base = 0;
@@ -216,7 +222,7 @@ inline uint32_t n_windows(uint64_t len, uint32_t L, uint32_t step) {
 // More than one view needs at least 32 buckets per view.
 gxy_status atomic_build_views(const gxy_dseq* seq, uint32_t n_views, const uint64_t* lo, const uint64_t* hi,
                               const Pattern& pat, uint32_t step, uint32_t* starts, uint32_t* positions,
-                              uint32_t* occ, uint32_t* first_host, Worker* W);
+                              uint32_t* occ, uint2* packed, uint32_t* first_host, Worker* W);
 // rec[8 j ..] = the window record of sequence word first + j (at least 1), for
 // j < n (SeqView::rec).
 void launch_window_records(const uint64_t* codes, const uint32_t* valid, uint64_t first, uint64_t n, uint32_t* rec,

@@ -198,7 +198,7 @@ __global__ __launch_bounds__(kFilterWarps * 32, 1) void k_filter_hits(const __gr
         if (surv && slot < a.hit_cap) {
             a.hits[slot] = t;
             a.hits[a.hit_cap + slot] = q;
-            a.hits[2 * a.hit_cap + slot] = u;
+            if (a.n_units > 1) a.hits[2 * a.hit_cap + slot] = u;
         }
     };
     auto enqueue = [&](bool on, uint32_t t, uint32_t q, uint32_t u, const FSide& R, const FSide& Lf, uint32_t state) {
@@ -234,7 +234,7 @@ __global__ __launch_bounds__(kFilterWarps * 32, 1) void k_filter_hits(const __gr
             if (idx < wend) {
                 t = __ldg(io.raw + idx);
                 q = __ldg(io.raw + io.raw_cap + idx);
-                u = __ldg(io.raw + 2 * io.raw_cap + idx);
+                u = q == kNoHit ? kNoUnit : (a.n_units > 1 ? __ldg(io.raw + 2 * io.raw_cap + idx) : 0u);
             }
             const bool on = u != kNoUnit;   // else an unused slot of a failed reservation
             if (on && u != cur_unit) take_unit(u);
@@ -373,15 +373,71 @@ __global__ __launch_bounds__(kFilterWarps * 32, 1) void k_filter_hits(const __gr
     if (lane == 0 && n_cols) atomicAdd(&a.stats[3], n_cols);
 }
 
-__global__ void k_occupancy(const uint32_t* __restrict__ starts, uint64_t nw, uint32_t* __restrict__ occ) {
+__global__ void k_occupancy(const uint32_t* __restrict__ starts, uint64_t nw, uint32_t* __restrict__ occ,
+                            uint2* __restrict__ packed) {
     const uint64_t warps = (uint64_t)gridDim.x * (blockDim.x >> 5);
     const uint64_t w0 = (uint64_t)blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5);
     const uint32_t lane = threadIdx.x & 31;
     for (uint64_t base = w0 * 32; base < nw; base += warps * 32) {
         const uint64_t w = base + lane;
-        const bool set = w < nw && __ldg(starts + w + 1) > __ldg(starts + w);
-        const uint32_t m = __ballot_sync(kFull, set);
+        const uint32_t b = w < nw ? __ldg(starts + w) : 0u, c = w < nw ? __ldg(starts + w + 1) - b : 0u;
+        const uint32_t m = __ballot_sync(kFull, c != 0);
         if (lane == 0) occ[base >> 5] = m;
+        if (packed) {
+            uint32_t y = c < 15 ? c << (4 * (lane & 7)) : 0xffffffffu;
+#pragma unroll
+            for (int o = 1; o < 8; o <<= 1) y |= __shfl_xor_sync(kFull, y, o);
+            if ((lane & 7) == 0 && w < nw) packed[w >> 3] = make_uint2(b, y);
+        }
+    }
+}
+
+// One thread per 32 buckets: the occupancy words of the bucket's own and its
+// neighbours' 32 (a transition flips the high bit of a care position: inside
+// the word for the last two positions, in another word for the rest), as 16
+// rows, transposed into 32 masks.
+__global__ void k_neighbours(const uint32_t* __restrict__ occ, uint64_t n_words, uint32_t words_per_view, uint32_t weight,
+                             uint16_t* __restrict__ nbr) {
+    for (uint64_t i = blockIdx.x * (uint64_t)blockDim.x + threadIdx.x; i < n_words; i += (uint64_t)gridDim.x * blockDim.x) {
+        const uint64_t view = i & ~(uint64_t)(words_per_view - 1);   // 4^weight / 32 words, a power of two
+        const uint32_t x = (uint32_t)(i - view);
+        const uint32_t w0 = __ldg(occ + i);
+        uint32_t r[16];
+        r[0] = w0;
+#pragma unroll
+        for (uint32_t v = 1; v < 16; v++) {
+            r[v] = 0;
+            if (v <= weight) {
+                const uint32_t bit = 2 * (weight - v) + 1;
+                if (bit == 1) r[v] = ((w0 >> 2) & 0x33333333u) | ((w0 & 0x33333333u) << 2);
+                else if (bit == 3) r[v] = ((w0 >> 8) & 0x00ff00ffu) | ((w0 & 0x00ff00ffu) << 8);
+                else r[v] = __ldg(occ + view + (x ^ (1u << (bit - 5))));
+            }
+        }
+        // Both 16 x 16 halves at once.
+        uint32_t m = 0x00ff00ffu;
+#pragma unroll
+        for (int j = 8; j; j >>= 1, m ^= m << j) {
+#pragma unroll
+            for (int k = 0; k < 16; k++) {
+                if (k & j) continue;
+                const uint32_t t = ((r[k] >> j) ^ r[k + j]) & m;
+                r[k + j] ^= t;
+                r[k] ^= t << j;
+            }
+        }
+        uint4* o = reinterpret_cast<uint4*>(nbr + 32 * i);
+#pragma unroll
+        for (int k = 0; k < 2; k++) {
+            uint32_t lo[4], hi[4];
+#pragma unroll
+            for (int c = 0; c < 4; c++) {
+                lo[c] = __byte_perm(r[8 * k + 2 * c], r[8 * k + 2 * c + 1], 0x5410);
+                hi[c] = __byte_perm(r[8 * k + 2 * c], r[8 * k + 2 * c + 1], 0x7632);
+            }
+            o[k] = make_uint4(lo[0], lo[1], lo[2], lo[3]);
+            o[2 + k] = make_uint4(hi[0], hi[1], hi[2], hi[3]);
+        }
     }
 }
 
@@ -436,11 +492,18 @@ void launch_filter_hits(const ScreenArgs& a, const FilterIO& io, uint64_t expect
     k_filter_hits<<<blocks, kFilterWarps * 32, kFilterSmem, st>>>(a, io);
 }
 
-void launch_occupancy(const uint32_t* starts, uint64_t num_words, uint32_t* occ, cudaStream_t st) {
+void launch_occupancy(const uint32_t* starts, uint64_t num_words, uint32_t* occ, uint2* packed, cudaStream_t st) {
     const uint64_t words = (num_words + 31) / 32;
     const int blocks = (int)std::min<uint64_t>((words + 7) / 8, 148 * 16);
     count_launch();
-    k_occupancy<<<std::max(blocks, 1), 256, 0, st>>>(starts, num_words, occ);
+    k_occupancy<<<std::max(blocks, 1), 256, 0, st>>>(starts, num_words, occ, packed);
+}
+
+void launch_neighbours(const uint32_t* occ, uint32_t n_views, uint32_t weight, uint16_t* nbr, cudaStream_t st) {
+    const uint32_t per_view = 1u << (2 * weight - 5);
+    const uint64_t words = (uint64_t)n_views * per_view;
+    count_launch();
+    k_neighbours<<<(int)std::min<uint64_t>((words + 255) / 256, 148 * 16), 256, 0, st>>>(occ, words, per_view, weight, nbr);
 }
 
 }  // namespace gxy

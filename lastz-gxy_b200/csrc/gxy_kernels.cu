@@ -323,218 +323,359 @@ __device__ __forceinline__ void scan_pair_any(SideScan& A, SideScan& B, uint32_t
 }
 
 // ---------------------------------------------------------------------------
-// Enumeration: one warp per tile of 32 consecutive query windows of one unit.
-// Each lane forms its window's seed word and transition variants
-// (src/seed_search.rs:76-90); the warp reserves room for all hits of the
-// tile with one atomic and writes (t, q, unit) for every position of every
-// variant's bucket (src/pos_table.rs:102-108).  Large buckets are copied by
-// the whole warp.
+// Enumeration: one warp per item -- a tile of 32 consecutive query windows of
+// one unit and a group of word variants.  Each lane forms its window's seed word
+// (src/seed_search.rs:76-90) by table, and a mask of the variants whose bucket
+// is not empty: with transitions, bit 1 + i stands for the word with care
+// position i's transition.  The table's neighbour masks give it in one read
+// (13 occupancy bits, one read each, took most of the L2 traffic before).  Two
+// transitions take a group for every first one: the masks of the words one
+// transition away, less the pairs other groups hold; a group is an item of its own while the items can be counted in
+// 32 bits (n_split), else a tile is.
+//
+// The masks' bits -- a tenth to half of the variants -- are listed across the
+// warp, so that the bucket bounds and the positions are read 32 entries at a
+// time with every lane at work; the warp reserves room for all hits of the item
+// with one atomic and writes (t, q[, unit]) for every position of every listed
+// bucket (src/pos_table.rs:102-108), neighbouring lanes to neighbouring slots.
+//
+// What bounds it: the latency of dependent reads (words, mask, bounds,
+// position) and the L2 sectors of the last two.  10 M windows against a table of
+// 10 M positions, one transition, 26.1 M hits: 0.38 ms, 101 M L2 sectors and
+// 0.60 GB of DRAM traffic (with 13 occupancy bits and the plain starts read per
+// window 0.74 ms; with the masks and the plain starts, 64 MB that push the masks
+// and positions out of L2, 0.59 ms and 1.7 GB; four entries a lane at a time
+// instead of two spill registers, 0.42 ms).
 // ---------------------------------------------------------------------------
 __device__ __forceinline__ void store_hit(const ScreenArgs& a, uint64_t i, uint32_t t, uint32_t q, uint32_t u) {
     a.hits[i] = t;
     a.hits[a.hit_cap + i] = q;
-    a.hits[2 * a.hit_cap + i] = u;
+    if (a.n_units > 1) a.hits[2 * a.hit_cap + i] = u;
 }
 
-// kRegVar: variants whose bucket bounds stay in registers between the two
-// passes (the rest are re-read): 1 without transitions, 13 for weight 12 with
-// one transition, else 16.
-template <uint32_t kRegVar>
-__global__ __launch_bounds__(256, 4) void k_enumerate(const __grid_constant__ ScreenArgs a) {
-    __shared__ unsigned long long s_stats[2];   // windows, raw hits
-    if (threadIdx.x < 2) s_stats[threadIdx.x] = 0;
-    __syncthreads();
+constexpr int kEnumWarps = 8, kEnumBlocks = 4;   // 39 KB of shared memory a block, 43 with a lane a byte
+constexpr uint32_t kWordBits = (1u << 27) - 1;   // of an entry; the lane above
+
+// kMode 0: the words themselves only; 1: neighbour masks; 2: masks formed from
+// the occupancy bitmap (tables without neighbour masks).
+template <int kMode>
+__global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(const __grid_constant__ ScreenArgs a) {
+    constexpr uint32_t kEntries = kMode == 0 ? 32 : 512;   // 32 masks of at most 16 bits
+    constexpr int K = kMode == 0 ? 1 : 2;                  // entries a lane holds at a time
+    __shared__ unsigned long long s_stats[2];              // windows, raw hits
+    __shared__ uint32_t s_word[8][256];                    // what byte k of a window's codes gives the word
+    __shared__ uint32_t s_ent[kEnumWarps][kEntries];       // the entries' words, then their buckets' starts
+    __shared__ uint32_t s_cnt[kEnumWarps][kMode == 0 ? 1 : kEntries - 64];   // lane and size from entry 64 on
+    __shared__ uint8_t s_who[kMode == 1 ? 1 : kEnumWarps][kEntries];          // the entries' lanes
     const int lane = threadIdx.x & 31;
-    const uint32_t ntile = a.tile_hi - a.tile_lo;
-    unsigned long long n_windows = 0, n_raw = 0;
+    const uint32_t n_bytes = (a.pat.len + 3) / 4, weight = a.pat.weight;
+    if (threadIdx.x < 2) s_stats[threadIdx.x] = 0;
+    for (uint32_t i = threadIdx.x; i < n_bytes * 256; i += blockDim.x) {
+        uint32_t w = 0;
+#pragma unroll
+        for (uint32_t c = 0; c < 4; c++) {
+            const uint32_t pos = 4 * (i >> 8) + c;
+            if ((a.pat.care_mask >> pos) & 1u)
+                w |= ((i >> (2 * c)) & 3u) << (2 * (weight - 1 - __popc(a.pat.care_mask & ((1u << pos) - 1u))));
+        }
+        s_word[i >> 8][i & 255] = w;
+    }
+    __syncthreads();
+    uint32_t* const ent = s_ent[threadIdx.x >> 5];
+    uint32_t* const cnt = s_cnt[threadIdx.x >> 5];
+    uint8_t* const who = s_who[kMode == 1 ? 0 : threadIdx.x >> 5];
+    const uint32_t n_items = a.n_items, n_groups = a.n_groups, n_split = a.n_split;
+    uint32_t windows = 0, n_raw = 0;   // of the lane, of the warp: fewer than the tiles and the buffer's slots
     uint32_t* const ctl = a.ctl;
     unsigned long long* const max_fail = reinterpret_cast<unsigned long long*>(ctl + kCMaxFail);
-    // This pass takes the tiles the previous pass could not fit first (its
-    // redo list), then fresh tiles until the hit buffer is full.
+    // This pass takes the items the previous pass could not fit first (its
+    // redo list), then fresh items until the hit buffer is full.
     const uint32_t pass = ctl[kCPass];
-    const uint32_t* redo_in = a.redo + ((pass - 1) & 1u) * kRedoCap;
-    uint32_t* redo_out = a.redo + (pass & 1u) * kRedoCap;
+    const uint2* redo_in = a.redo + ((pass - 1) & 1u) * kRedoCap;
+    uint2* redo_out = a.redo + (pass & 1u) * kRedoCap;
     const uint32_t n_redo = ctl[kCRedoN + ((pass - 1) & 1u)];
     uint32_t* const n_redo_out = ctl + kCRedoN + (pass & 1u);
-    // A tile that did not fit this pass goes to the next pass's list.
-    auto defer = [&](uint32_t tl, unsigned long long wtot) {
+    // A tile's group that did not fit this pass goes to the next pass's list.
+    auto defer = [&](uint32_t tile, uint32_t group, unsigned long long wtot) {
         atomicExch(ctl + kCStop, 1u);
         const uint32_t i = atomicAdd(n_redo_out, 1u);
-        if (i < kRedoCap) redo_out[i] = tl;
+        if (i < kRedoCap) redo_out[i] = make_uint2(tile, group);
         else atomicExch(ctl + kCRedoOver, 1u);
         atomicMax(max_fail, wtot);
     };
-    bool redo_done = false;
-    // Fresh tiles are claimed kClaim at a time, and the next claim is made
-    // while the current tiles are processed: one atomic per kClaim tiles
+    bool redo_done = n_redo == 0;
+    // Fresh items are claimed kClaim at a time, and the next claim is made
+    // while the current items are processed: one atomic per kClaim items
     // (all warps hit that counter), its round trip off the critical path.
     // (Measured on the 10 Mbp plain launch: 2 beats 4 by 2 % and 8 is slower.)
     constexpr uint32_t kClaim = 2;
     uint32_t next = 0xffffffffu;   // a claimed batch not yet started (warp-uniform)
+    uint32_t u = 0, u_lo = 1, u_hi = 0;   // the current unit and its tiles (none yet)
+    const UnitDev* U = a.units;   // (read where used: kept in registers, they spilled others)
     for (;;) {
-      uint32_t batch, batch_end;
+      uint32_t batch, batch_end, group, group_end;   // items (or one listed tile), their groups
       if (!redo_done) {
           uint32_t i = 0;
           if (lane == 0) i = atomicAdd(ctl + kCRedoTake, 1u);
           i = __shfl_sync(kFull, i, 0);
           if (i < n_redo) {
-              batch = redo_in[i];
-              batch_end = batch + 1;
+              const uint2 r = redo_in[i];
+              batch = r.x;
+              batch_end = r.x + 1;
+              group = r.y;
+              group_end = n_split > 1 ? r.y + 1 : n_groups;
           } else {
               redo_done = true;
               continue;
           }
       } else {
           if (next == 0xffffffffu) {
-              // Stop claiming once the buffer is full; the tiles not claimed
-              // yet wait for the next pass behind the tile cursor.
+              // Stop claiming once the buffer is full; the items not claimed
+              // yet wait for the next pass behind the cursor.
               if (*reinterpret_cast<volatile uint32_t*>(ctl + kCStop)) break;
               uint32_t c = 0;
               if (lane == 0) c = atomicAdd(a.tile_counter, kClaim);
               next = __shfl_sync(kFull, c, 0);
           }
           batch = next;
-          if (batch >= ntile) break;
+          if (batch >= n_items) break;
           next = 0xffffffffu;
           if (!*reinterpret_cast<volatile uint32_t*>(ctl + kCStop)) {
               uint32_t c = 0;
               if (lane == 0) c = atomicAdd(a.tile_counter, kClaim);
               next = __shfl_sync(kFull, c, 0);
           }
-          batch_end = min(ntile, batch + kClaim);
+          batch_end = min(n_items, batch + kClaim);
+          group = 0;
+          group_end = n_groups;
       }
-      for (uint32_t tl = batch; tl < batch_end; tl++) {
-        uint32_t tile = tl + a.tile_lo;
-        uint32_t lo = 0, hi = a.n_units;
-        while (hi - lo > 1) {
-            const uint32_t mid = (lo + hi) >> 1;
-            if (a.units[mid].tile_base <= tile) lo = mid;
-            else hi = mid;
+      for (uint32_t item = batch; item < batch_end; item++) {
+        uint32_t tile = item, g = group, g_end = group_end;
+        if (n_split > 1 && redo_done) {   // an item is one group of a tile
+            tile = item / n_split;
+            g = item - tile * n_split;
+            g_end = g + 1;
         }
-        const uint32_t u = lo;
-        const UnitDev U = a.units[u];
-        const uint32_t k = (tile - U.tile_base) * 32 + lane;
-        const uint32_t q = k * a.step;
-        uint32_t word = 0;
+        if (tile < u_lo || tile >= u_hi) {
+            uint32_t lo = 0, hi = a.n_units;
+            while (hi - lo > 1) {
+                const uint32_t mid = (lo + hi) >> 1;
+                if (a.units[mid].tile_base <= tile) lo = mid;
+                else hi = mid;
+            }
+            u = lo;
+            U = a.units + u;
+            u_lo = U->tile_base;
+            u_hi = u_lo + (U->nwin + 31) / 32;
+        }
+        const uint32_t k = (tile - u_lo) * 32 + lane;
+        // The window's word: its codes a byte at a time through the tables.
+        uint32_t word0 = 0;
         bool wv = false;
-        if (k < U.nwin) wv = word_at(a.qsegs[U.qseg], a.pat, q, word);
-        // Pass 1: this lane's hit count over all variants.  The bucket
-        // bounds of the first kRegVar variants stay in registers for pass 2.
-        uint32_t rb[kRegVar], rc[kRegVar];
-        uint32_t tot = 0;
-        // The occupancy bit first: `starts` is read for non-empty buckets
-        // only (about two thirds of the variant words of a 10 Mbp target
-        // fall in empty buckets, and the 2 MB bitmap stays in L2).
-        uint32_t ob[kRegVar];
+        if (k < U->nwin) {
+            const SeqView& Q = a.qsegs[U->qseg];
+            const uint64_t gq = Q.base + (uint64_t)k * a.step;
+            const uint32_t ok = load_bits32(Q.valid, gq) & ~load_bits32(Q.mask, gq);
+            const uint64_t c = load_codes32(Q.codes, gq);
+            wv = (ok & a.pat.care_mask) == a.pat.care_mask;
 #pragma unroll
-        for (uint32_t v = 0; v < kRegVar; v++)
-            ob[v] = (wv && v < a.n_var) ? __ldg(U.occ + ((word ^ a.var_xor[v]) >> 5)) : 0u;
-#pragma unroll
-        for (uint32_t v = 0; v < kRegVar; v++) {
-            rb[v] = 0;
-            rc[v] = 0;
-            const uint32_t vw = word ^ a.var_xor[v];
-            if ((ob[v] >> (vw & 31u)) & 1u) {
-                rb[v] = __ldg(U.starts + vw);
-                rc[v] = __ldg(U.starts + vw + 1) - rb[v];
-                tot += rc[v];
-            }
+            for (uint32_t x = 0; x < 8; x++)
+                if (x < n_bytes) word0 |= s_word[x][(uint32_t)(c >> (8 * x)) & 255u];
         }
+        for (; g < g_end; g++) {
+        if (g == 0) windows += wv ? 1 : 0;
+        // Group g > 0: the words one transition (of care position g - 1) away, with
+        // a second one at a later position.
+        const uint32_t word = kMode != 0 && g ? word0 ^ (2u << (2 * (weight - g))) : word0;
+        uint32_t mask = 0;
         if (wv) {
-            for (uint32_t v = kRegVar; v < a.n_var; v++) {
-                const uint32_t vw = word ^ a.var_xor[v];
-                tot += __ldg(U.starts + vw + 1) - __ldg(U.starts + vw);
+            if (kMode == 0) {
+                mask = (__ldg(U->occ + (word >> 5)) >> (word & 31u)) & 1u;
+            } else if (kMode == 1) {
+                mask = __ldg(U->nbr + word);
+            } else {
+                for (uint32_t i = 0; i <= weight; i++) {
+                    const uint32_t w = i ? word ^ (2u << (2 * (weight - i))) : word;
+                    mask |= ((__ldg(U->occ + (w >> 5)) >> (w & 31u)) & 1u) << i;
+                }
             }
+            if (kMode != 0 && g) mask &= ~((2u << g) - 1u);
         }
-        uint32_t incl = tot;
+        // ---- the masks' bits, listed: bucket word and lane of each.
+        const uint32_t mine = __popc(mask);
+        uint32_t pos = mine;
 #pragma unroll
         for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, incl, o);
-            if (lane >= o) incl += y;
+            const uint32_t y = __shfl_up_sync(kFull, pos, o);
+            if (lane >= o) pos += y;
         }
-        const uint32_t wtot = __shfl_sync(kFull, incl, 31);
-        if (wtot == 0) {
-            n_windows += wv ? 1 : 0;
-            continue;
+        const uint32_t n_ent = __shfl_sync(kFull, pos, 31);
+        if (n_ent == 0) continue;
+        pos -= mine;
+        __syncwarp();
+        if (kMode == 1) {   // (bit by bit: finding the next one set has a longer latency)
+            const uint32_t tagged = word | (uint32_t)lane << 27;
+            if (mask & 1u) ent[pos++] = tagged;
+            uint32_t flip = 2u << (2 * (weight - 1));
+#pragma unroll
+            for (uint32_t v = 1; v <= kNbrMaxWeight; v++, flip >>= 2)
+                if ((mask >> v) & 1u) ent[pos++] = tagged ^ flip;
+        } else {
+            while (mask) {
+                const uint32_t v = __ffs(mask) - 1;
+                mask &= mask - 1;
+                ent[pos] = v ? word ^ (2u << (2 * (weight - v))) : word;
+                who[pos] = (uint8_t)lane;
+                pos++;
+            }
         }
+        __syncwarp();
+        // ---- their bounds: start, and size with the lane in the top bits, the first 64 entries' in
+        // registers, the others' in place of the words; and the item's hits.
+        uint32_t rb[K], rc[K], wtot = 0;
+        auto bounds = [&](uint32_t e0) {
+            uint32_t w[K];
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                w[k] = 0;
+                rc[k] = 0;
+                if (e0 + 32 * k + lane < n_ent) w[k] = ent[e0 + 32 * k + lane];
+            }
+            if (kMode == 1) {
+                uint2 p[K];
+#pragma unroll
+                for (int k = 0; k < K; k++)
+                    if (e0 + 32 * k + lane < n_ent) p[k] = __ldg(U->packed + ((w[k] & kWordBits) >> 3));
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    if (e0 + 32 * k + lane < n_ent) {
+                        const uint32_t sh = 4 * (w[k] & 7u), below = p[k].y & ((1u << sh) - 1u);
+                        rb[k] = p[k].x + __dp4a((below & 0x0f0f0f0fu) + ((below >> 4) & 0x0f0f0f0fu), 0x01010101u, 0u);
+                        uint32_t c = (p[k].y >> sh) & 15u;
+                        if (p[k].y == 0xffffffffu) {   // a bucket of 15 or more among the eight
+                            rb[k] = __ldg(U->starts + (w[k] & kWordBits));
+                            c = __ldg(U->starts + (w[k] & kWordBits) + 1) - rb[k];
+                        }
+                        wtot += c;
+                        rc[k] = min(c, kWordBits) | (w[k] & ~kWordBits);
+                    }
+                }
+            } else {
+                uint32_t h[K];
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    if (e0 + 32 * k + lane < n_ent) {
+                        rb[k] = __ldg(U->starts + w[k]);
+                        h[k] = __ldg(U->starts + w[k] + 1);
+                    }
+                }
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    if (e0 + 32 * k + lane < n_ent) {
+                        wtot += h[k] - rb[k];
+                        rc[k] = min(h[k] - rb[k], kWordBits) | (uint32_t)who[e0 + 32 * k + lane] << 27;
+                    }
+                }
+            }
+        };
+        for (uint32_t e0 = (n_ent - 1) & ~63u; e0; e0 -= 64) {
+            bounds(e0);
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                if (e0 + 32 * k + lane < n_ent) {
+                    ent[e0 + 32 * k + lane] = rb[k];
+                    cnt[e0 - 64 + 32 * k + lane] = rc[k];
+                }
+            }
+        }
+        bounds(0);
+        wtot = __reduce_add_sync(kFull, wtot);
         unsigned long long base = 0;
         if (lane == 0) base = atomicAdd(a.hit_count, (unsigned long long)wtot);
-        // Pass 2: write this lane's hits into its slots [dst, dst + tot).
-        // Their order within the slots is free (candidates are sorted by a
-        // unique (diagonal, t) key later), so the first position of every
-        // small bucket is loaded at once, before the rest; the first batch of
-        // those loads is in flight while the reservation comes back.
-        uint32_t first[8];
+        // ---- entry e's first hit takes slot e, the second hits of the larger buckets
+        // come behind those, and so on: both 32 consecutive slots at a time.  The
+        // hits' order in the buffer is free (candidates are sorted by a unique
+        // (diagonal, t) key later).
+        uint32_t first[K];
 #pragma unroll
-        for (uint32_t i = 0; i < 8; i++)
-            if (i < kRegVar) first[i] = (rc[i] != 0 && rc[i] <= 16) ? __ldg(U.positions + rb[i]) : 0u;
+        for (int k = 0; k < K; k++)   // on their way while the reservation comes back
+            if (32 * k + lane < n_ent) first[k] = __ldg(U->positions + rb[k]);
         base = __shfl_sync(kFull, base, 0);
         if (base + wtot > a.hit_cap) {
-            // The buffer is full: this tile goes to the next pass, and the
+            // The buffer is full: this item goes to the next pass, and the
             // part of its reservation inside the buffer is marked unused.
-            if (lane == 0) defer(tl, wtot);
+            if (lane == 0) defer(tile, g, wtot);
             for (uint64_t j = base + lane; j < min((unsigned long long)a.hit_cap, base + wtot); j += 32)
-                a.hits[2 * a.hit_cap + j] = kNoUnit;
-            continue;
+                a.hits[a.hit_cap + j] = kNoHit;
+            if (g == 0) windows -= wv ? 1 : 0;
+            break;   // with the groups after it
         }
-        n_windows += wv ? 1 : 0;
         n_raw += lane == 0 ? wtot : 0;
-        uint64_t dst = base + (incl - tot);
+        const uint32_t q0 = (tile - u_lo) * 32;
+        uint64_t more = base + n_ent;   // where the next further hits go
+        for (uint32_t e0 = 0;;) {
 #pragma unroll
-        for (uint32_t v0 = 0; v0 < kRegVar; v0 += 8) {
-            if (v0) {
+            for (int k = 0; k < K; k++)
+                if (e0 + 32 * k + lane < n_ent)
+                    store_hit(a, base + e0 + 32 * k + lane, first[k], (q0 + (rc[k] >> 27)) * a.step, u);
 #pragma unroll
-                for (uint32_t i = 0; i < 8; i++)
-                    if (v0 + i < kRegVar)
-                        first[i] = (rc[v0 + i] != 0 && rc[v0 + i] <= 16) ? __ldg(U.positions + rb[v0 + i]) : 0u;
-            }
-#pragma unroll
-            for (uint32_t i = 0; i < 8; i++)
-                if (v0 + i < kRegVar && rc[v0 + i] != 0 && rc[v0 + i] <= 16)
-                    store_hit(a, dst++, first[i], q, u);
-        }
-        for (uint32_t v = 0; v < a.n_var; v++) {
-            uint32_t b = 0, c = 0;
-            if (v < kRegVar) {
-#pragma unroll
-                for (uint32_t x = 0; x < kRegVar; x++)
-                    if (x == v) {
-                        b = rb[x];
-                        c = rc[x];
+            for (int k = 0; k < K; k++) {
+                if (e0 + 32 * k >= n_ent) break;
+                const uint32_t c = rc[k] & kWordBits, q = (q0 + (rc[k] >> 27)) * a.step;
+                const bool big = c > 16;
+                for (uint32_t j = 1;; j++) {
+                    const uint32_t m = __ballot_sync(kFull, c > j && !big);
+                    if (m == 0) break;
+                    if (c > j && !big)
+                        store_hit(a, more + __popc(m & ((1u << lane) - 1u)), __ldg(U->positions + rb[k] + j), q, u);
+                    more += __popc(m);
+                }
+                uint32_t bm = __ballot_sync(kFull, big);
+                while (bm) {   // a large bucket is copied by the whole warp
+                    const int src = __ffs(bm) - 1;
+                    bm &= bm - 1;
+                    const uint32_t bb = __shfl_sync(kFull, rb[k], src);
+                    uint32_t cc = __shfl_sync(kFull, c, src);
+                    const uint32_t qq = __shfl_sync(kFull, q, src);
+                    if (cc == kWordBits) {   // its size did not fit: the next larger start ends it
+                        uint32_t lo = 0, hi = 1u << (2 * weight);
+                        while (lo < hi) {
+                            const uint32_t mid = lo + (hi - lo) / 2;
+                            if (U->starts[mid] > bb) hi = mid;
+                            else lo = mid + 1;
+                        }
+                        cc = U->starts[lo] - bb;
                     }
-            } else if (wv) {
-                const uint32_t vw = word ^ a.var_xor[v];
-                b = __ldg(U.starts + vw);
-                c = __ldg(U.starts + vw + 1) - b;
+                    for (uint32_t j = 1 + lane; j < cc; j += 32)
+                        store_hit(a, more + j - 1, __ldg(U->positions + bb + j), qq, u);
+                    more += cc - 1;
+                }
             }
-            const bool big = c > 16;
-            // Small buckets of the first kRegVar variants wrote their first position above.
-            const uint32_t j0 = (v < kRegVar && !big) ? 1u : 0u;
-            if (!big) {
-                for (uint32_t j = j0; j < c; j++) store_hit(a, dst++, __ldg(U.positions + b + j), q, u);
+            e0 += 64;
+            if (e0 >= n_ent) break;
+#pragma unroll
+            for (int k = 0; k < K; k++) {
+                rc[k] = 0;
+                if (e0 + 32 * k + lane < n_ent) {
+                    rb[k] = ent[e0 + 32 * k + lane];
+                    rc[k] = cnt[e0 - 64 + 32 * k + lane];
+                    first[k] = __ldg(U->positions + rb[k]);
+                }
             }
-            uint32_t bm = __ballot_sync(kFull, big);
-            while (bm) {
-                const int src = __ffs(bm) - 1;
-                bm &= bm - 1;
-                const uint32_t bb = __shfl_sync(kFull, b, src), cc = __shfl_sync(kFull, c, src);
-                const uint32_t qq = __shfl_sync(kFull, q, src);
-                const uint64_t dd = __shfl_sync(kFull, dst, src);
-                for (uint32_t j = lane; j < cc; j += 32) store_hit(a, dd + j, __ldg(U.positions + bb + j), qq, u);
-            }
-            if (big) dst += c;
+        }
         }
       }
     }
     // A batch claimed ahead but not started: the next pass takes it.
     if (next != 0xffffffffu && lane == 0)
-        for (uint32_t tl = next; tl < min(ntile, next + kClaim); tl++) defer(tl, 0);
+        for (uint32_t item = next; item < min(n_items, next + kClaim); item++) defer(item / n_split, item % n_split, 0);
+    unsigned long long n_windows = windows;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) n_windows += __shfl_xor_sync(kFull, n_windows, o);
     // One pair of global atomics a block: every warp's own took longer than the
     // work of a small launch.
     if (lane == 0 && n_windows) atomicAdd(&s_stats[0], n_windows);
-    if (lane == 0 && n_raw) atomicAdd(&s_stats[1], n_raw);
+    if (lane == 0 && n_raw) atomicAdd(&s_stats[1], (unsigned long long)n_raw);
     __syncthreads();
     if (threadIdx.x < 2 && s_stats[threadIdx.x]) atomicAdd(&a.stats[threadIdx.x], s_stats[threadIdx.x]);
 }
@@ -564,12 +705,12 @@ void launch_pass_reset(uint32_t* ctl, uint64_t surv_cap, cudaStream_t st) {
 
 void launch_enumerate(const ScreenArgs& a, int sm_count, cudaStream_t st) {
     count_launch();
-    // A warp per tile at most: the idle warps of a full grid took 30 us to claim
+    // A warp per item at most: the idle warps of a full grid took 30 us to claim
     // nothing on a 30 kbp query (938 tiles).
-    const int blocks = (int)std::max<uint64_t>(1, umin64(((uint64_t)(a.tile_hi - a.tile_lo) + 7) / 8, (uint64_t)sm_count * 8));
-    if (a.n_var == 1) k_enumerate<1><<<blocks, 256, 0, st>>>(a);
-    else if (a.n_var == 13) k_enumerate<13><<<blocks, 256, 0, st>>>(a);
-    else k_enumerate<16><<<blocks, 256, 0, st>>>(a);
+    const int blocks = (int)std::max<uint64_t>(1, umin64(((uint64_t)a.n_items + kEnumWarps - 1) / kEnumWarps, (uint64_t)sm_count * kEnumBlocks));
+    if (a.enum_mode == 0) k_enumerate<0><<<blocks, kEnumWarps * 32, 0, st>>>(a);
+    else if (a.enum_mode == 1) k_enumerate<1><<<blocks, kEnumWarps * 32, 0, st>>>(a);
+    else k_enumerate<2><<<blocks, kEnumWarps * 32, 0, st>>>(a);
 }
 
 // ---------------------------------------------------------------------------
@@ -627,7 +768,7 @@ __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen_wide(const __grid_c
             if (rk < take) {
                 ht = a.hits[base + rk];
                 hq = a.hits[a.hit_cap + base + rk];
-                hu = a.hits[2 * a.hit_cap + base + rk];
+                hu = hq == kNoHit ? kNoUnit : (a.n_units > 1 ? a.hits[2 * a.hit_cap + base + rk] : 0u);
                 if (hu != kNoUnit && hu != cur_unit) {
                     cur_unit = hu;
                     const UnitDev U = a.units[hu];
@@ -975,7 +1116,7 @@ __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen(const __grid_consta
             if (hidx != 0xffffffffu) {
                 ht = a.hits[hidx];
                 hq = a.hits[a.hit_cap + hidx];
-                hu = a.hits[2 * a.hit_cap + hidx];
+                hu = hq == kNoHit ? kNoUnit : (a.n_units > 1 ? a.hits[2 * a.hit_cap + hidx] : 0u);
                 if (hu != kNoUnit && hu != cur_unit) {
                     cur_unit = hu;
                     const UnitDev U = a.units[hu];

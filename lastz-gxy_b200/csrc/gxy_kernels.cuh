@@ -60,15 +60,17 @@ void launch_prune_copy(const uint32_t* positions, const uint32_t* starts, uint64
 
 // --- search ------------------------------------------------------------------
 // Seed hits: target position t, query window q, unit, in three arrays of the
-// buffer's capacity (hits[i], hits[cap + i], hits[2 cap + i]).  unit kNoUnit
-// marks a slot of a hit-buffer reservation that failed (skipped by readers).
+// buffer's capacity (hits[i], hits[cap + i], hits[2 cap + i]; the units are
+// not kept when the launch has one).  q kNoHit marks a slot of a hit-buffer
+// reservation that failed (skipped by readers).
+constexpr uint32_t kNoHit = 0xffffffffu;
 constexpr size_t kHitBytes = 12;
 constexpr uint32_t kNoUnit = 0xffffffffu;
 
 // Layout of a worker's device counters (u32 indices).  The ones every warp
 // hits with atomics sit 1-4 KB apart so that they fall in different L2
 // slices.
-//  - per launch: [kCTile] tile cursor, [kCPass] passes run, [kCCand]
+//  - per launch: [kCTile] item cursor, [kCPass] passes run, [kCCand]
 //    candidates, [kCHsps] HSPs, [kCRecs] records, u64 [kCStats] statistics,
 //    [kCRedoN + 0/1] redo-list lengths, u64 [kCMaxFail] largest tile that
 //    did not fit the hit buffer, flags [kCSurvOver] and [kCRedoOver],
@@ -90,13 +92,13 @@ struct ScreenArgs {
     const SeqView* tsegs;
     const SeqView* qsegs;
     uint32_t n_units;
-    uint32_t tile_lo;      // this pass enumerates tiles [tile_lo, tile_hi)
-    uint32_t tile_hi;
+    uint32_t n_items;      // enumeration items: tiles of 32 query windows x n_split
+    uint32_t n_groups;     // 1, or with two transitions one per first transition and one for the rest
+    uint32_t n_split;      // n_groups: an item is one group of a tile; 1: all groups
+    int enum_mode;         // 0: no transitions, 1: neighbour masks, 2: masks from the occupancy bitmaps
     uint32_t* tile_counter;
     Pattern pat;
     uint32_t step;
-    uint32_t n_var;
-    uint32_t var_xor[kMaxVariants];
     Score sc;
     uint32_t cap;          // columns per side before a hit is deferred
     uint32_t qkey_total;   // size of the query key axis
@@ -120,13 +122,13 @@ struct ScreenArgs {
     // Passes that resume on the device: the worker's counters (layout
     // above) and the two redo lists of tiles that did not fit the hit buffer.
     uint32_t* ctl;
-    uint32_t* redo;
+    uint2* redo;           // (tile, first group) each
 };
-// Seed-hit enumeration: one warp per tile of 32 query windows; writes the
-// hits of every (window, variant) bucket to a.hits.  A pass takes the tiles
-// the previous pass could not fit first, then fresh tiles from a.tile_counter
-// until the hit buffer is full; a tile that does not fit goes to the next
-// pass's list.
+// Seed-hit enumeration: one warp per item (a tile of 32 query windows and a
+// group of variants); writes the hits of every (window, variant) bucket to
+// a.hits.  A pass takes the items the previous pass could not fit first, then
+// fresh ones from a.tile_counter until the hit buffer is full; an item that
+// does not fit goes to the next pass's list.
 void launch_enumerate(const ScreenArgs& a, int sm_count, cudaStream_t st);
 // Starts a pass: flags survivor overflow of the previous pass (its count above
 // surv_cap), advances the pass counter and resets the per-pass counters.
@@ -155,7 +157,17 @@ void launch_filter_hits(const ScreenArgs& a, const FilterIO& io, uint64_t expect
 void filter_init();
 // Bucket occupancy bitmap of a table: bit (w & 31) of occ[w >> 5] is set iff
 // bucket w holds a position.
-void launch_occupancy(const uint32_t* starts, uint64_t num_words, uint32_t* occ, cudaStream_t st);
+// and, if packed is not null, its packed bounds: one uint2 for eight buckets, x
+// the first one's start, y their sizes in four bits each, or ~0 when one of
+// them holds 15 positions or more.  A quarter of the starts' bytes:
+// those of 16.7 M buckets stay in L2 beside masks and positions.
+void launch_occupancy(const uint32_t* starts, uint64_t num_words, uint32_t* occ, uint2* packed, cudaStream_t st);
+// Neighbour masks of n_views tables of 4^weight buckets (kNbrMinWeight <=
+// weight <= kNbrMaxWeight) from their occupancy bitmaps, one after the other:
+// bit 0 of nbr[w] is bucket w's occupancy, bit 1 + i that of w with the
+// transition of care position i.
+constexpr uint32_t kNbrMinWeight = 3, kNbrMaxWeight = 13;
+void launch_neighbours(const uint32_t* occ, uint32_t n_views, uint32_t weight, uint16_t* nbr, cudaStream_t st);
 
 struct WalkArgs {
     const uint64_t* keys;      // candidate keys in sorted order

@@ -150,6 +150,8 @@ gxy_status run_batch(gxy_server* s, Worker* W, std::vector<Request*>& batch) {
             u.starts = t->starts;
             u.positions = t->positions;
             u.occ = t->occ;
+            u.nbr = t->nbr;
+            u.packed = t->packed;
             u.nwin = n_windows(q->len, pat.len, s->params.step);
             u.primary_lo = u.primary_hi = 0;
             u.avg_bucket = t->num_words ? (double)t->npos / (double)t->num_words : 0.0;

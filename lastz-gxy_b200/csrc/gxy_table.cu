@@ -118,7 +118,8 @@ __device__ __forceinline__ void order_bucket(uint32_t* __restrict__ pos, uint32_
 // index, size) pairs.  The lists hold every such bucket: at most n / 4 + 1,
 // n / 33 + 1 and n / (kBlockBucket + 1) + 1 of them for n positions.
 __global__ void k_sort_small_buckets(const uint32_t* __restrict__ starts, uint64_t nb, uint32_t* __restrict__ pos,
-                                     uint32_t* __restrict__ occ, uint2* __restrict__ mid, uint32_t* n_mid,
+                                     uint32_t* __restrict__ occ, uint2* __restrict__ packed,
+                                     uint2* __restrict__ mid, uint32_t* n_mid,
                                      uint2* __restrict__ big, uint32_t* n_big, uint2* __restrict__ huge,
                                      uint32_t* n_huge) {
     const uint32_t lane = threadIdx.x & 31;
@@ -153,6 +154,13 @@ __global__ void k_sort_small_buckets(const uint32_t* __restrict__ starts, uint64
         word |= __shfl_xor_sync(kFull, word, 2);
         word |= __shfl_xor_sync(kFull, word, 4);
         if ((lane & 7) == 0 && g0 < nb) occ[g0 >> 5] = word;
+        if (packed) {   // two lanes cover eight buckets
+            uint32_t sizes = 0;
+#pragma unroll
+            for (int k = 0; k < 4; k++) sizes |= n[k] < 15 ? n[k] << (4 * (4 * (lane & 1) + k)) : 0xffffffffu;
+            sizes |= __shfl_xor_sync(kFull, sizes, 1);
+            if ((lane & 1) == 0 && g0 < nb) packed[g0 >> 3] = make_uint2(s[0], sizes);
+        }
 #pragma unroll
         for (int k = 0; k < 4; k++) order_bucket(pos, s[k], n[k], mid, n_mid, big, n_big, huge, n_huge);
     }
@@ -248,7 +256,7 @@ void launch_window_records(const uint64_t* codes, const uint32_t* valid, uint64_
 
 gxy_status atomic_build_views(const gxy_dseq* seq, uint32_t n_views, const uint64_t* lo, const uint64_t* hi,
                               const Pattern& pat, uint32_t step, uint32_t* starts, uint32_t* positions,
-                              uint32_t* occ, uint32_t* first_host, Worker* W) {
+                              uint32_t* occ, uint2* packed, uint32_t* first_host, Worker* W) {
     cudaStream_t st = W->st;
     const uint64_t nw = 1ull << (2 * pat.weight);
     const uint64_t G = (uint64_t)n_views * nw;
@@ -299,7 +307,7 @@ gxy_status atomic_build_views(const gxy_dseq* seq, uint32_t n_views, const uint6
             views[v], pat, step, nwin[v], counts + (uint64_t)v * nw, positions);
     }
     count_launch(4);
-    k_sort_small_buckets<<<148 * 16, 256, 0, st>>>(starts, G, positions, occ, mid, ctr + 2, big, ctr, huge, ctr + 1);
+    k_sort_small_buckets<<<148 * 16, 256, 0, st>>>(starts, G, positions, occ, packed, mid, ctr + 2, big, ctr, huge, ctr + 1);
     k_sort_warp_buckets<<<148 * 4, 256, 0, st>>>(mid, ctr + 2, positions);
     k_sort_block_buckets<<<148 * 2, 256, 0, st>>>(big, ctr, positions);
     k_view_firsts<<<1, 256, 0, st>>>(starts, nw, n_views, first);

@@ -498,3 +498,38 @@ def test_filter_windows(gxy, ctx, pattern, n):
             sp = gxy.SearchParams(1, gxy.HspParams(400, 900), 1)
             g, o = both(gxy, ctx, t, bytes(q), pattern, sp)
             assert g == o, (i, t is target)
+
+
+@pytest.mark.parametrize("pattern,n,nq", [("111", 1 << 19, 60), ("1101", (1 << 19) + 40, 90), ("1" * 11, (1 << 19) + 9, 4000),
+                                          (P12, (1 << 19) + 17, 4000), (P12, (1 << 19) + 18, 4000),
+                                          ("11101100110010101111", 700_000, 4000), ("11101100110110101111", 700_000, 4000)])
+@pytest.mark.parametrize("transitions,mwc", [(0, 0), (1, 0), (2, 0), (1, 6), (2, 6)])
+def test_enumerate_tables(gxy, ctx, pattern, n, nq, transitions, mwc):
+    # Tables from 2^19 windows on, of weights 3 to 13, carry neighbour masks and
+    # packed bounds (buckets of 15 positions or more fall back to their starts), all
+    # others are looked up through the occupancy bits: weights 3, 4, 11, 12, 13 and 14,
+    # the last table without and the first one with masks, pruned and not; also in
+    # passes of 4,096 hits, where groups of a tile's variants wait for the next pass.
+    rng = np.random.default_rng(n + transitions)
+    t = bytearray(rand_ascii(rng, n - 300, b"ACGT") + b"A" * 150 + b"AC" * 75)
+    lo = int(rng.integers(0, n - 2 * nq))
+    q = bytearray(t[lo:lo + nq]) + t[-100:-60]
+    for i in rng.integers(0, len(q), len(q) // 12):
+        q[i] = b"ACGTNacgt"[rng.integers(9)]
+    sp = gxy.SearchParams(1, gxy.HspParams(910, 3000 if nq > 100 else 2000), transitions)
+    m = gxy.ScoringMatrix.hoxd70()
+    st = {}
+    g = gpu_search(gxy, ctx, bytes(t), bytes(q), pattern, sp, m, mwc, stats=st)
+    o, ost = oracle_search(bytes(t), bytes(q), pattern, m, sp, mwc)
+    assert as_tuples(g) == as_tuples(o)
+    if nq < 100:
+        return
+    c2 = gxy.Context(0)
+    try:
+        c2.set_tuning(max_hits_per_pass=4096)
+        st2 = {}
+        g2 = gpu_search(gxy, c2, bytes(t), bytes(q), pattern, sp, m, mwc, stats=st2)
+        assert g2.tobytes() == g.tobytes()
+        assert st2["raw_hits"] == st["raw_hits"] and st2["windows"] == st["windows"]
+    finally:
+        c2.close()
