@@ -339,12 +339,11 @@ gxy_status gxy_ctx_destroy(gxy_ctx* ctx) {
         DevBuf* bufs[] = {&w->prim_sums, &w->prim_hist, &w->counters, &w->d_units, &w->d_tsegs, &w->d_qsegs,
                           &w->ck0, &w->ck1, &w->cv0, &w->cv1, &w->cands, &w->flags, &w->offsets, &w->ohsp,
                           &w->rhsp, &w->runit, &w->rhsp2, &w->runit2, &w->perm, &w->perm2, &w->hits,
-                          &w->d_place, &w->rrec, &w->surv, &w->redo, &w->rk0, &w->rk1, &w->rv0, &w->rv1};
+                          &w->d_place, &w->rrec, &w->surv, &w->redo, &w->rc, &w->rc_items, &w->rk0, &w->rk1, &w->rv0, &w->rv1};
         for (DevBuf* b : bufs) b->release();
         if (w->gexec) cudaGraphExecDestroy(w->gexec);
         dseq_destroy(w->qstage);
         dseq_destroy(w->tstage);
-        for (gxy_dseq* d : w->rc_tmp) dseq_destroy(d);
         DevBuf* tb[] = {&w->tk0, &w->tv0, &w->tk1, &w->tv1, &w->tocc, &w->gpool, &w->gruns, &w->gaux, &w->gscr};
         for (DevBuf* b : tb) b->release();
         for (int i = 0; i < 5; i++)
@@ -698,9 +697,29 @@ static gxy_status batch_run(gxy_ctx* ctx, uint32_t n_tables, const gxy_table* co
     WorkerLease L(ctx);
     if (!L.w) return L.err;
     Worker* W = L.w;
-    // Reverse complements once per query that needs one.
-    for (gxy_dseq* d : W->rc_tmp) dseq_destroy(d);
-    W->rc_tmp.clear();
+    // Reverse complements once per query that needs one, all in one launch, in a
+    // buffer that the worker keeps unless it is more than twice (and 64 MB over) what
+    // this batch needs.
+    std::vector<char> want_rc(n_queries, 0);
+    size_t rc_bytes = 0;
+    uint32_t n_rc = 0;
+    for (uint32_t i = 0; i < n_units; i++) {
+        const uint32_t qi = units[i].query;
+        if (units[i].strand == 1 && !want_rc[qi]) {
+            want_rc[qi] = 1;
+            n_rc++;
+            rc_bytes += seq_layout(queries[qi]->len).bytes;
+        }
+    }
+    if (W->rc.bytes > 2 * rc_bytes + (64u << 20)) W->rc.release();
+    std::vector<RcItem> rc_items;
+    rc_items.reserve(n_rc);
+    uint64_t rc_blocks = 0;
+    size_t rc_at = 0;
+    if (n_rc) {
+        GXY_CK(W->rc.ensure(rc_bytes));
+        GXY_CK(W->rc_items.ensure(n_rc * sizeof(RcItem)));
+    }
     std::vector<int> qseg_of(2 * (size_t)n_queries, -1);
     std::vector<int> tseg_of(n_tables, -1);
     std::vector<SeqView> tsegs, qsegs;
@@ -715,15 +734,21 @@ static gxy_status batch_run(gxy_ctx* ctx, uint32_t n_tables, const gxy_table* co
         const size_t qi = 2 * (size_t)u.query + u.strand;
         if (qseg_of[qi] < 0) {
             const gxy_dseq* q = queries[u.query];
-            if (u.strand == 1) {
-                gxy_dseq* rc = nullptr;
-                API_TRY(dseq_alloc(ctx, q->len, &rc, W->st));
-                launch_reverse_complement(q->codes, q->valid, q->mask, q->len, rc->codes, rc->valid, rc->mask, W->st);
-                W->rc_tmp.push_back(rc);
-                q = rc;
-            }
             qseg_of[qi] = (int)qsegs.size();
             qsegs.push_back(view_of(q, 0, q->len));
+            if (u.strand == 1) {
+                const SeqLayout at = seq_layout(q->len);
+                char* p = W->rc.as<char>() + rc_at;
+                rc_items.push_back(RcItem{q->codes, q->valid, q->mask, q->len, reinterpret_cast<uint64_t*>(p),
+                                          reinterpret_cast<uint32_t*>(p + at.valid_at),
+                                          reinterpret_cast<uint32_t*>(p + at.mask_at), at.nwords, (uint32_t)rc_blocks});
+                SeqView& v = qsegs.back();
+                v.codes = rc_items.back().ocodes;
+                v.valid = rc_items.back().ovalid;
+                v.mask = rc_items.back().omask;
+                rc_at += at.bytes;
+                rc_blocks += (at.nwords + 255) / 256;
+            }
         }
         plan[i].tseg = (uint32_t)tseg_of[u.table];
         plan[i].qseg = (uint32_t)qseg_of[qi];
@@ -736,6 +761,14 @@ static gxy_status batch_run(gxy_ctx* ctx, uint32_t n_tables, const gxy_table* co
         plan[i].primary_lo = u.primary_lo;
         plan[i].primary_hi = u.primary_hi;
         plan[i].avg_bucket = t->num_words ? (double)t->npos / (double)t->num_words : 0.0;
+    }
+    if (n_rc) {
+        if (rc_blocks >= (1ull << 31)) {
+            set_error("the queries of one batch are too long to reverse-complement");
+            return GXY_EUNSUPPORTED;
+        }
+        GXY_CK(cudaMemcpyAsync(W->rc_items.p, rc_items.data(), n_rc * sizeof(RcItem), cudaMemcpyHostToDevice, W->st));
+        launch_reverse_complement_many(W->rc_items.as<RcItem>(), n_rc, (uint32_t)rc_blocks, W->st);
     }
     return run_units(ctx, W, plan, tsegs, qsegs, pat, *params, opts && opts->use_graph, r);
 }

@@ -53,16 +53,21 @@ void dev_free(void* p) {
     cudaStreamSynchronize(0);
 }
 
+SeqLayout seq_layout(uint64_t len) {
+    uint64_t nw = (kPad + len + kTailPad + 31) / 32;
+    nw = (nw + 3) & ~3ull;   // each array a multiple of 16 bytes
+    const size_t cb = align256(nw * 8), vb = align256(nw * 4);
+    return SeqLayout{nw, cb, cb + vb, cb + 2 * vb};
+}
+
 gxy_status dseq_alloc(gxy_ctx* ctx, uint64_t len, gxy_dseq** out, cudaStream_t st) {
     gxy_dseq* d = new gxy_dseq();
     d->ctx = ctx;
     d->device = ctx->device;
     d->len = len;
-    uint64_t nw = (kPad + len + kTailPad + 31) / 32;
-    nw = (nw + 3) & ~3ull;   // each array a multiple of 16 bytes
-    d->nwords = nw;
-    const size_t cb = align256(nw * 8), vb = align256(nw * 4);
-    d->bytes = cb + 2 * vb;
+    const SeqLayout at = seq_layout(len);
+    d->nwords = at.nwords;
+    d->bytes = at.bytes;
     cudaError_t e = dev_alloc(&d->alloc, d->bytes, st);
     if (e != cudaSuccess) {
         delete d;
@@ -71,8 +76,8 @@ gxy_status dseq_alloc(gxy_ctx* ctx, uint64_t len, gxy_dseq** out, cudaStream_t s
     }
     d->st = st;
     d->codes = static_cast<uint64_t*>(d->alloc);
-    d->valid = reinterpret_cast<uint32_t*>(static_cast<char*>(d->alloc) + cb);
-    d->mask = reinterpret_cast<uint32_t*>(static_cast<char*>(d->alloc) + cb + vb);
+    d->valid = reinterpret_cast<uint32_t*>(static_cast<char*>(d->alloc) + at.valid_at);
+    d->mask = reinterpret_cast<uint32_t*>(static_cast<char*>(d->alloc) + at.mask_at);
     e = cudaMemsetAsync(d->alloc, 0, d->bytes, st);
     if (e != cudaSuccess) {
         dev_free(d->alloc);
@@ -147,7 +152,7 @@ Worker* checkout(gxy_ctx* ctx, gxy_status* err) {
     for (DevBuf* b : {&w->tk0, &w->tv0, &w->tk1, &w->tv1, &w->prim_sums, &w->prim_hist, &w->counters, &w->d_units,
                       &w->d_tsegs, &w->d_qsegs, &w->ck0, &w->ck1, &w->cv0, &w->cv1, &w->cands, &w->flags,
                       &w->offsets, &w->ohsp, &w->rhsp, &w->runit, &w->rhsp2, &w->runit2, &w->perm, &w->perm2,
-                      &w->hits, &w->surv, &w->redo, &w->rk0, &w->rk1, &w->rv0, &w->rv1, &w->tocc,
+                      &w->hits, &w->surv, &w->redo, &w->rc, &w->rc_items, &w->rk0, &w->rk1, &w->rv0, &w->rv1, &w->tocc,
                       &w->gpool, &w->gruns, &w->gaux, &w->gscr})
         b->st = w->st;
     for (int i = 0; i < 5 && e == cudaSuccess; i++) e = cudaEventCreate(&w->ev[i]);

@@ -65,7 +65,7 @@ struct Worker {
     // Host-query staging for gxy_search.
     gxy_dseq* qstage = nullptr;
     gxy_dseq* tstage = nullptr;
-    std::vector<gxy_dseq*> rc_tmp;
+    DevBuf rc, rc_items;          // a batch's reverse complements and their list
 };
 
 // One unit as the engine plans it (host side).
@@ -190,6 +190,12 @@ void checkin(gxy_ctx* ctx, Worker* w);
 
 gxy_status dseq_alloc(gxy_ctx* ctx, uint64_t len, gxy_dseq** out, cudaStream_t st);
 void dseq_destroy(gxy_dseq* s);
+// A sequence's three arrays (words of each, bytes of all) as dseq_alloc lays them out.
+struct SeqLayout {
+    uint64_t nwords;
+    size_t valid_at, mask_at, bytes;
+};
+SeqLayout seq_layout(uint64_t len);
 // Frees in stream order on st: for sequences only st has used.
 void dseq_destroy_async(gxy_dseq* s, cudaStream_t st);
 gxy_status dseq_fill_host(gxy_dseq* d, const gxy_packed_seq* h, cudaStream_t st);

@@ -44,6 +44,21 @@ void launch_pack_ascii(const uint8_t* ascii, uint64_t n, uint64_t* codes, uint32
 void launch_reverse_complement(const uint64_t* icodes, const uint32_t* ivalid, const uint32_t* imask,
                                uint64_t n, uint64_t* ocodes, uint32_t* ovalid, uint32_t* omask,
                                cudaStream_t st);
+// The same for many sequences in one launch, pads and tails (zeros) included:
+// items on the device, in the order of their blocks; item i has
+// ceil(nwords / 256) of the n_blocks blocks, from block_base on.
+struct RcItem {
+    const uint64_t* icodes;
+    const uint32_t* ivalid;
+    const uint32_t* imask;
+    uint64_t n;
+    uint64_t* ocodes;
+    uint32_t* ovalid;
+    uint32_t* omask;
+    uint64_t nwords;
+    uint32_t block_base;
+};
+void launch_reverse_complement_many(const RcItem* items, uint32_t n_items, uint32_t n_blocks, cudaStream_t st);
 
 // --- table build (src/pos_table.rs:35-136) -----------------------------------
 // Seed words of the windows k*step of a view; key = word, or num_words for a

@@ -251,3 +251,27 @@ def test_epilogue_sizes(gxy, ctx, n_units, lo, hi, thresh):
     assert n_units == 1 or sum(len(w) for w in want) > 0   # (the single unit finds nothing: an empty sort)
     for u, (g, w) in enumerate(zip(got, want)):
         assert g.tobytes() == w.tobytes(), u
+
+
+@pytest.mark.parametrize("lens", [[0], [33], [0, 5, 19, 31, 32, 33, 64, 65], [7999, 8000, 8001, 8063, 8064, 8065, 8191, 8192, 8193],
+                                  [16_255, 40, 16_257, 0, 24_600, 31]])
+def test_batch_reverse_complements(gxy, ctx, lens):
+    # A batch's reverse complements are made by one launch, 256 words of one sequence
+    # a block: lengths around words and blocks, pieces of the target's own reverse
+    # complement, each both strands and the minus strand twice; a second call reuses
+    # the buffer that the first one filled with other lengths.
+    rng = np.random.default_rng(sum(lens))
+    target = rand_ascii(rng, 60_000, b"ACGTACGTacgtN")
+    comp = bytes.maketrans(b"ACGTacgt", b"TGCAtgca")
+    queries = []
+    for n in lens:
+        lo = int(rng.integers(0, len(target) - n))
+        queries.append(target[lo:lo + n].translate(comp)[::-1])
+    tab = gxy.PosTable.build(gxy.PackedSeq.from_ascii(target), P12, 1, ctx=ctx)
+    sp = gxy.SearchParams(1, gxy.HspParams(910, 1200), 1)
+    for qs in (queries, queries[::-1]):
+        dq = [gxy.DeviceSeq.from_ascii(q, ctx) for q in qs]
+        units = [(0, i, s) for i in range(len(qs)) for s in (1, 0, 1)]
+        got = gxy.batch_search([tab], dq, units, gxy.ScoringMatrix.hoxd70(), sp, ctx=ctx)
+        for u, (g, w) in enumerate(zip(got, oracle_units(target, qs, units, sp=O.params(hspthresh=1200)))):
+            assert g.tobytes() == w.tobytes(), u
