@@ -207,9 +207,11 @@ class DeviceSeq:
 
     def to_host(self) -> PackedSeq:
         n = self.length
-        c = np.zeros(max((n + 3) // 4, 1), np.uint8)
-        v = np.zeros(max((n + 7) // 8, 1), np.uint8)
-        m = np.zeros(max((n + 7) // 8, 1), np.uint8)
+        nc, nv = max((n + 3) // 4, 1), max((n + 7) // 8, 1)
+        # One allocation: numpy asks for huge pages from 4 MB on.
+        vo, mo = -(-nc // 64) * 64, -(-nc // 64) * 64 + -(-nv // 64) * 64
+        buf = np.zeros(mo + nv, np.uint8)
+        c, v, m = buf[:nc], buf[vo:vo + nv], buf[mo:]
         check(lib().gxy_dseq_download(self.h, c.ctypes.data, v.ctypes.data, m.ctypes.data))
         return PackedSeq(c, v, m, n)
 

@@ -355,6 +355,7 @@ gxy_status gxy_ctx_destroy(gxy_ctx* ctx) {
     }
     for (int i = 0; i < 16; i++)
         if (ctx->marks[i]) cudaEventDestroy(ctx->marks[i]);
+    ctx->copy.destroy();
     delete ctx;
     return GXY_OK;
 }
@@ -484,12 +485,12 @@ gxy_status gxy_dseq_download(const gxy_dseq* s, uint8_t* codes, uint8_t* valid, 
     API_TRY(set_device(s->ctx));
     const uint64_t n = s->len;
     if (!n) return GXY_OK;
-    if (codes) API_CK(cudaMemcpy(codes, reinterpret_cast<const char*>(s->codes) + kPad / 4, (n + 3) / 4,
-                                 cudaMemcpyDeviceToHost));
-    if (valid) API_CK(cudaMemcpy(valid, reinterpret_cast<const char*>(s->valid) + kPad / 8, (n + 7) / 8,
-                                 cudaMemcpyDeviceToHost));
-    if (mask) API_CK(cudaMemcpy(mask, reinterpret_cast<const char*>(s->mask) + kPad / 8, (n + 7) / 8,
-                                cudaMemcpyDeviceToHost));
+    CopyPiece pieces[3];
+    int k = 0;
+    if (codes) pieces[k++] = {codes, reinterpret_cast<char*>(s->codes) + kPad / 4, (n + 3) / 4};
+    if (valid) pieces[k++] = {valid, reinterpret_cast<char*>(s->valid) + kPad / 8, (n + 7) / 8};
+    if (mask) pieces[k++] = {mask, reinterpret_cast<char*>(s->mask) + kPad / 8, (n + 7) / 8};
+    API_CK(host_copy(s->ctx, pieces, k, true, 0));
     return GXY_OK;
 }
 

@@ -104,12 +104,11 @@ void dseq_destroy(gxy_dseq* s) {
 gxy_status dseq_fill_host(gxy_dseq* d, const gxy_packed_seq* h, cudaStream_t st) {
     const uint64_t n = h->len;
     if (!n) return GXY_OK;
-    GXY_CK(cudaMemcpyAsync(reinterpret_cast<char*>(d->codes) + kPad / 4, h->codes, (n + 3) / 4,
-                           cudaMemcpyHostToDevice, st));
-    GXY_CK(cudaMemcpyAsync(reinterpret_cast<char*>(d->valid) + kPad / 8, h->valid, (n + 7) / 8,
-                           cudaMemcpyHostToDevice, st));
-    GXY_CK(cudaMemcpyAsync(reinterpret_cast<char*>(d->mask) + kPad / 8, h->mask, (n + 7) / 8,
-                           cudaMemcpyHostToDevice, st));
+    const CopyPiece pieces[3] = {
+        {const_cast<uint8_t*>(h->codes), reinterpret_cast<char*>(d->codes) + kPad / 4, (n + 3) / 4},
+        {const_cast<uint8_t*>(h->valid), reinterpret_cast<char*>(d->valid) + kPad / 8, (n + 7) / 8},
+        {const_cast<uint8_t*>(h->mask), reinterpret_cast<char*>(d->mask) + kPad / 8, (n + 7) / 8}};
+    GXY_CK(host_copy(d->ctx, pieces, 3, false, st));
     return GXY_OK;
 }
 

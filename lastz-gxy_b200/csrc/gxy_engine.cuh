@@ -2,10 +2,13 @@
 // entry points.
 #pragma once
 
+#include <condition_variable>
 #include <cstdint>
+#include <functional>
 #include <memory>
 #include <mutex>
 #include <string>
+#include <thread>
 #include <vector>
 
 #include <cuda_runtime.h>
@@ -166,6 +169,30 @@ struct gxy_table {
     uint64_t hlen = 0;
 };
 
+namespace gxy {
+// Pinned halves, streams, events and helper threads of copies to and from
+// pageable host memory.  One copy at a time holds mu; the helpers sleep on cv and
+// run job(1 .. n_job - 1) of each generation.
+constexpr int kCopyThreads = 8;
+struct HostCopy {
+    std::mutex mu;
+    char* pinned = nullptr;
+    cudaStream_t st[kCopyThreads] = {};
+    cudaEvent_t ev[kCopyThreads][2] = {};
+    std::thread helper[kCopyThreads];
+    int n_helpers = 0;
+    std::mutex job_mu;
+    std::condition_variable cv, cv_done;
+    const std::function<void(int)>* job = nullptr;
+    uint64_t generation = 0;
+    int n_job = 0, running = 0;
+    bool stop = false;
+    void run(const std::function<void(int)>& f, int threads);   // f(0) here, f(1 .. threads - 1) on helpers
+    void help(int me, int device);
+    void destroy();
+};
+}  // namespace gxy
+
 struct gxy_ctx {
     int device = 0;
     int sm_count = 148;
@@ -177,6 +204,7 @@ struct gxy_ctx {
     // re-extend (two searches 4.27 ms, against 4.31 ms at 128 and 4.51 at 64).
     gxy_tuning tuning{8, 192, 4, 8, 256u << 20, 0, 96, 1, 0, 4};
     cudaEvent_t marks[16] = {};
+    gxy::HostCopy copy;
 };
 
 namespace gxy {
@@ -196,6 +224,17 @@ struct SeqLayout {
     size_t valid_at, mask_at, bytes;
 };
 SeqLayout seq_layout(uint64_t len);
+// Copies pieces after what st holds; to the host it is done on return, to the
+// device the host memory is read (or staged by the driver) on return and st's later
+// work comes after it.  seen(lo, hi), if given, is called for the ranges of a
+// single piece to the device, in no order and from several threads.
+struct CopyPiece {
+    void* host;
+    void* dev;
+    size_t bytes;
+};
+cudaError_t host_copy(gxy_ctx* ctx, const CopyPiece* pieces, int n, bool to_host, cudaStream_t st,
+                      const std::function<void(size_t, size_t)>& seen = {});
 // Frees in stream order on st: for sequences only st has used.
 void dseq_destroy_async(gxy_dseq* s, cudaStream_t st);
 gxy_status dseq_fill_host(gxy_dseq* d, const gxy_packed_seq* h, cudaStream_t st);

@@ -16,6 +16,7 @@
 // T/C/A/G/N/t/c/a/g).
 #include <algorithm>
 #include <cstring>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -201,48 +202,69 @@ gxy_status gxy_parse_fasta(gxy_ctx* ctx, const uint8_t* bytes, uint64_t n, gxy_s
     // Header lines: a line (split at LF) whose first byte is '>' (src/sequences.rs:354).
     // Line i starts after the i-th LF.  Empty lines are skipped by the
     // reference; they hold no bytes here either.
-    std::vector<uint64_t> hdr;          // header line [start, end) pairs, end excludes the LF
-    std::vector<std::string> names;
-    for (uint64_t pos = 0; pos < n;) {
-        const void* gt = memchr(bytes + pos, '>', n - pos);
-        if (!gt) break;
-        const uint64_t i = static_cast<const uint8_t*>(gt) - bytes;
-        if (i == 0 || bytes[i - 1] == '\n') {
-            const void* lf = memchr(bytes + i, '\n', n - i);
-            const uint64_t e = lf ? (uint64_t)(static_cast<const uint8_t*>(lf) - bytes) : n;
-            // The name: the first whitespace-delimited token after '>'.
-            uint64_t a = i + 1;
-            auto ws = [](uint8_t c) { return c == ' ' || c == '\t' || c == '\n' || c == '\f' || c == '\r'; };
-            while (a < e && ws(bytes[a])) a++;
-            uint64_t b = a;
-            while (b < e && !ws(bytes[b])) b++;
-            if (b == a) {
-                uint64_t line = 1;
-                for (uint64_t k = 0; k < i; k++) line += bytes[k] == '\n';
-                set_error("empty FASTA header at line " + std::to_string(line) + " (src/sequences.rs:357-361)");
-                return GXY_EINVAL;
-            }
-            names.emplace_back(reinterpret_cast<const char*>(bytes + a), b - a);
-            hdr.push_back(i);
-            hdr.push_back(e);
-            pos = e;
-        } else {
-            pos = i + 1;
-        }
-    }
-    const uint64_t nrec = names.size();
-    if (alloc_set(out, nrec) != GXY_OK) return fail_set(out, "host allocation of the sequence set", GXY_ENOMEM);
-    for (uint64_t r = 0; r < nrec; r++) {
-        out->names[r] = dup_name(reinterpret_cast<const uint8_t*>(names[r].data()), names[r].size());
-        if (!out->names[r]) return fail_set(out, "host allocation of FASTA names", GXY_ENOMEM);
-    }
-    if (nrec == 0) return GXY_OK;   // no header: the reference returns no sequences
+    // Line starts with a '>' are looked for while the bytes go to the device.
+    uint8_t* dbytes = nullptr;
     WorkerLease L(ctx);
-    if (!L.w) return fail_set(out, "no worker", L.err);
+    if (!L.w) return L.err;
     Worker* W = L.w;
     cudaStream_t st = W->st;
+    auto failed = [&](gxy_status s) {
+        if (dbytes) cudaFreeAsync(dbytes, st);
+        cudaStreamSynchronize(st);
+        return s;
+    };
+    std::vector<uint64_t> at;
+    std::mutex at_mu;
+    auto scan = [&](size_t lo, size_t hi) {
+        std::vector<uint64_t> mine;
+        for (uint64_t pos = lo; pos < hi;) {
+            const void* gt = memchr(bytes + pos, '>', hi - pos);
+            if (!gt) break;
+            const uint64_t i = static_cast<const uint8_t*>(gt) - bytes;
+            if (i == 0 || bytes[i - 1] == '\n') mine.push_back(i);
+            pos = i + 1;
+        }
+        std::lock_guard<std::mutex> g(at_mu);
+        at.insert(at.end(), mine.begin(), mine.end());
+    };
+    cudaError_t e = cudaMallocAsync((void**)&dbytes, std::max<uint64_t>(n, 1), st);
+    const CopyPiece piece{const_cast<uint8_t*>(bytes), dbytes, n};
+    if (e == cudaSuccess) e = host_copy(ctx, &piece, 1, false, st, scan);
+    if (e != cudaSuccess) {
+        set_error(std::string("FASTA bytes to the device: ") + cudaGetErrorString(e));
+        return failed(e == cudaErrorMemoryAllocation ? GXY_ENOMEM : GXY_ECUDA);
+    }
+    std::sort(at.begin(), at.end());
+    std::vector<uint64_t> hdr;          // header line [start, end) pairs, end excludes the LF
+    std::vector<std::string> names;
+    for (const uint64_t i : at) {
+        const void* lf = memchr(bytes + i, '\n', n - i);
+        const uint64_t end = lf ? (uint64_t)(static_cast<const uint8_t*>(lf) - bytes) : n;
+        // The name: the first whitespace-delimited token after '>'.
+        uint64_t a = i + 1;
+        auto ws = [](uint8_t c) { return c == ' ' || c == '\t' || c == '\n' || c == '\f' || c == '\r'; };
+        while (a < end && ws(bytes[a])) a++;
+        uint64_t b = a;
+        while (b < end && !ws(bytes[b])) b++;
+        if (b == a) {
+            uint64_t line = 1;
+            for (uint64_t k = 0; k < i; k++) line += bytes[k] == '\n';
+            set_error("empty FASTA header at line " + std::to_string(line) + " (src/sequences.rs:357-361)");
+            return failed(GXY_EINVAL);
+        }
+        names.emplace_back(reinterpret_cast<const char*>(bytes + a), b - a);
+        hdr.push_back(i);
+        hdr.push_back(end);
+    }
+    const uint64_t nrec = names.size();
+    if (alloc_set(out, nrec) != GXY_OK) return failed(fail_set(out, "host allocation of the sequence set", GXY_ENOMEM));
+    for (uint64_t r = 0; r < nrec; r++) {
+        out->names[r] = dup_name(reinterpret_cast<const uint8_t*>(names[r].data()), names[r].size());
+        if (!out->names[r]) return failed(fail_set(out, "host allocation of FASTA names", GXY_ENOMEM));
+    }
+    if (nrec == 0) return failed(GXY_OK);   // no header: the reference returns no sequences
     // Device buffers: file bytes, keep flags, offsets, compacted bases.
-    uint8_t *dbytes = nullptr, *dkeep = nullptr, *dcomp = nullptr;
+    uint8_t *dkeep = nullptr, *dcomp = nullptr;
     uint32_t* doff = nullptr;
     uint64_t* dhdr = nullptr;
     uint64_t* dat = nullptr;
@@ -257,8 +279,7 @@ gxy_status gxy_parse_fasta(gxy_ctx* ctx, const uint8_t* bytes, uint64_t n, gxy_s
         cudaFreeAsync(dbound, st);
         cudaStreamSynchronize(st);
     };
-    cudaError_t e = cudaMallocAsync((void**)&dbytes, n, st);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&dkeep, n, st);
+    e = cudaMallocAsync((void**)&dkeep, n, st);
     if (e == cudaSuccess) e = cudaMallocAsync((void**)&dcomp, n, st);
     if (e == cudaSuccess) e = cudaMallocAsync((void**)&doff, (n + 1) * 4, st);
     if (e == cudaSuccess) e = cudaMallocAsync((void**)&dhdr, hdr.size() * 8, st);
@@ -270,12 +291,10 @@ gxy_status gxy_parse_fasta(gxy_ctx* ctx, const uint8_t* bytes, uint64_t n, gxy_s
     }
     // Record r's bases are those kept in [boundary r, boundary r + 1): record
     // 0 also takes bases before the first header, as the reference does.
-    std::vector<uint64_t> at(nrec + 1);
-    at[0] = 0;
+    at.assign(nrec + 1, 0);
     for (uint64_t r = 1; r < nrec; r++) at[r] = hdr[2 * r];
     at[nrec] = n;
-    e = cudaMemcpyAsync(dbytes, bytes, n, cudaMemcpyHostToDevice, st);
-    if (e == cudaSuccess) e = cudaMemcpyAsync(dhdr, hdr.data(), hdr.size() * 8, cudaMemcpyHostToDevice, st);
+    e = cudaMemcpyAsync(dhdr, hdr.data(), hdr.size() * 8, cudaMemcpyHostToDevice, st);
     if (e == cudaSuccess) e = cudaMemcpyAsync(dat, at.data(), at.size() * 8, cudaMemcpyHostToDevice, st);
     const int grid = ctx->sm_count * 8;
     if (e == cudaSuccess) {
@@ -361,6 +380,15 @@ gxy_status gxy_parse_2bit(gxy_ctx* ctx, const uint8_t* bytes, uint64_t n, gxy_se
     WorkerLease L(ctx);
     if (!L.w) return fail_set(out, "no worker", L.err);
     cudaStream_t st = L.w->st;
+    // The structure of all records first; their packed bases go to the device together.
+    struct Rec {
+        uint32_t i;
+        const uint8_t* packed;
+        uint64_t pb, pk_at, rng_at, nn, nm;
+    };
+    std::vector<Rec> recs;
+    std::vector<uint32_t> rng;
+    uint64_t pk_bytes = 0;
     for (uint32_t i = 0; i < count; i++) {
         Reader q{bytes, n, 0, be};
         if (index[i].second > n) {
@@ -404,29 +432,35 @@ gxy_status gxy_parse_2bit(gxy_ctx* ctx, const uint8_t* bytes, uint64_t n, gxy_se
             return s;
         }
         if (dna == 0) continue;
-        uint8_t* dpk = nullptr;
-        uint32_t* drng = nullptr;
-        cudaError_t e = cudaMallocAsync((void**)&dpk, pb, st);
-        if (e == cudaSuccess) e = cudaMallocAsync((void**)&drng, (nr.size() + mr.size() + 2) * 4, st);
-        if (e == cudaSuccess) e = cudaMemcpyAsync(dpk, packed, pb, cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess && !nr.empty())
-            e = cudaMemcpyAsync(drng, nr.data(), nr.size() * 4, cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess && !mr.empty())
-            e = cudaMemcpyAsync(drng + nr.size(), mr.data(), mr.size() * 4, cudaMemcpyHostToDevice, st);
-        if (e == cudaSuccess) {
-            gxy_dseq* d = out->seqs[i];
-            const uint64_t nw = (dna + 31) / 32;
-            count_launch();
-            k_2bit_decode<<<(unsigned)std::min<uint64_t>((nw + 255) / 256, (uint64_t)ctx->sm_count * 16), 256, 0,
-                            st>>>(dpk, dna, drng, (uint32_t)(nr.size() / 2), drng + nr.size(),
-                                  (uint32_t)(mr.size() / 2), d->codes, d->valid, d->mask);
-            e = cudaStreamSynchronize(st);   // the host buffers of this record die here
-        }
-        cudaFreeAsync(dpk, st);
-        cudaFreeAsync(drng, st);
-        if (e == cudaSuccess) e = cudaGetLastError();
-        if (e != cudaSuccess) return fail_set(out, std::string("2bit decode: ") + cudaGetErrorString(e), GXY_ECUDA);
+        recs.push_back(Rec{i, packed, pb, pk_bytes, rng.size(), nr.size(), mr.size()});
+        pk_bytes += (pb + 255) & ~(uint64_t)255;
+        rng.insert(rng.end(), nr.begin(), nr.end());
+        rng.insert(rng.end(), mr.begin(), mr.end());
     }
+    if (recs.empty()) return cudaStreamSynchronize(st) == cudaSuccess ? GXY_OK : fail_set(out, "2bit decode", GXY_ECUDA);
+    uint8_t* dpk = nullptr;
+    uint32_t* drng = nullptr;
+    cudaError_t e = cudaMallocAsync((void**)&dpk, pk_bytes, st);
+    if (e == cudaSuccess) e = cudaMallocAsync((void**)&drng, (rng.size() + 2) * 4, st);
+    std::vector<CopyPiece> pieces;
+    for (const Rec& x : recs) pieces.push_back({const_cast<uint8_t*>(x.packed), dpk + x.pk_at, x.pb});
+    if (e == cudaSuccess) e = host_copy(ctx, pieces.data(), (int)pieces.size(), false, st);
+    if (e == cudaSuccess && !rng.empty()) e = cudaMemcpyAsync(drng, rng.data(), rng.size() * 4, cudaMemcpyHostToDevice, st);
+    for (const Rec& x : recs) {
+        if (e != cudaSuccess) break;
+        gxy_dseq* d = out->seqs[x.i];
+        const uint64_t nw = (d->len + 31) / 32;
+        count_launch();
+        k_2bit_decode<<<(unsigned)std::min<uint64_t>((nw + 255) / 256, (uint64_t)ctx->sm_count * 16), 256, 0, st>>>(
+            dpk + x.pk_at, d->len, drng + x.rng_at, (uint32_t)(x.nn / 2), drng + x.rng_at + x.nn, (uint32_t)(x.nm / 2),
+            d->codes, d->valid, d->mask);
+    }
+    const cudaError_t synced = cudaStreamSynchronize(st);   // the host buffers die here
+    if (e == cudaSuccess) e = synced;
+    if (dpk) cudaFreeAsync(dpk, st);
+    if (drng) cudaFreeAsync(drng, st);
+    if (e == cudaSuccess) e = cudaGetLastError();
+    if (e != cudaSuccess) return fail_set(out, std::string("2bit decode: ") + cudaGetErrorString(e), GXY_ECUDA);
     if (cudaStreamSynchronize(st) != cudaSuccess) return fail_set(out, "2bit decode", GXY_ECUDA);
     return GXY_OK;
 }

@@ -103,3 +103,43 @@ def test_2bit_errors(gxy, ctx, bad):
         data = bytes(data)
     with pytest.raises(gxy.GxyError):
         gxy.parse_2bit(data, ctx)
+
+
+@pytest.mark.parametrize("n", [(2 << 20) - 1, 2 << 20, (2 << 20) + 1, 5 * (1 << 19), 9_000_007])
+def test_large_copies(gxy, ctx, n):
+    # From 2 MB on, host memory is copied in chunks of 512 KB by several threads,
+    # which also look for the header lines: a FASTA file of n bytes with a header
+    # around every other chunk's end and a '>' inside lines, the sequences' way back
+    # and up again, and four threads at a time, of which one finds the pinned halves free.
+    import threading
+    rng = np.random.default_rng(n)
+    buf = bytearray(rand_ascii(rng, n, b"ACGTacgtN"))
+    buf[60::61] = b"\n" * len(range(60, n, 61))
+    buf[:9] = b">a first\n"
+    for k, c in enumerate(range(1 << 19, n - 40, 1 << 19)):
+        at = c - 8 + 3 * k % 16
+        buf[at:at + 16] = b"\n>r%06d x>y z\n" % k if k % 2 == 0 else b"ACGT>ACGTNNNACGT"
+    data = bytes(buf)
+    want = O.parse_fasta(data)
+    seqs = gxy.parse_fasta(data, ctx)
+    same(gxy, seqs, want)
+    big = max((d for _, d in seqs), key=lambda d: d.length)
+    one = gxy.DeviceSeq.from_ascii(data.replace(b"\n", b""), ctx)
+    host = one.to_host()
+    back = host.to_device(ctx).to_host()
+    for a, b in ((host.codes, back.codes), (host.valid, back.valid), (host.mask, back.mask)):
+        assert np.array_equal(a, b)
+    ref = big.to_host()
+    got = [None] * 4
+
+    def work(i):
+        h = host.to_device(ctx).to_host()
+        got[i] = (np.array_equal(h.codes, host.codes) and np.array_equal(h.valid, host.valid)
+                  and np.array_equal(h.mask, host.mask) and np.array_equal(big.to_host().codes, ref.codes))
+
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(4)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert got == [True] * 4
