@@ -86,17 +86,21 @@ __device__ __forceinline__ void f_scan2(FSide& R, uint32_t r0, uint32_t r1, FSid
 }
 
 __device__ __forceinline__ void lut_fill(unsigned char* lut, const int32_t* fub) {
-    for (uint32_t i = threadIdx.x; i < 2u * 256u * 32u; i += blockDim.x) {
-        const uint32_t b = (i >> 5) & 255u;
-        const bool down = i >> 13;
-        int32_t p = 0, mp = INT32_MIN;
+    // Sixteen entries a warp, one a lane, then each to all 32 copies.  (With every
+    // lane forming the entry it stored, this took 12 us of a block.)
+    static_assert(kFilterWarps * 16 == 512, "two tables of 256 entries");
+    const uint32_t lane = threadIdx.x & 31, e0 = (threadIdx.x >> 5) * 16;
+    const uint32_t b = (e0 + (lane & 15)) & 255u;
+    const bool down = e0 >> 8;
+    int32_t p = 0, mp = INT32_MIN;
 #pragma unroll
-        for (int c = 0; c < 4; c++) {
-            p += fub[(b >> (2 * (down ? 3 - c : c))) & 3u];
-            mp = max(mp, p);
-        }
-        reinterpret_cast<int2*>(lut)[i] = make_int2(p, mp);
+    for (int c = 0; c < 4; c++) {
+        p += fub[(b >> (2 * (down ? 3 - c : c))) & 3u];
+        mp = max(mp, p);
     }
+#pragma unroll
+    for (uint32_t k = 0; k < 16; k++)
+        reinterpret_cast<int2*>(lut)[(e0 + k) * 32 + lane] = make_int2(__shfl_sync(kFull, p, k), __shfl_sync(kFull, mp, k));
 }
 
 // The seed footprint's bound: all L columns from column 0 of x (src/hsp.rs:119-123).

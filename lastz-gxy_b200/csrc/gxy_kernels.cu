@@ -407,15 +407,16 @@ __global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(cons
     const int lane = threadIdx.x & 31;
     const uint32_t n_bytes = (a.pat.len + 3) / 4, weight = a.pat.weight;
     if (threadIdx.x < 2) s_stats[threadIdx.x] = 0;
-    for (uint32_t i = threadIdx.x; i < n_bytes * 256; i += blockDim.x) {
+    static_assert(kEnumWarps * 32 == 256, "a thread a byte value");
+    for (uint32_t x = 0; x < n_bytes; x++) {
         uint32_t w = 0;
 #pragma unroll
-        for (uint32_t c = 0; c < 4; c++) {
-            const uint32_t pos = 4 * (i >> 8) + c;
+        for (uint32_t c = 0; c < 4; c++) {   // (the shifts are the block's, not the thread's)
+            const uint32_t pos = 4 * x + c;
             if ((a.pat.care_mask >> pos) & 1u)
-                w |= ((i >> (2 * c)) & 3u) << (2 * (weight - 1 - __popc(a.pat.care_mask & ((1u << pos) - 1u))));
+                w |= ((threadIdx.x >> (2 * c)) & 3u) << (2 * (weight - 1 - __popc(a.pat.care_mask & ((1u << pos) - 1u))));
         }
-        s_word[i >> 8][i & 255] = w;
+        s_word[x][threadIdx.x] = w;
     }
     __syncthreads();
     uint32_t* const ent = s_ent[threadIdx.x >> 5];
@@ -1006,30 +1007,6 @@ __device__ __forceinline__ void pk_step(PkSide& S, int32_t T, const int32_t* plu
     S.b = max(S.b, S.p);
 }
 
-// Column k of a side that cannot break yet (no x-drop test).
-template <int k>
-__device__ __forceinline__ void pk_step_free(PkSide& S, const int32_t* plut) {
-    const uint32_t idx = (uint32_t)(((k & 1) ? S.o : S.e) >> (4 * (k >> 1))) & 15u;
-    S.p += plut[idx];
-    S.b = max(S.b, S.p);
-}
-
-// The fast path with side B fresh: its first kFree columns cannot reach the
-// x-drop (each column lowers p by at most 256 * |min score| + 1), so they skip
-// the test.  A dead B (no columns) is updated too, but its result is unused.
-template <int kFree>
-__device__ __forceinline__ void pk_scan_pair_bfresh(PkSide& A, PkSide& B, int32_t T, const int32_t* plut,
-                                                    int32_t pamb) {
-#define GXY_PKF(k)                                                         \
-    pk_step<false, k>(A, T, plut, pamb);                                   \
-    if (k < kFree) pk_step_free<k>(B, plut); else pk_step<false, k>(B, T, plut, pamb);
-    GXY_PKF(0) GXY_PKF(1) GXY_PKF(2) GXY_PKF(3) GXY_PKF(4) GXY_PKF(5) GXY_PKF(6) GXY_PKF(7)
-    GXY_PKF(8) GXY_PKF(9) GXY_PKF(10) GXY_PKF(11) GXY_PKF(12) GXY_PKF(13) GXY_PKF(14) GXY_PKF(15)
-    GXY_PKF(16) GXY_PKF(17) GXY_PKF(18) GXY_PKF(19) GXY_PKF(20) GXY_PKF(21) GXY_PKF(22) GXY_PKF(23)
-    GXY_PKF(24) GXY_PKF(25) GXY_PKF(26) GXY_PKF(27) GXY_PKF(28) GXY_PKF(29) GXY_PKF(30) GXY_PKF(31)
-#undef GXY_PKF
-}
-
 // Both sides column by column in lockstep: two independent serial chains.
 template <bool kSlow>
 __device__ __forceinline__ void pk_scan_pair(PkSide& A, PkSide& B, int32_t T, const int32_t* plut, int32_t pamb) {
@@ -1055,20 +1032,20 @@ __device__ __forceinline__ uint64_t funnel64(uint64_t lo, uint64_t hi, uint32_t 
     return s ? ((lo >> s) | (hi << (64 - s))) : lo;
 }
 
-// Seed footprint score, all L columns at t / q (src/hsp.rs:119-123): three
-// columns per table read, the rest singly, invalid columns re-scored ambig.
+// Seed footprint score, all L columns at t / q (src/hsp.rs:119-123): two
+// columns per table read, an odd last one singly, invalid columns re-scored ambig.
 __device__ __forceinline__ int32_t seed_score(const SeqView& T, const SeqView& Q, uint32_t t, uint32_t q,
-                                              uint32_t L, uint32_t seed_mask, const int32_t* s_tri,
+                                              uint32_t L, uint32_t seed_mask, const int32_t* s_duo,
                                               const int32_t* s_lut, int32_t ambig) {
     const uint64_t tc = load_codes32(T.codes, T.base + t), qc = load_codes32(Q.codes, Q.base + q);
     const uint32_t vv = load_bits32(T.valid, T.base + t) & load_bits32(Q.valid, Q.base + q);
     int32_t sd = 0;
 #pragma unroll
-    for (int k = 0; k + 3 <= 32; k += 3) {
-        if ((uint32_t)k + 3 > L) break;
-        sd += s_tri[((((uint32_t)(tc >> (2 * k))) & 63u) << 6) | ((uint32_t)(qc >> (2 * k)) & 63u)];
+    for (int k = 0; k < 32; k += 2) {
+        if ((uint32_t)k + 2 > L) break;
+        sd += s_duo[((((uint32_t)(tc >> (2 * k))) & 15u) << 4) | ((uint32_t)(qc >> (2 * k)) & 15u)];
     }
-    for (uint32_t k = L - L % 3; k < L; k++)
+    for (uint32_t k = L & ~1u; k < L; k++)
         sd += s_lut[((((uint32_t)(tc >> (2 * k))) & 3u) << 2) | ((uint32_t)(qc >> (2 * k)) & 3u)];
     uint32_t bad = ~vv & seed_mask;
     while (bad) {
@@ -1083,13 +1060,9 @@ template <int WARPS, int MINB>
 __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen(const __grid_constant__ ScreenArgs a) {
     __shared__ int32_t s_lut[16];     // raw column scores, index (t << 2) | q
     __shared__ int32_t s_plut[16];    // 256 * score - 1, index (q << 2) | t
-    __shared__ int32_t s_tri[4096];   // sum of three columns' scores, index (t3 << 6) | q3
-    for (uint32_t i = threadIdx.x; i < 4096; i += blockDim.x) {
-        int32_t v = 0;
-#pragma unroll
-        for (int c = 0; c < 3; c++) v += a.sc.sub[(((i >> (6 + 2 * c)) & 3u) << 2) | ((i >> (2 * c)) & 3u)];
-        s_tri[i] = v;
-    }
+    __shared__ int32_t s_duo[256];    // sum of two columns' scores, index (t2 << 4) | q2
+    for (uint32_t i = threadIdx.x; i < 256; i += blockDim.x)
+        s_duo[i] = a.sc.sub[((i >> 4 & 3u) << 2) | (i & 3u)] + a.sc.sub[((i >> 6 & 3u) << 2) | (i >> 2 & 3u)];
     if (threadIdx.x < 16) {
         s_lut[threadIdx.x] = a.sc.sub[threadIdx.x];
         s_plut[threadIdx.x] = a.sc.sub[((threadIdx.x & 3u) << 2) | (threadIdx.x >> 2)] * 256 - 1;
@@ -1101,11 +1074,6 @@ __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen(const __grid_consta
     const int32_t ambig = a.sc.ambig, thresh = a.sc.hspthresh;
     const int32_t pamb = ambig * 256 - 1;
     const int32_t T = (a.sc.xdrop + 1) * 256;
-    // Columns a fresh side scans before its first possible break.
-    int32_t worst = a.sc.ambig;
-    for (int i = 0; i < 16; i++) worst = min(worst, a.sc.sub[i]);
-    const int32_t per_col = worst < 0 ? 256 * (-worst) + 1 : 1;
-    const int free_cols = (int)min(8, (T - 1) / per_col);
     const uint32_t seed_mask = L >= 32 ? 0xffffffffu : ((1u << L) - 1u);
     // No seed footprint scores above this: a hit whose two sides' bests stay
     // below thresh - seed_ub can never pass, whatever its seed scores.
@@ -1179,13 +1147,11 @@ __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen(const __grid_consta
         }
 
         // ---------------- chunk data ----------------
-        // Side A: the next chunk of the side this hit is on (a fresh hit's
-        // first right chunk); side B: a fresh hit's first left chunk.  Right
-        // chunks read forward from the column after the last one scanned,
-        // left chunks the 32 positions below it, reversed.
+        // The next chunk of each side that still runs: A right, forward from the
+        // column after the last one scanned, B left, the 32 positions below it,
+        // reversed.
         uint64_t atc = 0, aqc = 0, btc = 0, bqc = 0;
         uint32_t avv = 0, bvv = 0, an = 0, bn = 0;
-        const bool a_right = fresh || !rdone;
         if (fresh) {
             rrem = min(T_.len - ht - L, Q_.len - hq - L);
             lrem = min(ht, hq);
@@ -1193,22 +1159,17 @@ __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen(const __grid_consta
             rdone = rrem == 0;
             ldone = lrem == 0;
         }
-        if (busy) {
-            const uint32_t ext = pk_ext(a_right ? rp : lp);
-            const uint64_t ta = a_right ? T_.base + ht + L + ext : T_.base + ht - ext - 32;
-            const uint64_t qa = a_right ? Q_.base + hq + L + ext : Q_.base + hq - ext - 32;
+        if (busy && !rdone) {
+            const uint32_t ext = pk_ext(rp);
+            const uint64_t ta = T_.base + ht + L + ext, qa = Q_.base + hq + L + ext;
             atc = load_codes32(T_.codes, ta);
             aqc = load_codes32(Q_.codes, qa);
             avv = load_bits32(T_.valid, ta) & load_bits32(Q_.valid, qa);
-            if (!a_right) {
-                atc = rev_pairs64(atc);
-                aqc = rev_pairs64(aqc);
-                avv = __brev(avv);
-            }
-            an = min(32u, a_right ? rrem : lrem);
+            an = min(32u, rrem);
         }
-        if (fresh) {
-            const uint64_t tb = T_.base + ht - 32, qb = Q_.base + hq - 32;
+        if (busy && !ldone) {
+            const uint32_t ext = pk_ext(lp);
+            const uint64_t tb = T_.base + ht - ext - 32, qb = Q_.base + hq - ext - 32;
             btc = rev_pairs64(load_codes32(T_.codes, tb));
             bqc = rev_pairs64(load_codes32(Q_.codes, qb));
             bvv = __brev(load_bits32(T_.valid, tb) & load_bits32(Q_.valid, qb));
@@ -1218,25 +1179,18 @@ __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen(const __grid_consta
         // ---------------- scans ----------------
         {
             PkSide A, B;
-            const int32_t a0 = a_right ? rp : lp;
-            pk_init(A, atc, aqc, avv, an, a0, a_right ? rb : lb, T);
+            pk_init(A, atc, aqc, avv, an, rp, rb, T);
             pk_init(B, btc, bqc, bvv, bn, lp, lb, T);
             const bool slow = (an != 0 && (an < 32 || avv != 0xffffffffu)) ||
                               (bn != 0 && (bn < 32 || bvv != 0xffffffffu));
             if (__any_sync(kFull, slow)) pk_scan_pair<true>(A, B, T, s_plut, pamb);
-            else if (free_cols >= 7) pk_scan_pair_bfresh<7>(A, B, T, s_plut, pamb);
             else pk_scan_pair<false>(A, B, T, s_plut, pamb);
             if (an) {
-                const uint32_t used = ((uint32_t)a0 & 255u) - ((uint32_t)A.p & 255u);
+                const uint32_t used = ((uint32_t)rp & 255u) - ((uint32_t)A.p & 255u);
                 const bool end = A.b - A.p >= T;
                 n_cols += used;
-                if (a_right) {
-                    rp = A.p; rb = A.b; rrem -= used;
-                    rdone = end || rrem == 0;
-                } else {
-                    lp = A.p; lb = A.b; lrem -= used;
-                    ldone = end || lrem == 0;
-                }
+                rp = A.p; rb = A.b; rrem -= used;
+                rdone = end || rrem == 0;
             }
             if (bn) {
                 const uint32_t used = ((uint32_t)lp & 255u) - ((uint32_t)B.p & 255u);
@@ -1267,7 +1221,7 @@ __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen(const __grid_consta
         }
         if (__any_sync(kFull, finish && cand && !is_long)) {
             if (finish && cand && !is_long) {
-                score += seed_score(T_, Q_, ht, hq, L, seed_mask, s_tri, s_lut, ambig);
+                score += seed_score(T_, Q_, ht, hq, L, seed_mask, s_duo, s_lut, ambig);
                 cand = score >= thresh;
             }
         }
@@ -1392,17 +1346,21 @@ __global__ __launch_bounds__(WARPS * 32) void k_walk(const __grid_constant__ Wal
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t n = min(*a.n_dev, a.n_cap);
     const uint32_t L = a.seed_len;
-    // Chunks of 32 sorted positions are claimed dynamically: a segment with
-    // long candidates (full re-extension) can take far longer than the rest.
+    // Chunks of sorted positions are claimed dynamically: a segment with
+    // long candidates (full re-extension) can take far longer than the rest.  A
+    // chunk is 32 positions where that leaves every warp four of them, and down to
+    // one position in a small launch, whose time is that of the warp with the most
+    // segments.
+    const uint32_t chunk = max(1u, min(32u, n / (gridDim.x * WARPS * 4u)));
     for (;;) {
         uint32_t r = 0;
         if (lane == 0) r = atomicAdd(a.chunk_next, 1u);
         r = __shfl_sync(kFull, r, 0);
-        if ((uint64_t)r * 32 >= n) break;
-        const uint32_t i = r * 32 + lane;
+        if ((uint64_t)r * chunk >= n) break;
+        const uint32_t i = r * chunk + lane;
         bool head = false;
         uint32_t key_hi = 0;
-        if (i < n) {
+        if (i < n && (uint32_t)lane < chunk) {
             key_hi = (uint32_t)(a.keys[i] >> 32);
             head = (i == 0) || (key_hi != (uint32_t)(a.keys[i - 1] >> 32));
         }
@@ -1431,7 +1389,7 @@ __global__ __launch_bounds__(WARPS * 32) void k_walk(const __grid_constant__ Wal
         }
         uint32_t hb = __ballot_sync(kFull, head && !alone);
         while (hb) {
-            const uint32_t h = r * 32 + (uint32_t)(__ffs(hb) - 1);
+            const uint32_t h = r * chunk + (uint32_t)(__ffs(hb) - 1);
             hb &= hb - 1;
             const uint32_t segkey = (uint32_t)(a.keys[h] >> 32);
             // A segment (one diagonal key) can hold the candidates of several
