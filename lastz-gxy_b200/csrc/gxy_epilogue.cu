@@ -181,12 +181,162 @@ __device__ __forceinline__ uint32_t epi_blocks(uint32_t n) {
     return min(gridDim.x, max(1u, (n + kEpiTile - 1) / kEpiTile));
 }
 
+// ---- Up to kMergeMax candidates: tiles sorted in registers, then each item's
+// place from its rank in every other tile.  A digit pass costs two grid barriers
+// and a scan whatever the count, some 4 us; 30 to 40 key bits took five of them.
+
+// Keys of E x 512 items, item threadIdx.x * E + e in k[e] and v[e], in ascending
+// order (bitonic: strides inside a thread, then lanes, then the block).
+template <int E>
+__device__ void sort_tile(EpiSmem& S, uint64_t (&k)[E], uint32_t (&v)[E]) {
+    const uint32_t tid = threadIdx.x;
+    auto keep = [&](int e, uint64_t pk, uint32_t pv, bool lower) {   // the smaller of the two, or the larger
+        const bool take = lower ? pk < k[e] : pk > k[e];
+        k[e] = take ? pk : k[e];
+        v[e] = take ? pv : v[e];
+    };
+    for (uint32_t size = 2; size <= E * kEpiThreads; size <<= 1) {
+        const bool asc = !((tid * E) & size);   // (of strides from E on; inside a thread it may depend on e)
+        for (uint32_t stride = size >> 1; stride >= E; stride >>= 1) {
+            const uint32_t d = stride / E;
+            const bool lower = !(tid & d) == asc;
+            if (d >= 32) {
+                __syncthreads();
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    S.keys[e * kEpiThreads + tid] = k[e];
+                    S.vals[e * kEpiThreads + tid] = v[e];
+                }
+                __syncthreads();
+#pragma unroll
+                for (int e = 0; e < E; e++) keep(e, S.keys[e * kEpiThreads + (tid ^ d)], S.vals[e * kEpiThreads + (tid ^ d)], lower);
+            } else {
+#pragma unroll
+                for (int e = 0; e < E; e++) {
+                    const uint64_t pk = __shfl_xor_sync(kFull, k[e], d);
+                    const uint32_t pv = __shfl_xor_sync(kFull, v[e], d);
+                    keep(e, pk, pv, lower);
+                }
+            }
+        }
+#pragma unroll
+        for (uint32_t stride = E / 2; stride; stride >>= 1) {
+            if (stride >= size) continue;
+#pragma unroll
+            for (uint32_t e = 0; e < E; e++) {
+                if (e & stride) continue;
+                const bool up = !((tid * E + e) & size);
+                if (up ? k[e + stride] < k[e] : k[e + stride] > k[e]) {
+                    const uint64_t tk = k[e];
+                    k[e] = k[e + stride];
+                    k[e + stride] = tk;
+                    const uint32_t tv = v[e];
+                    v[e] = v[e + stride];
+                    v[e + stride] = tv;
+                }
+            }
+        }
+    }
+}
+
+constexpr uint32_t kMergeTiles = 32;
+constexpr uint32_t kMergeMax = kMergeTiles * 2 * kEpiThreads;
+
+template <int E>
+__device__ void sort_by_ranks(EpiSmem& S, const EpiSort& a, uint32_t n, uint32_t nb, uint32_t& phase) {
+    constexpr uint32_t kTile = E * kEpiThreads;
+    const uint32_t nt = (n + kTile - 1) / kTile, tid = threadIdx.x;
+    const bool odd = a.npass & 1;
+    uint64_t* const kout = odd ? a.k1 : a.k0;
+    uint32_t* const vout = odd ? a.v1 : a.v0;
+    // The sorted tiles: the result itself when there is one, else the buffer
+    // that the result does not take.
+    uint64_t* const kt = nt == 1 ? kout : (odd ? a.k0 : a.k1);
+    uint32_t* const vt = nt == 1 ? vout : (odd ? a.v0 : a.v1);
+    for (uint32_t t = blockIdx.x; t < nt; t += nb) {
+        uint64_t k[E];
+        uint32_t v[E];
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const uint32_t i = t * kTile + tid * E + e;
+            k[e] = i < n ? a.k0[i] : ~0ull;
+            v[e] = i < n ? a.v0[i] : 0xffffffffu;
+        }
+        __syncthreads();   // all of the tile is read: it may be written in place
+        sort_tile<E>(S, k, v);
+#pragma unroll
+        for (int e = 0; e < E; e++) {
+            const uint32_t i = t * kTile + tid * E + e;
+            if (i < n) {
+                kt[i] = k[e];
+                vt[i] = v[e];
+            }
+        }
+    }
+    if (nt == 1) return;
+    if (!grid_barrier(a.bar, nb, phase, &S.ok)) return;
+    // 128 neighbours of one tile a turn (their searches take almost the same
+    // path), a quarter of the tiles by each four warps, four searches at a time.
+    const uint32_t mine = tid & 127u, part = tid >> 7;
+    for (uint32_t i0 = blockIdx.x * 128; i0 < n; i0 += nb * 128) {
+        __syncthreads();
+        if (tid < 128) S.off[tid] = 0;
+        __syncthreads();
+        const uint32_t i = i0 + mine, own = i0 / kTile;
+        const uint64_t key = i < n ? kt[i] : ~0ull;
+        uint32_t rank = 0;
+        for (uint32_t t0 = part; t0 < nt; t0 += 16) {
+            uint32_t pos[4] = {0, 0, 0, 0}, cnt[4];
+#pragma unroll
+            for (uint32_t x = 0; x < 4; x++) {
+                const uint32_t t = t0 + 4 * x;
+                cnt[x] = t < nt && t != own ? min(kTile, n - t * kTile) : 0u;
+            }
+#pragma unroll
+            for (uint32_t s = kTile; s; s >>= 1) {
+#pragma unroll
+                for (uint32_t x = 0; x < 4; x++) {
+                    if (pos[x] + s <= cnt[x]) {
+                        const uint32_t t = t0 + 4 * x;
+                        const uint64_t other = kt[t * kTile + pos[x] + s - 1];
+                        if (other < key || (t < own && other == key)) pos[x] += s;
+                    }
+                }
+            }
+            rank += pos[0] + pos[1] + pos[2] + pos[3];
+        }
+        if (rank) atomicAdd(&S.off[mine], rank);
+        __syncthreads();
+        if (tid < 128 && i < n) {
+            const uint32_t o = i - own * kTile + S.off[tid];
+            kout[o] = key;
+            vout[o] = vt[i];
+        }
+    }
+}
+
+// What bounds it: up to 32,768 candidates the latency of the sorting network and
+// of the searches; above, two crossings of the buffers a digit.  By ranks and by
+// five digits: 721 candidates 10 and 22 us, 4,639 14 and 61, 15,346 22 and 68,
+// 32,187 48 and 69; with tiles of 2,048, 46,590 take 71 and 70, 64,123 96 and 68.
 __global__ __launch_bounds__(kEpiThreads, 1) void k_sort_candidates(const __grid_constant__ EpiSort a) {
     extern __shared__ __align__(16) unsigned char epi_smem[];
     EpiSmem& S = *reinterpret_cast<EpiSmem*>(epi_smem);
-    const uint32_t n = min(*a.n_dev, a.n_cap), nb = epi_blocks(n);
-    if (blockIdx.x >= nb) return;
+    const uint32_t n = min(*a.n_dev, a.n_cap);
     uint32_t phase = 0;
+    if (n <= kMergeMax && a.npass > 0) {
+        // The smallest tiles of which there are at most kMergeTiles; as many blocks
+        // as have 128 items to place.
+        const uint32_t nb = n <= kEpiThreads ? 1u : min(gridDim.x, (n + 127) / 128);
+        if (blockIdx.x >= nb) return;
+        if (a.clear)
+            for (uint32_t i = blockIdx.x * kEpiThreads + threadIdx.x; i < n; i += nb * kEpiThreads) a.clear[i] = 0;
+        if (n <= kMergeMax / 2) sort_by_ranks<1>(S, a, n, nb, phase);
+        else sort_by_ranks<2>(S, a, n, nb, phase);
+        return;
+    }
+    const uint32_t nb = epi_blocks(n);
+    if (blockIdx.x >= nb) return;
     if (a.clear)
         for (uint32_t i = blockIdx.x * kEpiThreads + threadIdx.x; i < n; i += nb * kEpiThreads) a.clear[i] = 0;
     for (int p = 0; p < a.npass; p++) {
@@ -308,16 +458,16 @@ void epilogue_init() {
     cudaFuncSetAttribute(k_finish_hsps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EpiSmem));
 }
 
-// Blocks for an expected count: one per tile, at most one per SM.
-static int epi_grid(uint64_t expected, int sm_count) {
-    return (int)std::max<uint64_t>(1, std::min<uint64_t>((expected + kEpiTile - 1) / kEpiTile, (uint64_t)sm_count));
+// Blocks for an expected count: one per `per` items, at most one per SM.
+static int epi_grid(uint64_t expected, uint64_t per, int sm_count) {
+    return (int)std::max<uint64_t>(1, std::min<uint64_t>((expected + per - 1) / per, (uint64_t)sm_count));
 }
 
 cudaError_t launch_sort_candidates(const EpiSort& a, uint64_t expected, int sm_count, cudaStream_t st) {
     EpiSort arg = a;
     void* args[] = {&arg};
     count_launch();
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_sort_candidates), dim3(epi_grid(expected, sm_count)),
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_sort_candidates), dim3(epi_grid(expected, 128, sm_count)),
                                        dim3(kEpiThreads), args, sizeof(EpiSmem), st);
 }
 
@@ -325,7 +475,7 @@ cudaError_t launch_finish_hsps(const EpiFinish& a, uint64_t expected, int sm_cou
     EpiFinish arg = a;
     void* args[] = {&arg};
     count_launch();
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_finish_hsps), dim3(epi_grid(expected, sm_count)),
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_finish_hsps), dim3(epi_grid(expected, kEpiTile, sm_count)),
                                        dim3(kEpiThreads), args, sizeof(EpiSmem), st);
 }
 

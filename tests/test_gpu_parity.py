@@ -533,3 +533,29 @@ def test_enumerate_tables(gxy, ctx, pattern, n, nq, transitions, mwc):
         assert st2["raw_hits"] == st["raw_hits"] and st2["windows"] == st["windows"]
     finally:
         c2.close()
+
+
+def test_candidate_sort_sizes(gxy, ctx):
+    # Candidates are sorted in one block up to 512, by tiles of 512 or 1,024 and their
+    # ranks up to 16,384 and 32,768, by digits above: random sequences at a threshold near the
+    # seeds' own score, so that a sizeable share of the raw hits are candidates, in
+    # steps that put a count into each range, on both sides of an odd and an even
+    # number of digit passes (which buffer takes the result); in a second call as well.
+    counts = []
+    for i, (n, nq) in enumerate([(20_000, 9_000), (60_000, 60_000), (150_000, 150_000), (300_000, 160_000), (350_000, 250_000),
+                                 (400_000, 400_000), (700_000, 700_000), (2_500_000, 180_000), (70, 70), (950_000, 950_000)]):
+        rng = np.random.default_rng(60 + i)
+        t, q = rand_ascii(rng, n, b"ACGT"), rand_ascii(rng, nq, b"ACGT")
+        m = gxy.ScoringMatrix.hoxd70()
+        sp = gxy.SearchParams(1, gxy.HspParams(910, 1000), 1)
+        T, Q = gxy.PackedSeq.from_ascii(t), gxy.PackedSeq.from_ascii(q)
+        tab = gxy.PosTable.build(T, P12, 1, ctx=ctx)
+        st = {}
+        o, _ = oracle_search(t, q, P12, m, sp)
+        for _ in range(2):
+            g = gxy.search(tab, T, Q, m, sp, stats=st)
+            assert as_tuples(g) == as_tuples(o), (n, nq)
+        counts.append(st["candidates"])
+        tab.free()
+    edges = [0, 512, 16_384, 32_768, 65_536, 131_072, 1 << 31]
+    assert all(any(lo < c <= hi for c in counts) for lo, hi in zip(edges, edges[1:])), counts
