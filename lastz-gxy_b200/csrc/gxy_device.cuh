@@ -227,33 +227,40 @@ __device__ __forceinline__ LaneExt extend_lane(const SeqView& T, const SeqView& 
 }
 
 // ---------------------------------------------------------------------------
-// Warp-cooperative x-drop: one warp per hit, 64 columns per step (two per
-// lane), the x-drop cut found with shuffle scans.  Column k of a step breaks the reference's
+// Warp-cooperative x-drop: one warp per hit, half a warp per side, 128 columns
+// per step (eight per lane), the x-drop cut found with shuffle scans.
+// Column k of a step breaks the reference's
 // loop iff run_k <= PM_{k-1} and PM_{k-1} - run_k > xdrop, where
 // PM_{k-1} = max(best, run_0..run_{k-1}); the best extent is the first column
 // whose running score equals the step's maximum (the reference updates only
 // on a strict increase).  Sequence bytes are staged through shared memory in
-// 16-byte vector loads: kStageSpan positions per refill.
+// 16-byte vector loads: kStageSpan positions per side and refill.
+//
+// What bounds it is latency -- the step's chain of shuffles, the refills, and in a
+// short kernel the fetch of its own code: one side after the other, 64 columns a
+// step in two unrolled copies, took 13,000 cycles for sides of a few hundred
+// columns.  The walk of 10 Mbp (its launch of one strand) went from 81 to 65 us,
+// that of 1 Mbp with entropy gates from 95 to 79 us.
 // ---------------------------------------------------------------------------
-constexpr uint32_t kStageCols = 1024;
-constexpr uint32_t kStageSpan = kStageCols + 128;          // positions staged per refill
-struct WarpStage {
-    uint64_t tcodes[kStageSpan / 32];
-    uint64_t qcodes[kStageSpan / 32];
-    uint32_t tvalid[kStageSpan / 32];
-    uint32_t qvalid[kStageSpan / 32];
+constexpr uint32_t kStageCols = 512;                       // columns a refill is good for
+constexpr uint32_t kStageSpan = 768;                       // positions per refill (+ 127 to the boundary, + a funnel read)
+struct WarpStage {   // [0]: the right side, [1]: the left one
+    uint64_t tcodes[2][kStageSpan / 32];
+    uint64_t qcodes[2][kStageSpan / 32];
+    uint32_t tvalid[2][kStageSpan / 32];
+    uint32_t qvalid[2][kStageSpan / 32];
 };
 
 // Copies positions [a, a + kStageSpan) (a a multiple of 128) of one sequence
-// into the stage with 16-byte loads: codes 288 bytes, valid 144 bytes.
+// into a side's stage with 16-byte loads by its 16 lanes: codes 192 bytes, valid 96.
 __device__ __forceinline__ void stage_fill(const uint64_t* codes, const uint32_t* valid, uint64_t a,
-                                           uint64_t* scodes, uint32_t* svalid, int lane) {
+                                           uint64_t* scodes, uint32_t* svalid, int hl) {
     const uint4* c4 = reinterpret_cast<const uint4*>(codes + (a >> 5));
     const uint4* v4 = reinterpret_cast<const uint4*>(valid + (a >> 5));
-    constexpr int kC4 = kStageSpan / 32 * 8 / 16;   // 18
-    constexpr int kV4 = kStageSpan / 32 * 4 / 16;   // 9
-    if (lane < kC4) reinterpret_cast<uint4*>(scodes)[lane] = __ldg(c4 + lane);
-    if (lane < kV4) reinterpret_cast<uint4*>(svalid)[lane] = __ldg(v4 + lane);
+    constexpr int kC4 = kStageSpan / 32 * 8 / 16;   // 12
+    constexpr int kV4 = kStageSpan / 32 * 4 / 16;   // 6
+    if (hl < kC4) reinterpret_cast<uint4*>(scodes)[hl] = __ldg(c4 + hl);
+    if (hl < kV4) reinterpret_cast<uint4*>(svalid)[hl] = __ldg(v4 + hl);
 }
 
 __device__ __forceinline__ uint64_t stage_codes32(const uint64_t* s, uint32_t off) {
@@ -265,100 +272,10 @@ __device__ __forceinline__ uint32_t stage_bits32(const uint32_t* s, uint32_t off
     return __funnelshift_r(s[off >> 5], s[(off >> 5) + 1], off & 31);
 }
 
-template <bool kForward>
-__device__ void side_warp(const SeqView& T, const SeqView& Q, uint32_t t0, uint32_t q0,
-                          uint32_t maxext, int32_t xdrop, const int32_t* lut, int32_t ambig,
-                          WarpStage* st, int32_t& best_out, uint32_t& bext_out) {
-    // 64 columns per step: lane l scores columns 2l and 2l+1.  A refill
-    // stages 1,152 positions, enough for 15 steps (960 columns) with every
-    // lane's 32-position funnel read inside the stage.
-    constexpr uint32_t kSteps = 960;
-    const int lane = threadIdx.x & 31;
-    int32_t run = 0, best = 0;
-    uint32_t bext = 0, ext = 0;
-    uint64_t ta = 0, qa = 0;   // staged windows' first global positions
-    uint32_t staged = 0;       // columns left in the current stage
-    const uint32_t c0 = 2u * (uint32_t)lane, c1 = c0 + 1;
-    while (ext < maxext) {
-        // The step's 64 positions: [tg, tg + 64).
-        const uint64_t tg = kForward ? T.base + t0 + ext : T.base + t0 - ext - 63;
-        const uint64_t qg = kForward ? Q.base + q0 + ext : Q.base + q0 - ext - 63;
-        if (staged < 64) {
-            __syncwarp();
-            if (kForward) {
-                ta = tg & ~127ull;
-                qa = qg & ~127ull;
-            } else {
-                const uint64_t tl = tg + 63 >= kSteps ? tg + 63 - (kSteps - 1) : 0;
-                const uint64_t ql = qg + 63 >= kSteps ? qg + 63 - (kSteps - 1) : 0;
-                ta = tl & ~127ull;
-                qa = ql & ~127ull;
-            }
-            stage_fill(T.codes, T.valid, ta, st->tcodes, st->tvalid, lane);
-            stage_fill(Q.codes, Q.valid, qa, st->qcodes, st->qvalid, lane);
-            __syncwarp();
-            staged = kSteps;
-        }
-        // This lane's two columns sit at window offsets c0, c1 (forward) or
-        // 63 - c0, 63 - c1 (backward): one funnel read from the lower one.
-        const uint32_t lo = kForward ? c0 : 62u - c0;
-        const uint32_t to = (uint32_t)(tg - ta) + lo, qo = (uint32_t)(qg - qa) + lo;
-        const uint64_t tc = stage_codes32(st->tcodes, to);
-        const uint64_t qc = stage_codes32(st->qcodes, qo);
-        const uint32_t vv = stage_bits32(st->tvalid, to) & stage_bits32(st->qvalid, qo);
-        const uint32_t n = min(64u, maxext - ext);
-        const bool a0 = c0 < n, a1 = c1 < n;
-        const int32_t x0 = a0 ? col_score(tc, qc, vv, kForward ? 0 : 1, lut, ambig) : 0;
-        const int32_t x1 = a1 ? col_score(tc, qc, vv, kForward ? 1 : 0, lut, ambig) : 0;
-        int32_t x = x0 + x1;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t y = __shfl_up_sync(kFull, x, o);
-            if (lane >= o) x += y;
-        }
-        const int32_t r1 = run + x;      // running score after column c1
-        const int32_t r0 = r1 - x1;      // after column c0
-        int32_t m = a0 ? (a1 ? max(r0, r1) : r0) : INT32_MIN;
-#pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const int32_t y = __shfl_up_sync(kFull, m, o);
-            if (lane >= o) m = max(m, y);
-        }
-        int32_t pm = __shfl_up_sync(kFull, m, 1);
-        if (lane == 0) pm = INT32_MIN;
-        pm = max(pm, best);              // prefix maximum before column c0
-        const bool brk0 = a0 && r0 <= pm && (pm - r0 > xdrop);
-        const int32_t pm1 = max(pm, r0); // before column c1
-        const bool brk1 = a1 && r1 <= pm1 && (pm1 - r1 > xdrop);
-        const uint32_t bm = __ballot_sync(kFull, brk0 || brk1);
-        uint32_t nproc = n;              // columns before the break column
-        if (bm) {
-            const int bl = __ffs(bm) - 1;
-            const bool b0 = __shfl_sync(kFull, brk0, bl);
-            nproc = 2u * (uint32_t)bl + (b0 ? 0u : 1u);
-        }
-        int32_t c = INT32_MIN;
-        if (c0 < nproc) c = r0;
-        if (c1 < nproc) c = max(c, r1);
-#pragma unroll
-        for (int o = 16; o > 0; o >>= 1) c = max(c, __shfl_xor_sync(kFull, c, o));
-        if (c > best) {
-            // The first column that reaches the step's maximum.
-            const bool e0 = c0 < nproc && r0 == c;
-            const bool e1 = c1 < nproc && r1 == c;
-            const uint32_t eq = __ballot_sync(kFull, e0 || e1);
-            const int el = __ffs(eq) - 1;
-            const bool f0 = __shfl_sync(kFull, e0, el);
-            bext = ext + 2u * (uint32_t)el + (f0 ? 1u : 2u);
-            best = c;
-        }
-        if (bm) break;
-        run = __shfl_sync(kFull, r1, 31);
-        ext += n;
-        staged -= 64;
-    }
-    best_out = best;
-    bext_out = bext;
+// The 8 columns in the low 16 bits in reverse order.
+__device__ __forceinline__ uint32_t rev_pairs16(uint32_t x) {
+    x = __brev(x) >> 16;
+    return ((x >> 1) & 0x5555u) | ((x & 0x5555u) << 1);
 }
 
 // extend_hit_scalar (src/hsp.rs:98-148) with one warp; every lane returns the
@@ -366,23 +283,118 @@ __device__ void side_warp(const SeqView& T, const SeqView& Q, uint32_t t0, uint3
 __device__ __forceinline__ LaneExt extend_warp(const SeqView& T, const SeqView& Q, uint32_t t,
                                                uint32_t q, uint32_t L, int32_t xdrop,
                                                const int32_t* lut, int32_t ambig, WarpStage* st) {
-    const int lane = threadIdx.x & 31;
-    LaneExt r;
-    const uint64_t tc = load_codes32(T.codes, T.base + t);
-    const uint64_t qc = load_codes32(Q.codes, Q.base + q);
-    const uint32_t vv = load_bits32(T.valid, T.base + t) & load_bits32(Q.valid, Q.base + q);
-    int32_t s = ((uint32_t)lane < L) ? col_score(tc, qc, vv, lane, lut, ambig) : 0;
+    const int lane = threadIdx.x & 31, hl = lane & 15;
+    const bool left = lane >= 16;
+    const uint32_t half = left ? 16u : 0u;   // the side's first lane
+    const uint64_t stc = load_codes32(T.codes, T.base + t);
+    const uint64_t sqc = load_codes32(Q.codes, Q.base + q);
+    const uint32_t svv = load_bits32(T.valid, T.base + t) & load_bits32(Q.valid, Q.base + q);
+    // The side's column 0 and columns; it runs up or (left) down from there.
+    const uint64_t t0 = left ? T.base + t - 1 : T.base + t + L, q0 = left ? Q.base + q - 1 : Q.base + q + L;
+    const uint32_t maxext = left ? min(t, q) : min(T.len - t - L, Q.len - q - L);
+    uint64_t* const tcodes = st->tcodes[left];
+    uint64_t* const qcodes = st->qcodes[left];
+    uint32_t* const tvalid = st->tvalid[left];
+    uint32_t* const qvalid = st->qvalid[left];
+    int32_t run = 0, best = 0;
+    uint32_t bext = 0, ext = 0;
+    uint64_t ta = 0, qa = 0;   // staged windows' first global positions
+    uint32_t staged = 0;       // columns left in the current stage
+    bool live = maxext > 0;
+    while (__any_sync(kFull, live)) {
+        const uint64_t tg = left ? t0 - ext : t0 + ext, qg = left ? q0 - ext : q0 + ext;
+        const bool refill = live && staged < 128;
+        if (__any_sync(kFull, refill)) {
+            __syncwarp();
+            if (refill) {
+                ta = (left ? (tg >= kStageCols ? tg - (kStageCols - 1) : 0) : tg) & ~127ull;
+                qa = (left ? (qg >= kStageCols ? qg - (kStageCols - 1) : 0) : qg) & ~127ull;
+                stage_fill(T.codes, T.valid, ta, tcodes, tvalid, hl);
+                stage_fill(Q.codes, Q.valid, qa, qcodes, qvalid, hl);
+                staged = kStageCols;
+            }
+            __syncwarp();
+        }
+        // Eight columns by one funnel read from the lowest position (a lane whose
+        // columns do not exist may lie before the stage).
+        const uint32_t c0 = 8u * (uint32_t)hl;
+        const int32_t lo = left ? -(int32_t)(c0 + 7) : (int32_t)c0;
+        const uint32_t to = live ? (uint32_t)max(0, (int32_t)(tg - ta) + lo) : 0u;
+        const uint32_t qo = live ? (uint32_t)max(0, (int32_t)(qg - qa) + lo) : 0u;
+        uint32_t tc = (uint32_t)stage_codes32(tcodes, to) & 0xffffu;
+        uint32_t qc = (uint32_t)stage_codes32(qcodes, qo) & 0xffffu;
+        uint32_t vv = stage_bits32(tvalid, to) & stage_bits32(qvalid, qo) & 0xffu;
+        if (left) {
+            tc = rev_pairs16(tc);
+            qc = rev_pairs16(qc);
+            vv = __brev(vv) >> 24;
+        }
+        const uint32_t n = live ? min(128u, maxext - ext) : 0u, mine = c0 < n ? min(8u, n - c0) : 0u;
+        // The lane's running sums and their maximum, then both before the lane.
+        int32_t p[8], sum = 0, top = INT32_MIN;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++) {
+            const int32_t x = (vv >> k) & 1u ? lut[((tc >> (2 * k)) & 3u) << 2 | ((qc >> (2 * k)) & 3u)] : ambig;
+            if (k < mine) {
+                sum += x;
+                top = max(top, sum);
+            }
+            p[k] = sum;
+        }
+        int32_t S = sum, M = top;
+#pragma unroll
+        for (int o = 1; o < 16; o <<= 1) {
+            const int32_t ys = __shfl_up_sync(kFull, S, o, 16), ym = __shfl_up_sync(kFull, M, o, 16);
+            if (hl >= o) {
+                M = M == INT32_MIN ? ym : max(ym, ys + M);
+                S += ys;
+            }
+        }
+        int32_t pm = __shfl_up_sync(kFull, M, 1, 16);
+        pm = hl == 0 || pm == INT32_MIN ? best : max(best, run + pm);   // before the lane's first column
+        const int32_t r = run + S - sum;
+        // Its columns up to the first break, their maximum and where it is first.
+        uint32_t upto = mine, at = 0;
+        int32_t c = INT32_MIN;
+#pragma unroll
+        for (uint32_t k = 0; k < 8; k++) {
+            const int32_t rk = r + p[k];
+            if (k < upto) {
+                if (rk <= pm && pm - rk > xdrop) {
+                    upto = k;
+                } else {
+                    pm = max(pm, rk);
+                    if (rk > c) {
+                        c = rk;
+                        at = k;
+                    }
+                }
+            }
+        }
+        const uint32_t bm = (__ballot_sync(kFull, upto < mine) >> half) & 0xffffu;
+        if (bm && hl > __ffs(bm) - 1) c = INT32_MIN;
+        const int32_t high0 = __reduce_max_sync(kFull, left ? INT32_MIN : c);
+        const int32_t high1 = __reduce_max_sync(kFull, left ? c : INT32_MIN);
+        const int32_t high = left ? high1 : high0;
+        const uint32_t eq = (__ballot_sync(kFull, c == high) >> half) & 0xffffu;   // (never empty)
+        const int el = __ffs(eq) - 1;
+        const uint32_t at_el = __shfl_sync(kFull, at, el, 16);
+        if (high > best) {
+            bext = ext + 8u * (uint32_t)el + at_el + 1;
+            best = high;
+        }
+        run = __shfl_sync(kFull, run + S, 15, 16);
+        ext += n;
+        staged -= live ? 128u : 0u;
+        live = live && bm == 0 && ext < maxext;
+    }
+    int32_t s = ((uint32_t)lane < L) ? col_score(stc, sqc, svv, lane, lut, ambig) : 0;
 #pragma unroll
     for (int o = 16; o > 0; o >>= 1) s += __shfl_xor_sync(kFull, s, o);
-    int32_t rb, lb = 0;
-    uint32_t re, le = 0;
-    const uint32_t rmax = min(T.len - t - L, Q.len - q - L);
-    side_warp<true>(T, Q, t + L, q + L, rmax, xdrop, lut, ambig, st, rb, re);
-    const uint32_t lmax = min(t, q);
-    if (lmax) side_warp<false>(T, Q, t - 1, q - 1, lmax, xdrop, lut, ambig, st, lb, le);
-    r.score = s + lb + rb;
-    r.lext = le;
-    r.rext = re;
+    LaneExt r;
+    r.score = s + __shfl_sync(kFull, best, 0) + __shfl_sync(kFull, best, 16);
+    r.rext = __shfl_sync(kFull, bext, 0);
+    r.lext = __shfl_sync(kFull, bext, 16);
     r.done = true;
     return r;
 }

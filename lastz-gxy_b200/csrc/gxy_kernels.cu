@@ -1411,20 +1411,22 @@ __global__ __launch_bounds__(WARPS * 32) void k_walk(const __grid_constant__ Wal
                 Cand c;
                 c.unit = 0xffffffffu; c.t = 0;
                 if (inseg) c = a.cands[a.idx[jj]];
-                const bool elig = inseg && c.unit == cur_unit && c.t >= cover;
                 const uint32_t be = __ballot_sync(kFull, !inseg);
-                const uint32_t bc = __ballot_sync(kFull, elig);
                 const uint32_t stop = be ? (uint32_t)(__ffs(be) - 1) : 32u;
-                const uint32_t first = bc ? (uint32_t)(__ffs(bc) - 1) : 32u;
-                // Other units among the positions this step passes over.
-                if (a.n_units > 1) {
-                    const uint32_t upto = min(first, stop);
-                    const bool seen = (uint32_t)lane <= upto && inseg;
-                    next = min(next, __reduce_min_sync(kFull, (seen && c.unit > cur_unit && c.unit < ceil)
-                                                                  ? c.unit : 0xffffffffu));
-                    below = min(below, __reduce_min_sync(kFull, (seen && c.unit < u0) ? c.unit : 0xffffffffu));
-                }
-                if (first < stop) {
+                // The candidates of these 32 positions that cover admits, one by one.
+                for (uint32_t from = 0;;) {
+                    const bool elig = inseg && c.unit == cur_unit && c.t >= cover && (uint32_t)lane >= from;
+                    const uint32_t bc = __ballot_sync(kFull, elig);
+                    const uint32_t first = bc ? (uint32_t)(__ffs(bc) - 1) : 32u;
+                    // Other units among the positions this step passes over.
+                    if (a.n_units > 1) {
+                        const uint32_t upto = min(first, stop);
+                        const bool seen = (uint32_t)lane <= upto && inseg;
+                        next = min(next, __reduce_min_sync(kFull, (seen && c.unit > cur_unit && c.unit < ceil)
+                                                                      ? c.unit : 0xffffffffu));
+                        below = min(below, __reduce_min_sync(kFull, (seen && c.unit < u0) ? c.unit : 0xffffffffu));
+                    }
+                    if (first >= stop) break;
                     const uint32_t unit = cur_unit;
                     const uint32_t t = __shfl_sync(kFull, c.t, first);
                     const uint32_t q = __shfl_sync(kFull, c.q, first);
@@ -1456,11 +1458,22 @@ __global__ __launch_bounds__(WARPS * 32) void k_walk(const __grid_constant__ Wal
                             a.out_flag[pos] = keep ? 1 : 0;
                         }
                     }
-                    j = j + first + 1;
-                    continue;
+                    from = first + 1;
                 }
                 if (stop < 32) break;
                 j += 32;
+                if (a.n_units == 1) {
+                    // Past the 32-position steps whose last key is still covered (with several
+                    // units every position is looked at: another one may hide there).
+                    const uint64_t uncovered = (uint64_t)segkey << 32 | (a.tsegs[a.units[0].tseg].key_base + cover);
+                    uint32_t skip = 32;
+                    while (skip == 32) {
+                        const uint64_t last = (uint64_t)j + 32u * (uint32_t)lane + 31;
+                        const uint32_t go = __ballot_sync(kFull, last >= n || a.keys[last] >= uncovered);
+                        skip = go ? (uint32_t)(__ffs(go) - 1) : 32u;
+                        j += 32 * skip;
+                    }
+                }
             }
             if (next != 0xffffffffu) {
                 cur_unit = next;                      // the next unit above

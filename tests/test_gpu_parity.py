@@ -559,3 +559,36 @@ def test_candidate_sort_sizes(gxy, ctx):
         tab.free()
     edges = [0, 512, 16_384, 32_768, 65_536, 131_072, 1 << 31]
     assert all(any(lo < c <= hi for c in counts) for lo, hi in zip(edges, edges[1:])), counts
+
+
+@pytest.mark.parametrize("side", [0, 1, 7, 8, 63, 119, 127, 128, 129, 135, 383, 385, 511, 512, 513, 519, 640, 1025, 5000])
+def test_extend_step_edges(gxy, ctx, side):
+    # The warp x-drop takes 128 columns of both sides a step (eight a lane) and
+    # restages after 512: sides that the sequence ends after `side`
+    # columns, and ones that a run of mismatches breaks there, after 0 to 7 more
+    # columns, with single mismatches and Ns before; either side of the seed.
+    rng = np.random.default_rng(side)
+    m = gxy.ScoringMatrix.hoxd70()
+    L = 12
+    flip = bytes.maketrans(b"ACGT", b"CATG")
+    for cut in range(9):
+        left, right = (side, 700 + 13 * cut) if cut % 2 else (30 + 41 * cut, side)
+        tail = 0 if cut == 8 else 40 + cut
+        core = bytearray(rand_ascii(rng, left + L + right, b"ACGT"))
+        q = bytearray(core)
+        for i in rng.integers(0, len(q), len(q) // 9):
+            if not left <= i < left + L:
+                q[i] = b"ACGTN"[rng.integers(5)]
+        junk = rand_ascii(rng, cut % 8, b"ACGT")
+        bad = rand_ascii(rng, tail, b"ACGT")
+        tb = bad + junk + bytes(core) + junk + bad
+        qb = bad.translate(flip) + junk + bytes(q) + junk + bad.translate(flip)
+        T, Q = gxy.DeviceSeq.from_ascii(tb, ctx=ctx), gxy.DeviceSeq.from_ascii(qb, ctx=ctx)
+        OT, OQ = O.pack_ascii(tb), O.pack_ascii(qb)
+        at = len(bad) + len(junk) + left
+        for xd in (300, 910, 1 << 20):
+            o = O.extend_hit(OT, OQ, O.params(xdrop=xd, hspthresh=0), at, at, L)
+            for mode in (0, 1):
+                h, ok = gxy.extend_hits(T, Q, m, gxy.HspParams(xd, 0), [at], [at], L, mode)
+                got = tuple(int(h[0][k]) for k in ("t_start", "q_start", "length", "score")) if ok[0] else None
+                assert got == o, (side, cut, xd, mode)
