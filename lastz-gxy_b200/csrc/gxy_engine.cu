@@ -218,6 +218,16 @@ gxy_status parse_pattern(const char* s, Pattern& pat) {
     }
     pat.len = len;
     pat.weight = w;
+    // Runs of adjacent care positions: in the reversed codes position i is at bits
+    // 2 (31 - i), in the word care position r at 2 (w - 1 - r).
+    for (uint32_t r = 0; r < w;) {
+        uint32_t e = r + 1;
+        while (e < w && pat.care[e] == pat.care[e - 1] + 1) e++;
+        const uint32_t low = 2 * (w - e);   // of the run's last position in the word
+        pat.run_shift[pat.n_runs] = (uint8_t)(2 * (31 - pat.care[e - 1]) - low);
+        pat.run_mask[pat.n_runs++] = (uint32_t)(((1ull << (2 * (e - r))) - 1) << low);
+        r = e;
+    }
     return GXY_OK;
 }
 

@@ -390,7 +390,7 @@ __device__ __forceinline__ void store_hit(const ScreenArgs& a, uint64_t i, uint3
     if (a.n_units > 1) a.hits[2 * a.hit_cap + i] = u;
 }
 
-constexpr int kEnumWarps = 8, kEnumBlocks = 4;   // 39 KB of shared memory a block, 43 with a lane a byte
+constexpr int kEnumWarps = 8, kEnumBlocks = 4;   // 31 KB of shared memory a block, 35 with a lane a byte
 constexpr uint32_t kWordBits = (1u << 27) - 1;   // of an entry; the lane above
 
 // kMode 0: the words themselves only; 1: neighbour masks; 2: masks formed from
@@ -400,24 +400,12 @@ __global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(cons
     constexpr uint32_t kEntries = kMode == 0 ? 32 : 512;   // 32 masks of at most 16 bits
     constexpr int K = kMode == 0 ? 1 : 2;                  // entries a lane holds at a time
     __shared__ unsigned long long s_stats[2];              // windows, raw hits
-    __shared__ uint32_t s_word[8][256];                    // what byte k of a window's codes gives the word
     __shared__ uint32_t s_ent[kEnumWarps][kEntries];       // the entries' words, then their buckets' starts
     __shared__ uint32_t s_cnt[kEnumWarps][kMode == 0 ? 1 : kEntries - 64];   // lane and size from entry 64 on
     __shared__ uint8_t s_who[kMode == 1 ? 1 : kEnumWarps][kEntries];          // the entries' lanes
     const int lane = threadIdx.x & 31;
-    const uint32_t n_bytes = (a.pat.len + 3) / 4, weight = a.pat.weight;
+    const uint32_t weight = a.pat.weight;
     if (threadIdx.x < 2) s_stats[threadIdx.x] = 0;
-    static_assert(kEnumWarps * 32 == 256, "a thread a byte value");
-    for (uint32_t x = 0; x < n_bytes; x++) {
-        uint32_t w = 0;
-#pragma unroll
-        for (uint32_t c = 0; c < 4; c++) {   // (the shifts are the block's, not the thread's)
-            const uint32_t pos = 4 * x + c;
-            if ((a.pat.care_mask >> pos) & 1u)
-                w |= ((threadIdx.x >> (2 * c)) & 3u) << (2 * (weight - 1 - __popc(a.pat.care_mask & ((1u << pos) - 1u))));
-        }
-        s_word[x][threadIdx.x] = w;
-    }
     __syncthreads();
     uint32_t* const ent = s_ent[threadIdx.x >> 5];
     uint32_t* const cnt = s_cnt[threadIdx.x >> 5];
@@ -507,18 +495,15 @@ __global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(cons
             u_hi = u_lo + (U->nwin + 31) / 32;
         }
         const uint32_t k = (tile - u_lo) * 32 + lane;
-        // The window's word: its codes a byte at a time through the tables.
+        // The window's word.
         uint32_t word0 = 0;
         bool wv = false;
         if (k < U->nwin) {
             const SeqView& Q = a.qsegs[U->qseg];
             const uint64_t gq = Q.base + (uint64_t)k * a.step;
             const uint32_t ok = load_bits32(Q.valid, gq) & ~load_bits32(Q.mask, gq);
-            const uint64_t c = load_codes32(Q.codes, gq);
             wv = (ok & a.pat.care_mask) == a.pat.care_mask;
-#pragma unroll
-            for (uint32_t x = 0; x < 8; x++)
-                if (x < n_bytes) word0 |= s_word[x][(uint32_t)(c >> (8 * x)) & 255u];
+            word0 = word_of(a.pat, load_codes32(Q.codes, gq));
         }
         for (; g < g_end; g++) {
         if (g == 0) windows += wv ? 1 : 0;

@@ -15,6 +15,9 @@ struct Pattern {
     uint32_t weight;      // care positions, <= kMaxWeight
     uint32_t care_mask;   // bit i set when offset i is a care position
     uint8_t care[16];     // care offsets, leftmost first
+    uint32_t n_runs;                 // runs of adjacent care positions (see word_of)
+    uint32_t run_mask[kMaxWeight];
+    uint8_t run_shift[kMaxWeight];
 };
 
 // SeedExtractor::word_at (src/seeds.rs:133-147) at view-local position p
@@ -72,6 +75,20 @@ void launch_prune_counts(const uint32_t* starts, uint64_t num_words, uint32_t li
 // kept buckets hold at most `limit` positions).
 void launch_prune_copy(const uint32_t* positions, const uint32_t* starts, uint64_t num_words,
                        const uint32_t* new_starts, uint32_t limit, uint32_t* new_positions, cudaStream_t st);
+
+// The same word from the codes of 32 positions (whose validity the caller
+// checks): reversed, the care positions' runs of code pairs only have to move down,
+// two instructions a run (Pattern::run_shift, run_mask).
+__device__ __forceinline__ uint32_t word_of_reversed(const Pattern& pat, uint64_t c) {
+    uint32_t w = 0;
+#pragma unroll
+    for (int i = 0; i < kMaxWeight; i++) {
+        if ((uint32_t)i >= pat.n_runs) break;
+        w |= (uint32_t)(c >> pat.run_shift[i]) & pat.run_mask[i];
+    }
+    return w;
+}
+__device__ __forceinline__ uint32_t word_of(const Pattern& pat, uint64_t c) { return word_of_reversed(pat, rev_pairs64(c)); }
 
 // --- search ------------------------------------------------------------------
 // Seed hits: target position t, query window q, unit, in three arrays of the

@@ -252,6 +252,8 @@ int radix_impl(K* ka, uint32_t* va, K* kb, uint32_t* vb, const uint32_t* n_dev, 
 
 }  // namespace
 
+void scan_small(uint32_t* a, int n, cudaStream_t st) { k_scan_small<<<1, 1024, 0, st>>>(a, n); }
+
 void prims_init() {
     radix_attr<uint32_t>();
     radix_attr<uint64_t>();

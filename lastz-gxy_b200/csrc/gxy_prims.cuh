@@ -30,6 +30,9 @@ struct PrimScratch {
     int sort_grid_max;      // radix passes use min(this, one block per two tiles of n_cap) blocks
 };
 
+// Exclusive scan of a short array in place by one block; a[n] = the total.
+void scan_small(uint32_t* a, int n, cudaStream_t st);
+
 // Exclusive scan of n u32 (or u8) values into out[0..n); out[n] and *total
 // (either may be null) receive the sum.  n is min(*n_dev, n_cap) when n_dev is
 // not null, else n_host.  The sum must fit in u32.

@@ -7,6 +7,26 @@
 // through per-word cursors (src/pos_table.rs:42-75).  Here the views share
 // one bucket space, view v's word w being bucket g = v * 4^w + w:
 //
+// Weights 6 to 13 (kPartBuckets and more words, at most kMaxParts partitions of
+// kPartBuckets a view) are built by partition, a group of views at a time:
+//
+//  1. k_part_count: every block counts its share of the windows by partition, in
+//     shared memory;  k_part_prefix and a scan turn the counts into every block's
+//     first slot in every partition;
+//  2. k_part_scatter writes each window's position and low word bits to its slot;
+//  3. k_part_build, a block a partition: counts, starts, occupancy, packed bounds
+//     and the positions of its 4,096 buckets in shared memory, buckets of up to 8
+//     positions put in order there, all written once and in order.
+//
+// What bounds it: the scattered 8-byte writes of step 2 (73 us for 10 M windows),
+// in step 3 the instructions for the buckets, empty or not (47 us for 16.7 M of
+// them, 88 us with 10 M positions); step 1 takes 26 us.  Bucket by bucket the same
+// table took 256 us (random atomics on 64 MB of counts, twice, a three-pass scan
+// and a copy of them), an all but empty one 95 us against 63.  Three and four
+// blocks an SM instead of two spill step 3's registers: 103 and 117 us.
+//
+// The other weights, bucket by bucket:
+//
 //  1. k_count_words counts the windows of every bucket (atomics on an array
 //     that stays in L2 for a chromosome-sized view);
 //  2. one exclusive scan turns the counts into global bucket starts, and
@@ -23,11 +43,12 @@
 // global starts g = v * 4^w .. v * 4^w + 4^w (global indices into the shared
 // positions array, which the searches use as they are; the download
 // subtracts the view's first index), and its occupancy bitmap is the shared
-// bitmap's words from v * 4^w / 32 on.  One count, one scan, one fill and one
-// sort serve all the views.
+// bitmap's words from v * 4^w / 32 on.
 #include "gxy_engine.cuh"
 #include "gxy_kernels.cuh"
+#include "gxy_radix.cuh"
 
+#include <algorithm>
 #include <vector>
 
 namespace gxy {
@@ -166,6 +187,230 @@ __global__ void k_sort_small_buckets(const uint32_t* __restrict__ starts, uint64
     }
 }
 
+// ---- The build by partition ------------------------------------------------
+constexpr uint32_t kPartBuckets = 4096;
+constexpr uint32_t kMaxParts = 16384;      // partitions of a group of views: their counts fit a block's shared memory
+constexpr int kPartThreads = 1024;
+constexpr int kBuildThreads = 512;
+constexpr uint32_t kStagedPositions = 7936;
+constexpr int kHeldWindows = 6;            // a thread holds in registers
+static_assert(kPartBuckets == 8 * kBuildThreads, "eight buckets a thread");
+
+struct PartView {
+    uint64_t base;   // of its first position, pad included
+    uint32_t n;      // windows
+    uint32_t pad_;
+};
+
+struct PartArgs {
+    const uint64_t* codes;
+    const uint32_t* valid;
+    const uint32_t* mask;
+    Pattern pat;
+    uint32_t step;
+    uint32_t n_views;           // of the group
+    const PartView* views;
+    uint32_t parts_per_view;
+    uint32_t parts;             // n_views * parts_per_view
+    uint32_t* hist;             // block x partition
+    uint32_t* part_start;       // totals, then starts
+    uint2* win;                 // the group's windows by partition: position, low word bits
+};
+
+// Calls f(partition, low word bits, position) for the block's share of the
+// windows.  A thread takes those that start in 16 positions from one read of 64
+// (read and reversed for each window alone they took 95 instructions apiece).
+template <typename F>
+__device__ __forceinline__ void for_windows(const PartArgs& a, F f) {
+    constexpr uint32_t kSpan = 16;
+    for (uint32_t v = 0; v < a.n_views; v++) {
+        const PartView view = a.views[v];
+        if (!view.n) continue;
+        const uint64_t last = (uint64_t)(view.n - 1) * a.step;   // the last window's position
+        const uint64_t spans = last / kSpan + 1, per = (spans + gridDim.x - 1) / gridDim.x;
+        const uint64_t beg = min(spans, per * blockIdx.x), end = min(spans, beg + per);
+        for (uint64_t x = beg + threadIdx.x; x < end; x += kPartThreads) {
+            const uint64_t p0 = x * kSpan, g = view.base + p0;
+            // The first window at or after p0, counted from there.
+            const uint32_t first = a.step == 1 ? 0u : (uint32_t)(((p0 + a.step - 1) / a.step) * a.step - p0);
+            if (first >= kSpan) continue;
+            const uint32_t stop = (uint32_t)min((uint64_t)kSpan, last - p0 + 1);
+            const uint64_t hi = rev_pairs64(load_codes32(a.codes, g)), lo = rev_pairs64(load_codes32(a.codes, g + 32));
+            const uint32_t ok0 = load_bits32(a.valid, g) & ~load_bits32(a.mask, g);
+            const uint32_t ok1 = load_bits32(a.valid, g + 32) & ~load_bits32(a.mask, g + 32);
+#pragma unroll 4
+            for (uint32_t j = first; j < stop; j += a.step) {
+                if ((__funnelshift_r(ok0, ok1, j) & a.pat.care_mask) != a.pat.care_mask) continue;
+                const uint32_t w = word_of_reversed(a.pat, j ? hi << (2 * j) | lo >> (64 - 2 * j) : hi);
+                f(v * a.parts_per_view + w / kPartBuckets, w % kPartBuckets, (uint32_t)p0 + j);
+            }
+        }
+    }
+}
+
+__global__ __launch_bounds__(kPartThreads, 1) void k_part_count(const __grid_constant__ PartArgs a) {
+    extern __shared__ uint32_t s_cnt[];
+    for (uint32_t i = threadIdx.x; i < a.parts; i += kPartThreads) s_cnt[i] = 0;
+    __syncthreads();
+    for_windows(a, [&](uint32_t p, uint32_t, uint32_t) { atomicAdd(&s_cnt[p], 1u); });
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < a.parts; i += kPartThreads) a.hist[(uint64_t)blockIdx.x * a.parts + i] = s_cnt[i];
+}
+
+// hist's columns become exclusive prefixes over the blocks, part_start the totals.
+__global__ void k_part_prefix(uint32_t* hist, uint32_t parts, uint32_t n_blocks, uint32_t* part_start) {
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= parts) return;
+    uint32_t run = 0;
+    for (uint32_t b0 = 0; b0 < n_blocks; b0 += 16) {
+        uint32_t c[16];
+#pragma unroll
+        for (uint32_t k = 0; k < 16; k++) c[k] = b0 + k < n_blocks ? hist[(uint64_t)(b0 + k) * parts + p] : 0u;
+#pragma unroll
+        for (uint32_t k = 0; k < 16; k++) {
+            if (b0 + k < n_blocks) hist[(uint64_t)(b0 + k) * parts + p] = run;
+            run += c[k];
+        }
+    }
+    part_start[p] = run;
+}
+
+__global__ __launch_bounds__(kPartThreads, 1) void k_part_scatter(const __grid_constant__ PartArgs a) {
+    extern __shared__ uint32_t s_cnt[];
+    for (uint32_t i = threadIdx.x; i < a.parts; i += kPartThreads)
+        s_cnt[i] = a.part_start[i] + a.hist[(uint64_t)blockIdx.x * a.parts + i];
+    __syncthreads();
+    for_windows(a, [&](uint32_t p, uint32_t low, uint32_t position) {
+        const uint32_t slot = atomicAdd(&s_cnt[p], 1u);
+        a.win[slot] = make_uint2(position, low);
+    });
+}
+
+// Partition p's buckets are first_bucket + p * kPartBuckets ..; their positions
+// start where the buckets before them end.  A partition of more positions than the
+// stage holds (a long repeat's) writes them to memory as they come.
+__global__ __launch_bounds__(kBuildThreads, 2) void k_part_build(const uint32_t* __restrict__ part_start, uint32_t parts,
+                                                                  const uint2* __restrict__ win, uint64_t first_bucket,
+                                                                  uint32_t* starts, uint32_t* positions,
+                                                                  uint32_t* __restrict__ occ, uint2* __restrict__ packed,
+                                                                  uint2* __restrict__ mid, uint32_t* n_mid,
+                                                                  uint2* __restrict__ big, uint32_t* n_big,
+                                                                  uint2* __restrict__ huge, uint32_t* n_huge) {
+    __shared__ __align__(16) uint32_t s_cnt[kPartBuckets];   // sizes, then cursors
+    __shared__ uint32_t s_pos[kStagedPositions];
+    __shared__ uint32_t s_warp[32];
+    __shared__ uint32_t s_total;
+    const uint32_t tid = threadIdx.x, lane = tid & 31;
+    // (the group before this one left its end here; written again with the same value)
+    const uint32_t base = first_bucket ? *reinterpret_cast<volatile uint32_t*>(starts + first_bucket) : 0u;
+    uint4* const mine = reinterpret_cast<uint4*>(s_cnt) + 2 * tid;
+    // A partition of up to 3,072 windows (at 10 M in 16.7 M buckets 2,441 on average)
+    // is read once, into registers, while the one before it is built; the count's
+    // atomics give each window its place in its bucket.
+    uint2 win_next[kHeldWindows];
+    uint32_t e0_next = 0, n_next = 0;
+    auto fetch = [&](uint32_t p) {
+        n_next = 0;
+        if (p >= parts) return;
+        e0_next = part_start[p];
+        n_next = part_start[p + 1] - e0_next;
+#pragma unroll
+        for (int k = 0; k < kHeldWindows; k++)
+            if (tid + k * kBuildThreads < n_next) win_next[k] = win[e0_next + tid + k * kBuildThreads];
+    };
+    fetch(blockIdx.x);
+    for (uint32_t p = blockIdx.x; p < parts; p += gridDim.x) {
+        const uint32_t e0 = e0_next, n = n_next;
+        const bool held = n <= kHeldWindows * kBuildThreads;
+        mine[0] = mine[1] = make_uint4(0, 0, 0, 0);
+        __syncthreads();
+        uint2 w[kHeldWindows];
+        uint32_t rank[kHeldWindows];
+#pragma unroll
+        for (int k = 0; k < kHeldWindows; k++) {
+            w[k] = win_next[k];
+            if (tid + k * kBuildThreads < n) rank[k] = atomicAdd(&s_cnt[w[k].y], 1u);
+        }
+        if (!held) {
+#pragma unroll 4
+            for (uint32_t i = tid + kHeldWindows * kBuildThreads; i < n; i += kBuildThreads) atomicAdd(&s_cnt[win[e0 + i].y], 1u);
+        }
+        fetch(p + gridDim.x);
+        __syncthreads();
+        uint32_t c[8], at[8], sum = 0;
+        {
+            const uint4 x = mine[0], y = mine[1];
+            c[0] = x.x; c[1] = x.y; c[2] = x.z; c[3] = x.w;
+            c[4] = y.x; c[5] = y.y; c[6] = y.z; c[7] = y.w;
+        }
+#pragma unroll
+        for (int k = 0; k < 8; k++) sum += c[k];
+        uint32_t run = block_excl_scan<kBuildThreads>(sum, s_warp, &s_total);
+        uint32_t sizes = 0, some = 0;
+#pragma unroll
+        for (int k = 0; k < 8; k++) {
+            at[k] = run;
+            run += c[k];
+            sizes |= c[k] < 15 ? c[k] << (4 * k) : 0xffffffffu;
+            some |= (c[k] ? 1u : 0u) << k;
+        }
+        mine[0] = make_uint4(at[0], at[1], at[2], at[3]);
+        mine[1] = make_uint4(at[4], at[5], at[6], at[7]);
+        const uint64_t g = first_bucket + (uint64_t)p * kPartBuckets + 8 * tid;
+        const uint32_t b = base + e0;
+        *reinterpret_cast<uint4*>(starts + g) = make_uint4(b + at[0], b + at[1], b + at[2], b + at[3]);
+        *reinterpret_cast<uint4*>(starts + g + 4) = make_uint4(b + at[4], b + at[5], b + at[6], b + at[7]);
+        if (packed) packed[g >> 3] = make_uint2(b + at[0], sizes);
+        some <<= 8 * (lane & 3);
+        some |= __shfl_xor_sync(kFull, some, 1);
+        some |= __shfl_xor_sync(kFull, some, 2);
+        if ((lane & 3) == 0) occ[g >> 5] = some;
+        if (p == parts - 1 && tid == 0) starts[first_bucket + (uint64_t)parts * kPartBuckets] = b + n;
+        __syncthreads();
+        const bool staged = n <= kStagedPositions;
+        auto place = [&](uint32_t* to) {
+            if (held) {
+#pragma unroll
+                for (int k = 0; k < kHeldWindows; k++)
+                    if (tid + k * kBuildThreads < n) to[s_cnt[w[k].y] + rank[k]] = w[k].x;
+            } else {
+#pragma unroll 4
+                for (uint32_t i = tid; i < n; i += kBuildThreads) {
+                    const uint2 x = win[e0 + i];
+                    to[atomicAdd(&s_cnt[x.y], 1u)] = x.x;
+                }
+            }
+            __syncthreads();
+#pragma unroll
+            for (int k = 0; k < 8; k++) {
+                if (c[k] < 2) continue;
+                if (c[k] > 8) {
+                    const uint2 e = make_uint2(b + at[k], c[k]);
+                    if (c[k] > kBlockBucket) huge[atomicAdd(n_huge, 1u)] = e;
+                    else if (c[k] > 32) big[atomicAdd(n_big, 1u)] = e;
+                    else mid[atomicAdd(n_mid, 1u)] = e;
+                    continue;
+                }
+                uint32_t* const x = to + at[k];
+                for (uint32_t i = 1; i < c[k]; i++) {
+                    const uint32_t y = x[i];
+                    uint32_t j = i;
+                    for (; j && x[j - 1] > y; j--) x[j] = x[j - 1];
+                    x[j] = y;
+                }
+            }
+        };
+        if (!staged) {
+            place(positions + b);
+        } else {
+            place(s_pos);
+            __syncthreads();
+            for (uint32_t i = tid; i < n; i += kBuildThreads) positions[b + i] = s_pos[i];
+        }
+        __syncthreads();
+    }
+}
+
 // Listed buckets of 4..32 positions, a warp each: a bitonic sort across the
 // lanes by shuffles.
 __global__ void k_sort_warp_buckets(const uint2* __restrict__ mid, const uint32_t* n_mid, uint32_t* __restrict__ pos) {
@@ -244,7 +489,10 @@ __global__ void k_window_records(const uint64_t* __restrict__ codes, const uint3
 
 }  // namespace
 
-void table_init() {}
+void table_init() {
+    cudaFuncSetAttribute(k_part_count, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxParts * 4);
+    cudaFuncSetAttribute(k_part_scatter, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxParts * 4);
+}
 
 void launch_window_records(const uint64_t* codes, const uint32_t* valid, uint64_t first, uint64_t n, uint32_t* rec,
                            cudaStream_t st) {
@@ -276,38 +524,85 @@ gxy_status atomic_build_views(const gxy_dseq* seq, uint32_t n_views, const uint6
     }
     const uint64_t n_mid_cap = total / 4 + 1, n_big_cap = total / 33 + 1,
                    n_huge_cap = total / (kBlockBucket + 1) + 1;
-    GXY_CK(W->tk0.ensure((G + 1) * 4));
     GXY_CK(W->tv0.ensure((n_mid_cap + n_big_cap + n_huge_cap) * 8));
     GXY_CK(W->tv1.ensure(64 + ((size_t)n_views + 1) * 4));
-    uint32_t* counts = W->tk0.as<uint32_t>();
     uint2* mid = W->tv0.as<uint2>();
     uint2* big = mid + n_mid_cap;
     uint2* huge = big + n_big_cap;
     uint32_t* ctr = W->tv1.as<uint32_t>();   // [0] big buckets, [1] huge buckets, [2] mid buckets
     uint32_t* first = ctr + 16;
-    GXY_CK(cudaMemsetAsync(counts, 0, (G + 1) * 4, st));
     GXY_CK(cudaMemsetAsync(ctr, 0, 12, st));
-    std::vector<SeqView> views(n_views);
-    for (uint32_t v = 0; v < n_views; v++) views[v] = view_of(seq, lo[v], hi[v]);
-    const int cblocks = 148 * 16;
-    for (uint32_t v = 0; v < n_views; v++) {
-        if (!nwin[v]) continue;
+    if (nw >= kPartBuckets && nw / kPartBuckets <= kMaxParts) {
+        const uint32_t ppv = (uint32_t)(nw / kPartBuckets), per_group = kMaxParts / ppv;
+        std::vector<PartView> spans(n_views);
+        for (uint32_t v = 0; v < n_views; v++) spans[v] = PartView{kPad + lo[v], nwin[v], 0};
+        uint64_t most = 0;   // windows of a group
+        for (uint32_t v0 = 0; v0 < n_views; v0 += per_group) {
+            uint64_t t = 0;
+            for (uint32_t v = v0; v < std::min(n_views, v0 + per_group); v++) t += nwin[v];
+            most = std::max(most, t);
+        }
+        // A block's share is 2,048 windows at least: below that its counts outweigh them.
+        const uint32_t max_blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(148, most / 2048));
+        const uint32_t max_parts = std::min(n_views, per_group) * ppv;
+        GXY_CK(W->tk0.ensure(n_views * sizeof(PartView) + ((uint64_t)max_blocks * max_parts + max_parts + 8) * 4));
+        GXY_CK(W->tk1.ensure(most * 8 + 64));
+        PartView* dspans = W->tk0.as<PartView>();
+        uint32_t* part_start = reinterpret_cast<uint32_t*>(dspans + n_views);   // (16-byte aligned)
+        GXY_CK(cudaMemcpyAsync(dspans, spans.data(), n_views * sizeof(PartView), cudaMemcpyHostToDevice, st));
+        for (uint32_t v0 = 0; v0 < n_views; v0 += per_group) {
+            PartArgs a;
+            a.codes = seq->codes;
+            a.valid = seq->valid;
+            a.mask = seq->mask;
+            a.pat = pat;
+            a.step = step;
+            a.n_views = std::min(per_group, n_views - v0);
+            a.views = dspans + v0;
+            a.parts_per_view = ppv;
+            a.parts = a.n_views * ppv;
+            a.part_start = part_start;
+            a.hist = part_start + ((a.parts + 1 + 3) & ~3u);
+            a.win = W->tk1.as<uint2>();
+            uint64_t t = 0;
+            for (uint32_t v = v0; v < v0 + a.n_views; v++) t += nwin[v];
+            const uint32_t blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(max_blocks, t / 2048));
+            count_launch(4);
+            k_part_count<<<blocks, kPartThreads, a.parts * 4, st>>>(a);
+            k_part_prefix<<<(a.parts + 63) / 64, 64, 0, st>>>(a.hist, a.parts, blocks, part_start);
+            scan_small(part_start, (int)a.parts, st);
+            k_part_scatter<<<blocks, kPartThreads, a.parts * 4, st>>>(a);
+            k_part_build<<<(int)std::min<uint32_t>(a.parts, 148 * 2), kBuildThreads, 0, st>>>(
+                part_start, a.parts, a.win, (uint64_t)v0 * nw, starts, positions, occ, packed, mid, ctr + 2, big, ctr, huge,
+                ctr + 1);
+        }
+    } else {
+        GXY_CK(W->tk0.ensure((G + 1) * 4));
+        uint32_t* counts = W->tk0.as<uint32_t>();
+        GXY_CK(cudaMemsetAsync(counts, 0, (G + 1) * 4, st));
+        std::vector<SeqView> views(n_views);
+        for (uint32_t v = 0; v < n_views; v++) views[v] = view_of(seq, lo[v], hi[v]);
+        const int cblocks = 148 * 16;
+        for (uint32_t v = 0; v < n_views; v++) {
+            if (!nwin[v]) continue;
+            count_launch();
+            k_count_words<<<(int)std::min<uint64_t>((nwin[v] + 255) / 256, cblocks), 256, 0, st>>>(
+                views[v], pat, step, nwin[v], counts + (uint64_t)v * nw);
+        }
+        // Global starts, and their copy back in counts: the fill's cursors (a
+        // fill that decremented the counts and read the start instead measured
+        // 169 us against 96 us: one more random load per window).
+        scan_u32(counts, starts, nullptr, G, G, true, nullptr, W->ps, st, counts);
+        for (uint32_t v = 0; v < n_views; v++) {
+            if (!nwin[v]) continue;
+            count_launch();
+            k_fill_buckets<<<(int)std::min<uint64_t>((nwin[v] + 255) / 256, cblocks), 256, 0, st>>>(
+                views[v], pat, step, nwin[v], counts + (uint64_t)v * nw, positions);
+        }
         count_launch();
-        k_count_words<<<(int)std::min<uint64_t>((nwin[v] + 255) / 256, cblocks), 256, 0, st>>>(
-            views[v], pat, step, nwin[v], counts + (uint64_t)v * nw);
+        k_sort_small_buckets<<<148 * 16, 256, 0, st>>>(starts, G, positions, occ, packed, mid, ctr + 2, big, ctr, huge, ctr + 1);
     }
-    // Global starts, and their copy back in counts: the fill's cursors (a
-    // fill that decremented the counts and read the start instead measured
-    // 169 us against 96 us: one more random load per window).
-    scan_u32(counts, starts, nullptr, G, G, true, nullptr, W->ps, st, counts);
-    for (uint32_t v = 0; v < n_views; v++) {
-        if (!nwin[v]) continue;
-        count_launch();
-        k_fill_buckets<<<(int)std::min<uint64_t>((nwin[v] + 255) / 256, cblocks), 256, 0, st>>>(
-            views[v], pat, step, nwin[v], counts + (uint64_t)v * nw, positions);
-    }
-    count_launch(4);
-    k_sort_small_buckets<<<148 * 16, 256, 0, st>>>(starts, G, positions, occ, packed, mid, ctr + 2, big, ctr, huge, ctr + 1);
+    count_launch(3);
     k_sort_warp_buckets<<<148 * 4, 256, 0, st>>>(mid, ctr + 2, positions);
     k_sort_block_buckets<<<148 * 2, 256, 0, st>>>(big, ctr, positions);
     k_view_firsts<<<1, 256, 0, st>>>(starts, nw, n_views, first);

@@ -592,3 +592,21 @@ def test_extend_step_edges(gxy, ctx, side):
                 h, ok = gxy.extend_hits(T, Q, m, gxy.HspParams(xd, 0), [at], [at], L, mode)
                 got = tuple(int(h[0][k]) for k in ("t_start", "q_start", "length", "score")) if ok[0] else None
                 assert got == o, (side, cut, xd, mode)
+
+
+@pytest.mark.parametrize("pattern", ["11111", "111111", "1101111", P12, "11101100110010101111", "11101100110110101111"])
+@pytest.mark.parametrize("n,step", [(0, 1), (25, 1), (4_000, 1), (40_000, 3), (1_200_000, 1)])
+def test_table_partitions(gxy, ctx, pattern, n, step):
+    # Tables of weight 6 to 13 are built by partition (4,096 buckets), the others
+    # (5 and 14 here) bucket by bucket: fewer windows than blocks' shares, partitions of
+    # more positions than the stage's 7,936 (a run of A, an AC repeat, weight 6's), and
+    # buckets of up to 8, 32, 4,096 and more positions.
+    rng = np.random.default_rng(n + len(pattern))
+    s = rand_ascii(rng, n, b"ACGTACGTACGTacgN")
+    if n > 4_000:
+        s = s[:n // 2] + b"A" * 9_000 + s[n // 2:] + b"AC" * 6_000 + s[:30] * 7 + s[100:130] * 31
+    tab = gxy.PosTable.build(gxy.PackedSeq.from_ascii(s), pattern, step, ctx=ctx)
+    starts, pos = tab.arrays()
+    ot = O.Table(O.pack_ascii(s), pattern, step, 0)
+    assert np.array_equal(starts, ot.starts()) and np.array_equal(pos, ot.positions())
+    tab.free()
