@@ -143,3 +143,24 @@ def test_large_copies(gxy, ctx, n):
     for t in threads:
         t.join()
     assert got == [True] * 4
+
+
+@pytest.mark.parametrize("n", [1, 15, 16, 17, 4095, 4096, 4097, 8191, 12_289, 70_000])
+def test_fasta_tiles(gxy, ctx, n):
+    # Bases are counted and gathered in tiles of 4,096 bytes, 16 a thread: files of n
+    # bytes after the first header whose further headers start or end beside the
+    # tiles' and threads' edges, headers longer than a tile, and tiles full of short ones.
+    rng = np.random.default_rng(n)
+    for case in range(4):
+        buf = bytearray(b">first\n" + rand_ascii(rng, n, b"ACGTacgtN\n\n \t\r"))
+        if case == 1:
+            for c in range(4096, len(buf) - 40, 4096):
+                at = c - 14 + int(rng.integers(0, 28))
+                buf[at:at + 9] = b"\n>h%05d\n" % (c % 99_999)
+        elif case == 2 and n > 5000:
+            buf[300:300 + 4500] = b"\n>long " + b"x>" * 2246 + b"\n"
+        elif case == 3:
+            short = b"".join(b">%d\nA%s" % (i, b"\n" * (i % 3)) if i % 3 else b">%d a\n" % i for i in range(n // 6))
+            buf = bytearray(b">first\n" + short.replace(b"A>", b"A\n>") + b"\nACGT")
+        data = bytes(buf)
+        same(gxy, gxy.parse_fasta(data, ctx), O.parse_fasta(data))
