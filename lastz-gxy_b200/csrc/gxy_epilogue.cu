@@ -463,11 +463,14 @@ static int epi_grid(uint64_t expected, uint64_t per, int sm_count) {
     return (int)std::max<uint64_t>(1, std::min<uint64_t>((expected + per - 1) / per, (uint64_t)sm_count));
 }
 
+// (At least 16 blocks: the expected count can be far off, and the blocks a launch
+// does not need return at once.)
 cudaError_t launch_sort_candidates(const EpiSort& a, uint64_t expected, int sm_count, cudaStream_t st) {
     EpiSort arg = a;
     void* args[] = {&arg};
     count_launch();
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_sort_candidates), dim3(epi_grid(expected, 128, sm_count)),
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_sort_candidates),
+                                       dim3(epi_grid(std::max<uint64_t>(expected, 16 * 128), 128, sm_count)),
                                        dim3(kEpiThreads), args, sizeof(EpiSmem), st);
 }
 

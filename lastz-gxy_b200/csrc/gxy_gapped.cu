@@ -106,7 +106,7 @@ struct GapArgs {
     const uint32_t* list;
     const uint64_t* base;
     uint64_t n_list;
-    // First pass: each CUDA block walks its sides' tracebacks into its own
+    // First pass: each warp walks its sides' tracebacks into its own
     // scratch of scratch_words words, then copies the runs out to a range of
     // exactly their number.
     uint32_t* scratch;

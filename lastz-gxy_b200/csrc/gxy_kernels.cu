@@ -377,8 +377,8 @@ __device__ __forceinline__ void scan_pair_any(SideScan& A, SideScan& B, uint32_t
 // bucket (src/pos_table.rs:102-108), neighbouring lanes to neighbouring slots.
 //
 // What bounds it: the latency of dependent reads (words, mask, bounds,
-// position) and the L2 sectors of the last two.  10 M windows against a table of
-// 10 M positions, one transition, 26.1 M hits: 0.38 ms, 101 M L2 sectors and
+// position) and the L2 sectors of the last two.  10 Mbp x 10 Mbp, one
+// transition, 26.1 M hits: 0.36 ms, 101 M L2 sectors and
 // 0.60 GB of DRAM traffic (with 13 occupancy bits and the plain starts read per
 // window 0.74 ms; with the masks and the plain starts, 64 MB that push the masks
 // and positions out of L2, 0.59 ms and 1.7 GB; four entries a lane at a time
@@ -506,186 +506,186 @@ __global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(cons
             word0 = word_of(a.pat, load_codes32(Q.codes, gq));
         }
         for (; g < g_end; g++) {
-        if (g == 0) windows += wv ? 1 : 0;
-        // Group g > 0: the words one transition (of care position g - 1) away, with
-        // a second one at a later position.
-        const uint32_t word = kMode != 0 && g ? word0 ^ (2u << (2 * (weight - g))) : word0;
-        uint32_t mask = 0;
-        if (wv) {
-            if (kMode == 0) {
-                mask = (__ldg(U->occ + (word >> 5)) >> (word & 31u)) & 1u;
-            } else if (kMode == 1) {
-                mask = __ldg(U->nbr + word);
+            if (g == 0) windows += wv ? 1 : 0;
+            // Group g > 0: the words one transition (of care position g - 1) away, with
+            // a second one at a later position.
+            const uint32_t word = kMode != 0 && g ? word0 ^ (2u << (2 * (weight - g))) : word0;
+            uint32_t mask = 0;
+            if (wv) {
+                if (kMode == 0) {
+                    mask = (__ldg(U->occ + (word >> 5)) >> (word & 31u)) & 1u;
+                } else if (kMode == 1) {
+                    mask = __ldg(U->nbr + word);
+                } else {
+                    for (uint32_t i = 0; i <= weight; i++) {
+                        const uint32_t w = i ? word ^ (2u << (2 * (weight - i))) : word;
+                        mask |= ((__ldg(U->occ + (w >> 5)) >> (w & 31u)) & 1u) << i;
+                    }
+                }
+                if (kMode != 0 && g) mask &= ~((2u << g) - 1u);
+            }
+            // ---- the masks' bits, listed: bucket word and lane of each.
+            const uint32_t mine = __popc(mask);
+            uint32_t pos = mine;
+#pragma unroll
+            for (int o = 1; o < 32; o <<= 1) {
+                const uint32_t y = __shfl_up_sync(kFull, pos, o);
+                if (lane >= o) pos += y;
+            }
+            const uint32_t n_ent = __shfl_sync(kFull, pos, 31);
+            if (n_ent == 0) continue;
+            pos -= mine;
+            __syncwarp();
+            if (kMode == 1) {   // (bit by bit: finding the next one set has a longer latency)
+                const uint32_t tagged = word | (uint32_t)lane << 27;
+                if (mask & 1u) ent[pos++] = tagged;
+                uint32_t flip = 2u << (2 * (weight - 1));
+#pragma unroll
+                for (uint32_t v = 1; v <= kNbrMaxWeight; v++, flip >>= 2)
+                    if ((mask >> v) & 1u) ent[pos++] = tagged ^ flip;
             } else {
-                for (uint32_t i = 0; i <= weight; i++) {
-                    const uint32_t w = i ? word ^ (2u << (2 * (weight - i))) : word;
-                    mask |= ((__ldg(U->occ + (w >> 5)) >> (w & 31u)) & 1u) << i;
+                while (mask) {
+                    const uint32_t v = __ffs(mask) - 1;
+                    mask &= mask - 1;
+                    ent[pos] = v ? word ^ (2u << (2 * (weight - v))) : word;
+                    who[pos] = (uint8_t)lane;
+                    pos++;
                 }
             }
-            if (kMode != 0 && g) mask &= ~((2u << g) - 1u);
-        }
-        // ---- the masks' bits, listed: bucket word and lane of each.
-        const uint32_t mine = __popc(mask);
-        uint32_t pos = mine;
+            __syncwarp();
+            // ---- their bounds: start, and size with the lane in the top bits, the first 64 entries' in
+            // registers, the others' in place of the words; and the item's hits.
+            uint32_t rb[K], rc[K], wtot = 0;
+            auto bounds = [&](uint32_t e0) {
+                uint32_t w[K];
 #pragma unroll
-        for (int o = 1; o < 32; o <<= 1) {
-            const uint32_t y = __shfl_up_sync(kFull, pos, o);
-            if (lane >= o) pos += y;
-        }
-        const uint32_t n_ent = __shfl_sync(kFull, pos, 31);
-        if (n_ent == 0) continue;
-        pos -= mine;
-        __syncwarp();
-        if (kMode == 1) {   // (bit by bit: finding the next one set has a longer latency)
-            const uint32_t tagged = word | (uint32_t)lane << 27;
-            if (mask & 1u) ent[pos++] = tagged;
-            uint32_t flip = 2u << (2 * (weight - 1));
+                for (int k = 0; k < K; k++) {
+                    w[k] = 0;
+                    rc[k] = 0;
+                    if (e0 + 32 * k + lane < n_ent) w[k] = ent[e0 + 32 * k + lane];
+                }
+                if (kMode == 1) {
+                    uint2 p[K];
 #pragma unroll
-            for (uint32_t v = 1; v <= kNbrMaxWeight; v++, flip >>= 2)
-                if ((mask >> v) & 1u) ent[pos++] = tagged ^ flip;
-        } else {
-            while (mask) {
-                const uint32_t v = __ffs(mask) - 1;
-                mask &= mask - 1;
-                ent[pos] = v ? word ^ (2u << (2 * (weight - v))) : word;
-                who[pos] = (uint8_t)lane;
-                pos++;
+                    for (int k = 0; k < K; k++)
+                        if (e0 + 32 * k + lane < n_ent) p[k] = __ldg(U->packed + ((w[k] & kWordBits) >> 3));
+#pragma unroll
+                    for (int k = 0; k < K; k++) {
+                        if (e0 + 32 * k + lane < n_ent) {
+                            const uint32_t sh = 4 * (w[k] & 7u), below = p[k].y & ((1u << sh) - 1u);
+                            rb[k] = p[k].x + __dp4a((below & 0x0f0f0f0fu) + ((below >> 4) & 0x0f0f0f0fu), 0x01010101u, 0u);
+                            uint32_t c = (p[k].y >> sh) & 15u;
+                            if (p[k].y == 0xffffffffu) {   // a bucket of 15 or more among the eight
+                                rb[k] = __ldg(U->starts + (w[k] & kWordBits));
+                                c = __ldg(U->starts + (w[k] & kWordBits) + 1) - rb[k];
+                            }
+                            wtot += c;
+                            rc[k] = min(c, kWordBits) | (w[k] & ~kWordBits);
+                        }
+                    }
+                } else {
+                    uint32_t h[K];
+#pragma unroll
+                    for (int k = 0; k < K; k++) {
+                        if (e0 + 32 * k + lane < n_ent) {
+                            rb[k] = __ldg(U->starts + w[k]);
+                            h[k] = __ldg(U->starts + w[k] + 1);
+                        }
+                    }
+#pragma unroll
+                    for (int k = 0; k < K; k++) {
+                        if (e0 + 32 * k + lane < n_ent) {
+                            wtot += h[k] - rb[k];
+                            rc[k] = min(h[k] - rb[k], kWordBits) | (uint32_t)who[e0 + 32 * k + lane] << 27;
+                        }
+                    }
+                }
+            };
+            for (uint32_t e0 = (n_ent - 1) & ~63u; e0; e0 -= 64) {
+                bounds(e0);
+#pragma unroll
+                for (int k = 0; k < K; k++) {
+                    if (e0 + 32 * k + lane < n_ent) {
+                        ent[e0 + 32 * k + lane] = rb[k];
+                        cnt[e0 - 64 + 32 * k + lane] = rc[k];
+                    }
+                }
             }
-        }
-        __syncwarp();
-        // ---- their bounds: start, and size with the lane in the top bits, the first 64 entries' in
-        // registers, the others' in place of the words; and the item's hits.
-        uint32_t rb[K], rc[K], wtot = 0;
-        auto bounds = [&](uint32_t e0) {
-            uint32_t w[K];
+            bounds(0);
+            wtot = __reduce_add_sync(kFull, wtot);
+            unsigned long long base = 0;
+            if (lane == 0) base = atomicAdd(a.hit_count, (unsigned long long)wtot);
+            // ---- entry e's first hit takes slot e, the second hits of the larger buckets
+            // come behind those, and so on: both 32 consecutive slots at a time.  The
+            // hits' order in the buffer is free (candidates are sorted by a unique
+            // (diagonal, t) key later).
+            uint32_t first[K];
 #pragma unroll
-            for (int k = 0; k < K; k++) {
-                w[k] = 0;
-                rc[k] = 0;
-                if (e0 + 32 * k + lane < n_ent) w[k] = ent[e0 + 32 * k + lane];
+            for (int k = 0; k < K; k++)   // on their way while the reservation comes back
+                if (32 * k + lane < n_ent) first[k] = __ldg(U->positions + rb[k]);
+            base = __shfl_sync(kFull, base, 0);
+            if (base + wtot > a.hit_cap) {
+                // The buffer is full: this item goes to the next pass, and the
+                // part of its reservation inside the buffer is marked unused.
+                if (lane == 0) defer(tile, g, wtot);
+                for (uint64_t j = base + lane; j < min((unsigned long long)a.hit_cap, base + wtot); j += 32)
+                    a.hits[a.hit_cap + j] = kNoHit;
+                if (g == 0) windows -= wv ? 1 : 0;
+                break;   // with the groups after it
             }
-            if (kMode == 1) {
-                uint2 p[K];
+            n_raw += lane == 0 ? wtot : 0;
+            const uint32_t q0 = (tile - u_lo) * 32;
+            uint64_t more = base + n_ent;   // where the next further hits go
+            for (uint32_t e0 = 0;;) {
 #pragma unroll
                 for (int k = 0; k < K; k++)
-                    if (e0 + 32 * k + lane < n_ent) p[k] = __ldg(U->packed + ((w[k] & kWordBits) >> 3));
+                    if (e0 + 32 * k + lane < n_ent)
+                        store_hit(a, base + e0 + 32 * k + lane, first[k], (q0 + (rc[k] >> 27)) * a.step, u);
 #pragma unroll
                 for (int k = 0; k < K; k++) {
-                    if (e0 + 32 * k + lane < n_ent) {
-                        const uint32_t sh = 4 * (w[k] & 7u), below = p[k].y & ((1u << sh) - 1u);
-                        rb[k] = p[k].x + __dp4a((below & 0x0f0f0f0fu) + ((below >> 4) & 0x0f0f0f0fu), 0x01010101u, 0u);
-                        uint32_t c = (p[k].y >> sh) & 15u;
-                        if (p[k].y == 0xffffffffu) {   // a bucket of 15 or more among the eight
-                            rb[k] = __ldg(U->starts + (w[k] & kWordBits));
-                            c = __ldg(U->starts + (w[k] & kWordBits) + 1) - rb[k];
+                    if (e0 + 32 * k >= n_ent) break;
+                    const uint32_t c = rc[k] & kWordBits, q = (q0 + (rc[k] >> 27)) * a.step;
+                    const bool big = c > 16;
+                    for (uint32_t j = 1;; j++) {
+                        const uint32_t m = __ballot_sync(kFull, c > j && !big);
+                        if (m == 0) break;
+                        if (c > j && !big)
+                            store_hit(a, more + __popc(m & ((1u << lane) - 1u)), __ldg(U->positions + rb[k] + j), q, u);
+                        more += __popc(m);
+                    }
+                    uint32_t bm = __ballot_sync(kFull, big);
+                    while (bm) {   // a large bucket is copied by the whole warp
+                        const int src = __ffs(bm) - 1;
+                        bm &= bm - 1;
+                        const uint32_t bb = __shfl_sync(kFull, rb[k], src);
+                        uint32_t cc = __shfl_sync(kFull, c, src);
+                        const uint32_t qq = __shfl_sync(kFull, q, src);
+                        if (cc == kWordBits) {   // its size did not fit: the next larger start ends it
+                            uint32_t lo = 0, hi = 1u << (2 * weight);
+                            while (lo < hi) {
+                                const uint32_t mid = lo + (hi - lo) / 2;
+                                if (U->starts[mid] > bb) hi = mid;
+                                else lo = mid + 1;
+                            }
+                            cc = U->starts[lo] - bb;
                         }
-                        wtot += c;
-                        rc[k] = min(c, kWordBits) | (w[k] & ~kWordBits);
+                        for (uint32_t j = 1 + lane; j < cc; j += 32)
+                            store_hit(a, more + j - 1, __ldg(U->positions + bb + j), qq, u);
+                        more += cc - 1;
                     }
                 }
-            } else {
-                uint32_t h[K];
+                e0 += 64;
+                if (e0 >= n_ent) break;
 #pragma unroll
                 for (int k = 0; k < K; k++) {
+                    rc[k] = 0;
                     if (e0 + 32 * k + lane < n_ent) {
-                        rb[k] = __ldg(U->starts + w[k]);
-                        h[k] = __ldg(U->starts + w[k] + 1);
-                    }
-                }
-#pragma unroll
-                for (int k = 0; k < K; k++) {
-                    if (e0 + 32 * k + lane < n_ent) {
-                        wtot += h[k] - rb[k];
-                        rc[k] = min(h[k] - rb[k], kWordBits) | (uint32_t)who[e0 + 32 * k + lane] << 27;
+                        rb[k] = ent[e0 + 32 * k + lane];
+                        rc[k] = cnt[e0 - 64 + 32 * k + lane];
+                        first[k] = __ldg(U->positions + rb[k]);
                     }
                 }
             }
-        };
-        for (uint32_t e0 = (n_ent - 1) & ~63u; e0; e0 -= 64) {
-            bounds(e0);
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                if (e0 + 32 * k + lane < n_ent) {
-                    ent[e0 + 32 * k + lane] = rb[k];
-                    cnt[e0 - 64 + 32 * k + lane] = rc[k];
-                }
-            }
-        }
-        bounds(0);
-        wtot = __reduce_add_sync(kFull, wtot);
-        unsigned long long base = 0;
-        if (lane == 0) base = atomicAdd(a.hit_count, (unsigned long long)wtot);
-        // ---- entry e's first hit takes slot e, the second hits of the larger buckets
-        // come behind those, and so on: both 32 consecutive slots at a time.  The
-        // hits' order in the buffer is free (candidates are sorted by a unique
-        // (diagonal, t) key later).
-        uint32_t first[K];
-#pragma unroll
-        for (int k = 0; k < K; k++)   // on their way while the reservation comes back
-            if (32 * k + lane < n_ent) first[k] = __ldg(U->positions + rb[k]);
-        base = __shfl_sync(kFull, base, 0);
-        if (base + wtot > a.hit_cap) {
-            // The buffer is full: this item goes to the next pass, and the
-            // part of its reservation inside the buffer is marked unused.
-            if (lane == 0) defer(tile, g, wtot);
-            for (uint64_t j = base + lane; j < min((unsigned long long)a.hit_cap, base + wtot); j += 32)
-                a.hits[a.hit_cap + j] = kNoHit;
-            if (g == 0) windows -= wv ? 1 : 0;
-            break;   // with the groups after it
-        }
-        n_raw += lane == 0 ? wtot : 0;
-        const uint32_t q0 = (tile - u_lo) * 32;
-        uint64_t more = base + n_ent;   // where the next further hits go
-        for (uint32_t e0 = 0;;) {
-#pragma unroll
-            for (int k = 0; k < K; k++)
-                if (e0 + 32 * k + lane < n_ent)
-                    store_hit(a, base + e0 + 32 * k + lane, first[k], (q0 + (rc[k] >> 27)) * a.step, u);
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                if (e0 + 32 * k >= n_ent) break;
-                const uint32_t c = rc[k] & kWordBits, q = (q0 + (rc[k] >> 27)) * a.step;
-                const bool big = c > 16;
-                for (uint32_t j = 1;; j++) {
-                    const uint32_t m = __ballot_sync(kFull, c > j && !big);
-                    if (m == 0) break;
-                    if (c > j && !big)
-                        store_hit(a, more + __popc(m & ((1u << lane) - 1u)), __ldg(U->positions + rb[k] + j), q, u);
-                    more += __popc(m);
-                }
-                uint32_t bm = __ballot_sync(kFull, big);
-                while (bm) {   // a large bucket is copied by the whole warp
-                    const int src = __ffs(bm) - 1;
-                    bm &= bm - 1;
-                    const uint32_t bb = __shfl_sync(kFull, rb[k], src);
-                    uint32_t cc = __shfl_sync(kFull, c, src);
-                    const uint32_t qq = __shfl_sync(kFull, q, src);
-                    if (cc == kWordBits) {   // its size did not fit: the next larger start ends it
-                        uint32_t lo = 0, hi = 1u << (2 * weight);
-                        while (lo < hi) {
-                            const uint32_t mid = lo + (hi - lo) / 2;
-                            if (U->starts[mid] > bb) hi = mid;
-                            else lo = mid + 1;
-                        }
-                        cc = U->starts[lo] - bb;
-                    }
-                    for (uint32_t j = 1 + lane; j < cc; j += 32)
-                        store_hit(a, more + j - 1, __ldg(U->positions + bb + j), qq, u);
-                    more += cc - 1;
-                }
-            }
-            e0 += 64;
-            if (e0 >= n_ent) break;
-#pragma unroll
-            for (int k = 0; k < K; k++) {
-                rc[k] = 0;
-                if (e0 + 32 * k + lane < n_ent) {
-                    rb[k] = ent[e0 + 32 * k + lane];
-                    rc[k] = cnt[e0 - 64 + 32 * k + lane];
-                    first[k] = __ldg(U->positions + rb[k]);
-                }
-            }
-        }
         }
       }
     }

@@ -18,9 +18,9 @@
 //     and the positions of its 4,096 buckets in shared memory, buckets of up to 8
 //     positions put in order there, all written once and in order.
 //
-// What bounds it: the scattered 8-byte writes of step 2 (73 us for 10 M windows),
+// What bounds it: the scattered 8-byte writes of step 2 (73 us for a 10 Mbp target),
 // in step 3 the instructions for the buckets, empty or not (47 us for 16.7 M of
-// them, 88 us with 10 M positions); step 1 takes 26 us.  Bucket by bucket the same
+// them, 88 us with a 10 Mbp target's positions); step 1 takes 26 us.  Bucket by bucket the same
 // table took 256 us (random atomics on 64 MB of counts, twice, a three-pass scan
 // and a copy of them), an all but empty one 95 us against 63.  Three and four
 // blocks an SM instead of two spill step 3's registers: 103 and 117 us.
