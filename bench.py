@@ -192,15 +192,15 @@ def table_bytes(npos: int, lt: int, weight: int = 12) -> float:
 
 
 def table_roofline(ms_list, npos, lt: int, peak: float, views: int = 1, workload: str = "", traffic=None) -> dict:
-    """PosTable::build on the device (counts, scan, fill through atomic
-    cursors, in-bucket sorts) against table_bytes; time = CUDA events around
+    """PosTable::build on the device (windows by partition, then each
+    partition's buckets in shared memory) against table_bytes; time = CUDA events around
     the whole build call (allocation and the host sync included).  For a
     multi-view build npos is a list of (positions, bp)."""
     ms = statistics.median(ms_list)
     b = sum(table_bytes(n, l) for n, l in npos) if views > 1 else table_bytes(npos if npos else lt, lt)
     ach = b / (ms / 1e3) / 1e9
-    out = {"bound": "hbm", "kernel": "table build (k_count_words + scan + k_fill_buckets + "
-                                     "k_sort_small_buckets / k_sort_block_buckets)",
+    out = {"bound": "hbm", "kernel": "table build (k_part_count + k_part_prefix + k_part_scatter + "
+                                     "k_part_build)",
            "achieved": round(ach, 1), "peak": peak, "unit": "GB/s", "frac": round(ach / peak, 4),
            "build_ms": round(ms, 3), "algorithmic_bytes": int(b)}
     if workload:
@@ -208,7 +208,7 @@ def table_roofline(ms_list, npos, lt: int, peak: float, views: int = 1, workload
     if traffic and "table_build" in traffic:
         tb = traffic["table_build"]
         out["traffic"] = int(sum(k["dram_read_bytes"] + k["dram_write_bytes"] for k in tb["kernels"].values()))
-        out["traffic_source"] = "measured: ncu DRAM bytes of the build's count, scan, fill and bucket-pass kernels " \
+        out["traffic_source"] = "measured: ncu DRAM bytes of the build's kernels " \
                                 "(profiles/kernel_traffic.json, %s)" % tb["workload"]
     return out
 
