@@ -116,8 +116,11 @@ TableMem::~TableMem() {
 namespace {
 
 // Tables of at least this many windows (a view, on average) carry neighbour
-// masks and packed bounds: writing 4^weight of them (48 MB, some 15 us, at weight
-// 12) then costs less than the searches of a query of that size save.
+// masks and packed bounds.  At weight 12 writing them (48 MB) takes 18 us; a query of
+// the target's size then takes, with one transition, 13 us of enumeration instead of
+// 22 at 130 kbp, 20 instead of 31 at 260, 26 instead of 44 at 530 and 41 instead of
+// 76 at 1.06 Mbp: from 2^19 on the first search repays it (with two transitions any
+// of these does: 40 instead of 83 us, 308 instead of 642 at 1.06 Mbp).
 constexpr uint64_t kNbrMinWindows = 1u << 19;
 
 // PosTable::build for n views [lo[v], hi[v]) of seq, as one sort; out[v] is
