@@ -97,6 +97,23 @@ struct Score {
     int32_t hspthresh;
 };
 
+// The hits of a tile's group: bucket sizes summed by 16-bit halves, which 32 bits
+// hold for up to 65,536 buckets of any size (32 windows over one repeat of 140 M
+// positions have more than 2^32 hits).  The halves can be reduced across a warp
+// before they are joined.
+struct HitSum {
+    uint32_t lo = 0, hi = 0;
+    __host__ __device__ __forceinline__ void add(uint32_t bucket) {
+        lo += bucket & 0xffffu;
+        hi += bucket >> 16;
+    }
+    __host__ __device__ __forceinline__ uint64_t total() const { return ((uint64_t)hi << 16) + lo; }
+};
+// Whether slots [base, base + hits) lie in a buffer of cap slots.
+__host__ __device__ __forceinline__ bool hits_fit(uint64_t base, uint64_t hits, uint64_t cap) {
+    return hits <= cap && base <= cap - hits;
+}
+
 __device__ __forceinline__ uint64_t load_codes32(const uint64_t* __restrict__ codes, uint64_t gp) {
     const uint64_t i = gp >> 5;
     const uint32_t s = (uint32_t)(gp & 31) * 2;

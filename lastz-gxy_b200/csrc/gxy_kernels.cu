@@ -555,7 +555,8 @@ __global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(cons
             __syncwarp();
             // ---- their bounds: start, and size with the lane in the top bits, the first 64 entries' in
             // registers, the others' in place of the words; and the item's hits.
-            uint32_t rb[K], rc[K], wtot = 0;
+            uint32_t rb[K], rc[K];
+            HitSum sum;
             auto bounds = [&](uint32_t e0) {
                 uint32_t w[K];
 #pragma unroll
@@ -579,7 +580,7 @@ __global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(cons
                                 rb[k] = __ldg(U->starts + (w[k] & kWordBits));
                                 c = __ldg(U->starts + (w[k] & kWordBits) + 1) - rb[k];
                             }
-                            wtot += c;
+                            sum.add(c);
                             rc[k] = min(c, kWordBits) | (w[k] & ~kWordBits);
                         }
                     }
@@ -595,7 +596,7 @@ __global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(cons
 #pragma unroll
                     for (int k = 0; k < K; k++) {
                         if (e0 + 32 * k + lane < n_ent) {
-                            wtot += h[k] - rb[k];
+                            sum.add(h[k] - rb[k]);
                             rc[k] = min(h[k] - rb[k], kWordBits) | (uint32_t)who[e0 + 32 * k + lane] << 27;
                         }
                     }
@@ -612,9 +613,11 @@ __global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(cons
                 }
             }
             bounds(0);
-            wtot = __reduce_add_sync(kFull, wtot);
+            sum.lo = __reduce_add_sync(kFull, sum.lo);
+            sum.hi = __reduce_add_sync(kFull, sum.hi);
+            const unsigned long long wtot = sum.total();
             unsigned long long base = 0;
-            if (lane == 0) base = atomicAdd(a.hit_count, (unsigned long long)wtot);
+            if (lane == 0) base = atomicAdd(a.hit_count, wtot);
             // ---- entry e's first hit takes slot e, the second hits of the larger buckets
             // come behind those, and so on: both 32 consecutive slots at a time.  The
             // hits' order in the buffer is free (candidates are sorted by a unique
@@ -624,7 +627,7 @@ __global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(cons
             for (int k = 0; k < K; k++)   // on their way while the reservation comes back
                 if (32 * k + lane < n_ent) first[k] = __ldg(U->positions + rb[k]);
             base = __shfl_sync(kFull, base, 0);
-            if (base + wtot > a.hit_cap) {
+            if (!hits_fit(base, wtot, a.hit_cap)) {
                 // The buffer is full: this item goes to the next pass, and the
                 // part of its reservation inside the buffer is marked unused.
                 if (lane == 0) defer(tile, g, wtot);
@@ -633,7 +636,7 @@ __global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(cons
                 if (g == 0) windows -= wv ? 1 : 0;
                 break;   // with the groups after it
             }
-            n_raw += lane == 0 ? wtot : 0;
+            n_raw += lane == 0 ? (uint32_t)wtot : 0;   // (no more than the buffer's slots)
             const uint32_t q0 = (tile - u_lo) * 32;
             uint64_t more = base + n_ent;   // where the next further hits go
             for (uint32_t e0 = 0;;) {
