@@ -24,6 +24,13 @@ namespace {
 
 constexpr int kEpiThreads = 512;
 constexpr int kEpiWarps = kEpiThreads / 32;
+// A cooperative launch starts when all of its blocks fit the device at once, so a
+// block must fit an SM beside what other streams run there: two a SM hold its
+// registers (64 a thread) and its 68 KB to half of one or less.  With 125 registers
+// a block took a whole SM, and a search waited for every SM to be empty: 4 streams
+// with a 2 Mbp request beside 40 small ones each took 140 ms and 85 ms a request on
+// average, against 70 and 10 now (same figures for three a SM, which spills).
+constexpr int kEpiPerSm = 2;
 constexpr int kEpiItems = 8;
 constexpr uint32_t kEpiTile = kEpiThreads * kEpiItems;
 constexpr uint32_t kSpinLimit = 1u << 24;   // polls of a grid barrier (seconds) before it gives up
@@ -319,7 +326,7 @@ __device__ void sort_by_ranks(EpiSmem& S, const EpiSort& a, uint32_t n, uint32_t
 // of the searches; above, two crossings of the buffers a digit.  By ranks and by
 // five digits: 721 candidates 10 and 22 us, 4,639 14 and 61, 15,346 22 and 68,
 // 32,187 48 and 69; with tiles of 2,048, 46,590 take 71 and 70, 64,123 96 and 68.
-__global__ __launch_bounds__(kEpiThreads, 1) void k_sort_candidates(const __grid_constant__ EpiSort a) {
+__global__ __launch_bounds__(kEpiThreads, kEpiPerSm) void k_sort_candidates(const __grid_constant__ EpiSort a) {
     extern __shared__ __align__(16) unsigned char epi_smem[];
     EpiSmem& S = *reinterpret_cast<EpiSmem*>(epi_smem);
     const uint32_t n = min(*a.n_dev, a.n_cap);
@@ -356,7 +363,7 @@ __device__ __forceinline__ bool hsp_less(const Hsp& x, const Hsp& y) {
 
 // The walk's flagged HSPs in candidate order, grouped by unit (stably), each
 // (unit, diagonal) run in (t_start, length, score) order.
-__global__ __launch_bounds__(kEpiThreads, 1) void k_finish_hsps(const __grid_constant__ EpiFinish a) {
+__global__ __launch_bounds__(kEpiThreads, kEpiPerSm) void k_finish_hsps(const __grid_constant__ EpiFinish a) {
     extern __shared__ __align__(16) unsigned char epi_smem[];
     EpiSmem& S = *reinterpret_cast<EpiSmem*>(epi_smem);
     const uint32_t n = min(*a.n_dev, a.n_cap), nb = epi_blocks(n);
