@@ -114,6 +114,14 @@ __host__ __device__ __forceinline__ bool hits_fit(uint64_t base, uint64_t hits, 
     return hits <= cap && base <= cap - hits;
 }
 
+// The blocks of a launch that take part when n items came, `per` a block: counts are
+// only known on the device, and inputs of repeats have hundreds of times the hits
+// that the sizes let one expect.  Grids are launched whole; the blocks past
+// these return at once.  The 8 spread what is little over SMs.
+__device__ __forceinline__ uint32_t live_blocks(uint64_t n, uint32_t per) {
+    return (uint32_t)min((uint64_t)gridDim.x, n / per + 8);
+}
+
 __device__ __forceinline__ uint64_t load_codes32(const uint64_t* __restrict__ codes, uint64_t gp) {
     const uint64_t i = gp >> 5;
     const uint32_t s = (uint32_t)(gp & 31) * 2;

@@ -500,18 +500,8 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
     // holds runs as several passes, each taking tiles until the buffer is
     // full and handing the tile that did not fit to the next pass, all on
     // the device.
-    double est = 1 << 20, exp_random = 0, exp_windows = 0;
-    for (const UnitPlan& u : units) {
-        exp_random += (double)u.nwin * n_var * u.avg_bucket;
-        exp_windows += (double)u.nwin;
-    }
-    est += 1.5 * exp_random;
-    // What the grids are sized for (every kernel takes any count): raw hits, the
-    // filter's survivors and the candidates, each with a share of the windows for
-    // what is homologous.
-    const uint64_t exp_raw = (uint64_t)(exp_random + exp_windows / 4) + 1;
-    const uint64_t exp_surv = use_filter ? (uint64_t)(exp_random / 16 + exp_windows / 4) + 1 : exp_raw;
-    const uint64_t exp_cands = (uint64_t)(exp_random / 32 + exp_windows / 8) + 1;
+    double est = 1 << 20;
+    for (const UnitPlan& u : units) est += 1.5 * (double)u.nwin * n_var * u.avg_bucket;
     {
         if (use_filter) {
             const uint64_t want_s = (uint64_t)std::min<double>((double)kMaxHitCap, (1 << 20) + est / kRawPerSurvivorSlot);
@@ -531,10 +521,8 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
         }
     }
     const int screen_per_sm = (int)std::max<uint32_t>(1, ctx->tuning.screen_blocks_per_sm);
-    const int blocks_screen = (int)std::min<uint64_t>((uint64_t)ctx->sm_count * screen_per_sm,
-                                                      exp_surv / (32 * std::max<uint32_t>(1, ctx->tuning.screen_warps)) + 8);
+    const int blocks_screen = ctx->sm_count * screen_per_sm;
     const int blocks_misc = ctx->sm_count * 4;
-    const int blocks_walk = (int)std::min<uint64_t>((uint64_t)blocks_misc, exp_cands / 32 + 8);
     const int walk_warps = ctx->tuning.walk_warps == 4 ? 4 : 8;
     GXY_CK(W->redo.ensure((size_t)2 * kRedoCap * sizeof(uint2)));
 
@@ -553,7 +541,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
             sv.hit_cap = W->surv_cap;
             sv.hit_count = survc;
             FilterIO io{sa.hits, hitc, sa.hit_cap, cnt + kCFiltNext};
-            launch_filter_hits(sv, io, exp_raw, ctx->sm_count, st);
+            launch_filter_hits(sv, io, ctx->sm_count, st);
             if (timing) cudaEventRecord(W->ev[3], st);
             launch_screen(sv, (int)ctx->tuning.screen_warps, screen_per_sm, blocks_screen, st);
         } else {
@@ -583,7 +571,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
         es.hist = W->ps.hist;
         es.bar = cnt + kCBar;
         GXY_CK(cudaMemsetAsync(cnt + kCWalk, 0, 64, st));   // the walk's cursor and the barriers
-        GXY_CK(launch_sort_candidates(es, exp_cands, ctx->sm_count, st));
+        GXY_CK(launch_sort_candidates(es, ctx->sm_count, st));
         const uint64_t* skeys = (npass & 1) ? es.k1 : es.k0;
         const uint32_t* sidx = (npass & 1) ? es.v1 : es.v0;
             WalkArgs wa;
@@ -604,7 +592,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
             wa.out_hsp = W->ohsp.as<Hsp>();
             wa.chunk_next = cnt + kCWalk;
             wa.n_units = nu;
-            launch_walk(wa, walk_warps, blocks_walk, st);
+            launch_walk(wa, walk_warps, blocks_misc, st);
             EpiFinish ef;
             memset(&ef, 0, sizeof(ef));
             ef.flag = W->flags.as<uint8_t>();
@@ -634,7 +622,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
                 fin = ef.hsp1;
                 fin_unit = ef.unit1;
             }
-            GXY_CK(launch_finish_hsps(ef, exp_cands, ctx->sm_count, st));
+            GXY_CK(launch_finish_hsps(ef, ctx->sm_count, st));
             if (records) {
                 // Driver records (src/driver.rs:371-391): stable LSD sort by
                 // (group, global t, q, span) over the unit-major HSP order, then

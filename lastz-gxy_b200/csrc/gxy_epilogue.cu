@@ -465,28 +465,20 @@ void epilogue_init() {
     cudaFuncSetAttribute(k_finish_hsps, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)sizeof(EpiSmem));
 }
 
-// Blocks for an expected count: one per `per` items, at most one per SM.
-static int epi_grid(uint64_t expected, uint64_t per, int sm_count) {
-    return (int)std::max<uint64_t>(1, std::min<uint64_t>((expected + per - 1) / per, (uint64_t)sm_count));
-}
-
-// (At least 16 blocks: the expected count can be far off, and the blocks a launch
-// does not need return at once.)
-cudaError_t launch_sort_candidates(const EpiSort& a, uint64_t expected, int sm_count, cudaStream_t st) {
+cudaError_t launch_sort_candidates(const EpiSort& a, int sm_count, cudaStream_t st) {
     EpiSort arg = a;
     void* args[] = {&arg};
     count_launch();
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_sort_candidates),
-                                       dim3(epi_grid(std::max<uint64_t>(expected, 16 * 128), 128, sm_count)),
-                                       dim3(kEpiThreads), args, sizeof(EpiSmem), st);
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_sort_candidates), dim3(sm_count), dim3(kEpiThreads),
+                                       args, sizeof(EpiSmem), st);
 }
 
-cudaError_t launch_finish_hsps(const EpiFinish& a, uint64_t expected, int sm_count, cudaStream_t st) {
+cudaError_t launch_finish_hsps(const EpiFinish& a, int sm_count, cudaStream_t st) {
     EpiFinish arg = a;
     void* args[] = {&arg};
     count_launch();
-    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_finish_hsps), dim3(epi_grid(expected, kEpiTile, sm_count)),
-                                       dim3(kEpiThreads), args, sizeof(EpiSmem), st);
+    return cudaLaunchCooperativeKernel(reinterpret_cast<const void*>(k_finish_hsps), dim3(sm_count), dim3(kEpiThreads), args,
+                                       sizeof(EpiSmem), st);
 }
 
 }  // namespace gxy

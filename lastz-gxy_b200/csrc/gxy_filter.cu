@@ -151,12 +151,16 @@ __device__ __forceinline__ void align96(const uint32_t (&w)[8], uint32_t s, uint
 __global__ __launch_bounds__(kFilterWarps * 32, 1) void k_filter_hits(const __grid_constant__ ScreenArgs a,
                                                                        const __grid_constant__ FilterIO io) {
     extern __shared__ __align__(16) unsigned char smem[];
-    unsigned char* lut = smem;
-    lut_fill(lut, a.fub);
-    __syncthreads();
     // Past the buffer's end the pass did not write (those tiles went to the
     // next pass).
     const uint32_t n_hits = (uint32_t)min(*io.raw_count, (unsigned long long)io.raw_cap);
+    // A hit a lane at most: small launches leave the rest of the GPU alone (each
+    // block fills its two 64 KB tables, each warp claims from the cursor).
+    const uint32_t n_blocks = live_blocks(n_hits, kFilterWarps * 32);
+    if (blockIdx.x >= n_blocks) return;
+    unsigned char* lut = smem;
+    lut_fill(lut, a.fub);
+    __syncthreads();
     const int lane = threadIdx.x & 31;
     // Word k of queued hit s at k * kQueue + s: t, q, unit, the right run and best,
     // the left ones, and the columns scanned << 2 | the sides that run (whose columns
@@ -167,7 +171,7 @@ __global__ __launch_bounds__(kFilterWarps * 32, 1) void k_filter_hits(const __gr
     const int32_t X = a.sc.xdrop, thresh = a.sc.hspthresh;
     const int32_t need = thresh - a.f_seed_max;
     const int32_t ub0 = a.fub[0];
-    const uint32_t n_warps = gridDim.x * kFilterWarps;
+    const uint32_t n_warps = n_blocks * kFilterWarps;
     const uint32_t chunk = a.f_claim ? a.f_claim : max(32u, min(512u, n_hits / max(1u, n_warps * 8u)) & ~31u);
     uint32_t wcur = 0, wend = 0, qn = 0;
     bool exhausted = false;
@@ -487,13 +491,9 @@ void filter_init() {
     cudaFuncSetAttribute(k_filter_hits, cudaFuncAttributeMaxDynamicSharedMemorySize, kFilterSmem);
 }
 
-void launch_filter_hits(const ScreenArgs& a, const FilterIO& io, uint64_t expected, int sm_count, cudaStream_t st) {
+void launch_filter_hits(const ScreenArgs& a, const FilterIO& io, int sm_count, cudaStream_t st) {
     count_launch();
-    // A hit a lane at most: small launches leave the rest of the GPU alone (each
-    // block fills its two 64 KB tables, each warp claims from the cursor).
-    const uint64_t want = (expected + kFilterWarps * 32 - 1) / (kFilterWarps * 32);
-    const int blocks = (int)std::max<uint64_t>(1, std::min<uint64_t>(want, (uint64_t)sm_count));
-    k_filter_hits<<<blocks, kFilterWarps * 32, kFilterSmem, st>>>(a, io);
+    k_filter_hits<<<sm_count, kFilterWarps * 32, kFilterSmem, st>>>(a, io);
 }
 
 void launch_occupancy(const uint32_t* starts, uint64_t num_words, uint32_t* occ, uint2* packed, cudaStream_t st) {

@@ -757,6 +757,10 @@ void launch_enumerate(const ScreenArgs& a, int sm_count, cudaStream_t st) {
 // ---------------------------------------------------------------------------
 template <int WARPS, int MINB>
 __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen_wide(const __grid_constant__ ScreenArgs a) {
+    // Past the buffer's end the pass did not write (those tiles went to the
+    // next pass).
+    const uint32_t n_hits = (uint32_t)min(*a.hit_count, (unsigned long long)a.hit_cap);
+    if (blockIdx.x >= live_blocks(n_hits, WARPS * 32)) return;
     __shared__ int32_t s_lut[16];
     if (threadIdx.x < 16) s_lut[threadIdx.x] = a.sc.sub[threadIdx.x];
     __syncthreads();
@@ -764,9 +768,6 @@ __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen_wide(const __grid_c
     const uint32_t lt = lanemask_lt();
     const uint32_t L = a.pat.len;
     const int32_t ambig = a.sc.ambig, xdrop = a.sc.xdrop, thresh = a.sc.hspthresh;
-    // Past the buffer's end the pass did not write (those tiles went to the
-    // next pass).
-    const uint32_t n_hits = (uint32_t)min(*a.hit_count, (unsigned long long)a.hit_cap);
     unsigned long long n_cols = 0;
     bool exhausted = false;
 
@@ -1046,6 +1047,11 @@ __device__ __forceinline__ int32_t seed_score(const SeqView& T, const SeqView& Q
 
 template <int WARPS, int MINB>
 __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen(const __grid_constant__ ScreenArgs a) {
+    // Past the buffer's end the pass did not write (those hits went to the
+    // next pass, or were lost with a survivor overflow, which reruns the launch).
+    const uint32_t n_hits = (uint32_t)min(*a.hit_count, (unsigned long long)a.hit_cap);
+    const uint32_t n_blocks = live_blocks(n_hits, WARPS * 32);
+    if (blockIdx.x >= n_blocks) return;
     __shared__ int32_t s_lut[16];     // raw column scores, index (t << 2) | q
     __shared__ int32_t s_plut[16];    // 256 * score - 1, index (q << 2) | t
     __shared__ int32_t s_duo[256];    // sum of two columns' scores, index (t2 << 4) | q2
@@ -1068,13 +1074,10 @@ __global__ __launch_bounds__(WARPS * 32, MINB) void k_screen(const __grid_consta
     int32_t top = ambig;
     for (int i = 0; i < 16; i++) top = max(top, a.sc.sub[i]);
     const int32_t seed_ub = top * (int32_t)L;
-    // Past the buffer's end the pass did not write (those hits went to the
-    // next pass, or were lost with a survivor overflow, which reruns the launch).
-    const uint32_t n_hits = (uint32_t)min(*a.hit_count, (unsigned long long)a.hit_cap);
     // Each warp claims hits in chunks (one atomic per chunk) and deals them
     // to its idle lanes; chunks shrink for small launches so that every warp
     // still gets work.
-    const uint32_t n_warps = gridDim.x * WARPS;
+    const uint32_t n_warps = n_blocks * WARPS;
     const uint32_t chunk = max(32u, min(256u, n_hits / max(1u, n_warps * 8u)));
     uint32_t wcur = 0, wend = 0;   // this warp's claimed, not yet dealt hits
     uint32_t n_cols = 0;
@@ -1327,19 +1330,20 @@ __device__ bool entropy_gate_warp(const SeqView& T, uint32_t ts, uint32_t te, in
 
 template <int WARPS>
 __global__ __launch_bounds__(WARPS * 32) void k_walk(const __grid_constant__ WalkArgs a) {
+    const uint32_t n = min(*a.n_dev, a.n_cap), n_blocks = live_blocks(n, 32);
+    if (blockIdx.x >= n_blocks) return;
     __shared__ int32_t s_lut[16];
     __shared__ WarpStage s_stage[WARPS];
     if (threadIdx.x < 16) s_lut[threadIdx.x] = a.sc.sub[threadIdx.x];
     __syncthreads();
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
-    const uint32_t n = min(*a.n_dev, a.n_cap);
     const uint32_t L = a.seed_len;
     // Chunks of sorted positions are claimed dynamically: a segment with
     // long candidates (full re-extension) can take far longer than the rest.  A
     // chunk is 32 positions where that leaves every warp four of them, and down to
     // one position in a small launch, whose time is that of the warp with the most
     // segments.
-    const uint32_t chunk = max(1u, min(32u, n / (gridDim.x * WARPS * 4u)));
+    const uint32_t chunk = max(1u, min(32u, n / (n_blocks * WARPS * 4u)));
     for (;;) {
         uint32_t r = 0;
         if (lane == 0) r = atomicAdd(a.chunk_next, 1u);

@@ -182,8 +182,7 @@ struct FilterIO {
     uint64_t raw_cap;
     uint32_t* cursor;      // zeroed by the caller
 };
-// expected: raw hits the grid is sized for (the kernel takes any number).
-void launch_filter_hits(const ScreenArgs& a, const FilterIO& io, uint64_t expected, int sm_count, cudaStream_t st);
+void launch_filter_hits(const ScreenArgs& a, const FilterIO& io, int sm_count, cudaStream_t st);
 // Per-device kernel attributes of the filter (its shared-memory table); call
 // once with the device current, before any stream capture.
 void filter_init();
@@ -238,8 +237,8 @@ struct EpiSort {
     uint32_t* hist;            // 256 words per block
     uint32_t* bar;
 };
-// Stable sort of (key, value) pairs; expected: the count the grid is sized for.
-cudaError_t launch_sort_candidates(const EpiSort& a, uint64_t expected, int sm_count, cudaStream_t st);
+// Sort of (key, value) pairs.
+cudaError_t launch_sort_candidates(const EpiSort& a, int sm_count, cudaStream_t st);
 
 struct EpiFinish {
     const uint8_t* flag;       // the walk's output, per sorted position
@@ -263,7 +262,7 @@ struct EpiFinish {
 };
 // The flagged HSPs, grouped by unit, each (unit, diagonal) run ordered by
 // (t_start, length, score).
-cudaError_t launch_finish_hsps(const EpiFinish& a, uint64_t expected, int sm_count, cudaStream_t st);
+cudaError_t launch_finish_hsps(const EpiFinish& a, int sm_count, cudaStream_t st);
 // Kernel attributes of the epilogue; once per device, before any capture.
 void epilogue_init();
 
