@@ -149,6 +149,9 @@ typedef struct {
 } gxy_tuning;
 gxy_status gxy_ctx_set_tuning(gxy_ctx* ctx, const gxy_tuning* t);
 gxy_status gxy_ctx_get_tuning(gxy_ctx* ctx, gxy_tuning* t);
+/* Polls a block of a search's kernels waits for the others before the search ends
+ * with GXY_ETIMEDOUT (0: the default, some seconds). */
+gxy_status gxy_ctx_set_barrier_polls(gxy_ctx* ctx, uint32_t polls);
 /* Device timing on the context's primary stream -- the stream every call
  * made from one host thread at a time runs on.  gxy_ctx_mark records CUDA
  * event `slot` (0..15) there; gxy_ctx_elapsed_ms waits for event b and

@@ -144,6 +144,7 @@ SIGNATURES = {
     "gxy_ctx_destroy": (C.c_int, [V]),
     "gxy_ctx_set_tuning": (C.c_int, [V, P(TuningC)]),
     "gxy_ctx_get_tuning": (C.c_int, [V, P(TuningC)]),
+    "gxy_ctx_set_barrier_polls": (C.c_int, [V, U32]),
     "gxy_ctx_mark": (C.c_int, [V, U32]),
     "gxy_ctx_elapsed_ms": (C.c_int, [V, U32, U32, P(C.c_double)]),
     "gxy_dseq_upload": (C.c_int, [V, P(PackedSeqC), P(V)]),

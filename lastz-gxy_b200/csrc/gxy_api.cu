@@ -416,6 +416,13 @@ gxy_status gxy_ctx_get_tuning(gxy_ctx* ctx, gxy_tuning* t) {
     return GXY_OK;
 }
 
+gxy_status gxy_ctx_set_barrier_polls(gxy_ctx* ctx, uint32_t polls) {
+    if (!ctx) return GXY_EINVAL;
+    std::lock_guard<std::mutex> g(ctx->mu);
+    ctx->barrier_polls = polls ? polls : kBarrierPolls;
+    return GXY_OK;
+}
+
 gxy_status gxy_dseq_upload(gxy_ctx* ctx, const gxy_packed_seq* host, gxy_dseq** out) {
     if (!ctx || !host || !out || (host->len && (!host->codes || !host->valid || !host->mask))) return GXY_EINVAL;
     if (host->len >= (1ull << 32)) {

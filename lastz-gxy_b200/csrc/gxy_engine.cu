@@ -570,6 +570,8 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
         es.npass = npass;
         es.hist = W->ps.hist;
         es.bar = cnt + kCBar;
+        es.gave_up = cnt + kCSortGaveUp;
+        es.polls = ctx->barrier_polls;
         GXY_CK(cudaMemsetAsync(cnt + kCWalk, 0, 64, st));   // the walk's cursor and the barriers
         GXY_CK(launch_sort_candidates(es, ctx->sm_count, st));
         const uint64_t* skeys = (npass & 1) ? es.k1 : es.k0;
@@ -592,6 +594,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
             wa.out_hsp = W->ohsp.as<Hsp>();
             wa.chunk_next = cnt + kCWalk;
             wa.n_units = nu;
+            wa.gave_up = cnt + kCSortGaveUp;
             launch_walk(wa, walk_warps, blocks_misc, st);
             EpiFinish ef;
             memset(&ef, 0, sizeof(ef));
@@ -608,6 +611,9 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
             ef.n_hsps = cnt + kCHsps;
             ef.hist = W->ps.hist;
             ef.bar = cnt + kCBar + 2;
+            ef.sort_gave_up = cnt + kCSortGaveUp;
+            ef.gave_up = cnt + kCFinishGaveUp;
+            ef.polls = ctx->barrier_polls;
             fin = ef.hsp0;
             fin_unit = ef.unit0;
             if (nu > 1) {
@@ -635,14 +641,14 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
                 if (rb_g + rb_t + rb_q + rb_l <= 64) {
                     const int sh_q = rb_l, sh_t = rb_l + rb_q, sh_g = rb_l + rb_q + rb_t;
                     launch_record_keys(fin, fin_unit, pl, nullptr, cnt + kCHsps, cap, 0, sh_g, sh_t, sh_q,
-                                       W->rk0.as<uint64_t>(), W->rv0.as<uint32_t>(), blocks_misc, st);
+                                       W->rk0.as<uint64_t>(), W->rv0.as<uint32_t>(), cnt + kCFinishGaveUp, blocks_misc, st);
                     const int np = plan_radix(0, rb_l + rb_q + rb_t + rb_g, 0, 0, rp, 16);
                     const int w = radix_sort_u64(W->rk0.as<uint64_t>(), W->rv0.as<uint32_t>(), W->rk1.as<uint64_t>(),
                                                  W->rv1.as<uint32_t>(), cnt + kCHsps, 0, cap, rp, np, W->ps, st);
                     perm = w ? W->rv1.as<uint32_t>() : W->rv0.as<uint32_t>();
                 } else {
                     launch_record_keys(fin, fin_unit, pl, nullptr, cnt + kCHsps, cap, 1, 0, 0, 0, W->rk0.as<uint64_t>(),
-                                       W->rv0.as<uint32_t>(), blocks_misc, st);
+                                       W->rv0.as<uint32_t>(), cnt + kCFinishGaveUp, blocks_misc, st);
                     int np = plan_radix(0, rb_l, 32, rb_q, rp, 16);
                     int w = radix_sort_u64(W->rk0.as<uint64_t>(), W->rv0.as<uint32_t>(), W->rk1.as<uint64_t>(),
                                            W->rv1.as<uint32_t>(), cnt + kCHsps, 0, cap, rp, np, W->ps, st);
@@ -651,16 +657,18 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
                     uint32_t* v2 = w ? W->rv0.as<uint32_t>() : W->rv1.as<uint32_t>();
                     uint64_t* k3 = w ? W->rk1.as<uint64_t>() : W->rk0.as<uint64_t>();
                     uint32_t* v3 = w ? W->rv1.as<uint32_t>() : W->rv0.as<uint32_t>();
-                    launch_record_keys(fin, fin_unit, pl, p1, cnt + kCHsps, cap, 2, 0, 0, 0, k2, v2, blocks_misc, st);
+                    launch_record_keys(fin, fin_unit, pl, p1, cnt + kCHsps, cap, 2, 0, 0, 0, k2, v2, cnt + kCFinishGaveUp,
+                                       blocks_misc, st);
                     np = plan_radix(0, rb_t, 32, rb_g, rp, 16);
                     w = radix_sort_u64(k2, v2, k3, v3, cnt + kCHsps, 0, cap, rp, np, W->ps, st);
                     perm = w ? v3 : v2;
                 }
-                launch_record_heads(fin, fin_unit, pl, perm, cnt + kCHsps, cap, W->flags.as<uint8_t>(), blocks_misc, st);
+                launch_record_heads(fin, fin_unit, pl, perm, cnt + kCHsps, cap, W->flags.as<uint8_t>(), cnt + kCFinishGaveUp,
+                                    blocks_misc, st);
                 scan_u8(W->flags.as<uint8_t>(), W->offsets.as<uint32_t>(), cnt + kCHsps, 0, cap, false, cnt + kCRecs,
                         W->ps, st);
                 launch_record_emit(fin, fin_unit, pl, perm, W->flags.as<uint8_t>(), W->offsets.as<uint32_t>(),
-                                   cnt + kCHsps, cap, W->rrec.as<Record>(), blocks_misc, st);
+                                   cnt + kCHsps, cap, W->rrec.as<Record>(), cnt + kCFinishGaveUp, blocks_misc, st);
             }
             GXY_CK(cudaMemcpyAsync(W->h_pinned, W->counters.p, kCounterWords * 4, cudaMemcpyDeviceToHost, st));
         return GXY_OK;
@@ -746,7 +754,7 @@ gxy_status run_units(gxy_ctx* ctx, Worker* W, const std::vector<UnitPlan>& units
             }
             const uint32_t np = hc[kCPass];
             const uint64_t tile_at = hc[kCTile], redo_left = hc[kCRedoN + (np & 1u)];
-            if (hc[kCBar + 1] || hc[kCBar + 3]) {
+            if (hc[kCSortGaveUp] || hc[kCFinishGaveUp]) {
                 set_error("a grid barrier of the epilogue ran out of time");
                 return GXY_ETIMEDOUT;
             }

@@ -33,7 +33,6 @@ constexpr int kEpiWarps = kEpiThreads / 32;
 constexpr int kEpiPerSm = 2;
 constexpr int kEpiItems = 8;
 constexpr uint32_t kEpiTile = kEpiThreads * kEpiItems;
-constexpr uint32_t kSpinLimit = 1u << 24;   // polls of a grid barrier (seconds) before it gives up
 
 struct EpiSmem {
     uint64_t keys[kEpiTile];
@@ -48,35 +47,41 @@ struct EpiSmem {
     uint32_t ok;
 };
 
-// Barrier of the first n blocks of a cooperative launch: bar[0] counts
-// arrivals (zero before the launch), bar[1] is set when a wait ran out.
-// False: some block gave up; the caller returns.
-__device__ __forceinline__ bool grid_barrier(uint32_t* bar, uint32_t n, uint32_t& phase, uint32_t* s_ok) {
-    if (n == 1) {
-        __syncthreads();
-        return true;
-    }
-    __syncthreads();
-    phase++;
-    if (threadIdx.x == 0) {
-        __threadfence();
-        atomicAdd(bar, 1u);
-        const uint32_t target = phase * n;
-        uint32_t seen = 0, polls = 0, ok = 1;
-        for (;;) {
-            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
-            if (seen >= target) break;
-            if (++polls > kSpinLimit) {
-                atomicExch(bar + 1, 1u);
-                ok = 0;
-                break;
-            }
+// Barrier of the first n blocks of a cooperative launch.  False: some block gave
+// up; the caller returns.
+struct GridBarrier {
+    uint32_t* bar;       // arrivals, zero before the launch
+    uint32_t* gave_up;
+    uint32_t polls;      // of a wait
+    uint32_t phase = 0;
+    __device__ GridBarrier(uint32_t* b, uint32_t* g, uint32_t p) : bar(b), gave_up(g), polls(p) {}
+    __device__ __forceinline__ bool wait(uint32_t n, uint32_t* s_ok) {
+        if (n == 1) {
+            __syncthreads();
+            return true;
         }
-        *s_ok = ok;
+        __syncthreads();
+        phase++;
+        if (threadIdx.x == 0) {
+            __threadfence();
+            atomicAdd(bar, 1u);
+            const uint32_t target = phase * n;
+            uint32_t seen = 0, ok = 1;
+            for (uint32_t p = 0;; p++) {
+                asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(seen) : "l"(bar) : "memory");
+                if (seen >= target) break;
+                if (p >= polls) {
+                    atomicExch(gave_up, 1u);
+                    ok = 0;
+                    break;
+                }
+            }
+            *s_ok = ok;
+        }
+        __syncthreads();
+        return *s_ok != 0;
     }
-    __syncthreads();
-    return *s_ok != 0;
-}
+};
 
 // The contiguous range of block b of nb when n items are split into whole tiles.
 __device__ __forceinline__ void epi_range(uint32_t n, uint32_t nb, uint32_t b, uint32_t& beg, uint32_t& end) {
@@ -91,7 +96,7 @@ __device__ __forceinline__ void epi_range(uint32_t n, uint32_t nb, uint32_t b, u
 template <typename K>
 __device__ bool epi_radix_pass(EpiSmem& S, const K* kin, const uint32_t* vin, K* kout, uint32_t* vout,
                                uint32_t n, uint32_t nb, int shift, int bits, uint32_t* hist,
-                               uint32_t* bar, uint32_t& phase) {
+                               GridBarrier& barrier) {
     const uint32_t dmask = (1u << bits) - 1;
     const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
     const uint32_t lt = lanemask_lt();
@@ -109,7 +114,7 @@ __device__ bool epi_radix_pass(EpiSmem& S, const K* kin, const uint32_t* vin, K*
         if (threadIdx.x < kRadixMax) all = S.hist[threadIdx.x];
     } else {
         if (threadIdx.x < kRadixMax) hist[blockIdx.x * kRadixMax + threadIdx.x] = S.hist[threadIdx.x];
-        if (!grid_barrier(bar, nb, phase, &S.ok)) return false;
+        if (!barrier.wait(nb, &S.ok)) return false;
         if (threadIdx.x < kRadixMax) {
 #pragma unroll 8
             for (uint32_t b = 0; b < nb; b++) {
@@ -180,7 +185,7 @@ __device__ bool epi_radix_pass(EpiSmem& S, const K* kin, const uint32_t* vin, K*
         if (threadIdx.x < kRadixMax) S.off[threadIdx.x] += S.tile_tot[threadIdx.x];
         __syncthreads();
     }
-    return grid_barrier(bar, nb, phase, &S.ok);
+    return barrier.wait(nb, &S.ok);
 }
 
 // Blocks that share n items: one per tile, as far as the grid has them.
@@ -250,7 +255,7 @@ constexpr uint32_t kMergeTiles = 32;
 constexpr uint32_t kMergeMax = kMergeTiles * 2 * kEpiThreads;
 
 template <int E>
-__device__ void sort_by_ranks(EpiSmem& S, const EpiSort& a, uint32_t n, uint32_t nb, uint32_t& phase) {
+__device__ void sort_by_ranks(EpiSmem& S, const EpiSort& a, uint32_t n, uint32_t nb, GridBarrier& barrier) {
     constexpr uint32_t kTile = E * kEpiThreads;
     const uint32_t nt = (n + kTile - 1) / kTile, tid = threadIdx.x;
     const bool odd = a.npass & 1;
@@ -281,7 +286,7 @@ __device__ void sort_by_ranks(EpiSmem& S, const EpiSort& a, uint32_t n, uint32_t
         }
     }
     if (nt == 1) return;
-    if (!grid_barrier(a.bar, nb, phase, &S.ok)) return;
+    if (!barrier.wait(nb, &S.ok)) return;
     // 128 neighbours of one tile a turn (their searches take almost the same
     // path), a quarter of the tiles by each four warps, four searches at a time.
     const uint32_t mine = tid & 127u, part = tid >> 7;
@@ -330,7 +335,7 @@ __global__ __launch_bounds__(kEpiThreads, kEpiPerSm) void k_sort_candidates(cons
     extern __shared__ __align__(16) unsigned char epi_smem[];
     EpiSmem& S = *reinterpret_cast<EpiSmem*>(epi_smem);
     const uint32_t n = min(*a.n_dev, a.n_cap);
-    uint32_t phase = 0;
+    GridBarrier barrier(a.bar, a.gave_up, a.polls);
     if (n <= kMergeMax && a.npass > 0) {
         // The smallest tiles of which there are at most kMergeTiles; as many blocks
         // as have 128 items to place.
@@ -338,8 +343,8 @@ __global__ __launch_bounds__(kEpiThreads, kEpiPerSm) void k_sort_candidates(cons
         if (blockIdx.x >= nb) return;
         if (a.clear)
             for (uint32_t i = blockIdx.x * kEpiThreads + threadIdx.x; i < n; i += nb * kEpiThreads) a.clear[i] = 0;
-        if (n <= kMergeMax / 2) sort_by_ranks<1>(S, a, n, nb, phase);
-        else sort_by_ranks<2>(S, a, n, nb, phase);
+        if (n <= kMergeMax / 2) sort_by_ranks<1>(S, a, n, nb, barrier);
+        else sort_by_ranks<2>(S, a, n, nb, barrier);
         return;
     }
     const uint32_t nb = epi_blocks(n);
@@ -349,7 +354,7 @@ __global__ __launch_bounds__(kEpiThreads, kEpiPerSm) void k_sort_candidates(cons
     for (int p = 0; p < a.npass; p++) {
         const bool odd = p & 1;
         if (!epi_radix_pass<uint64_t>(S, odd ? a.k1 : a.k0, odd ? a.v1 : a.v0, odd ? a.k0 : a.k1, odd ? a.v0 : a.v1, n, nb,
-                                      a.passes[p].shift, a.passes[p].bits, a.hist, a.bar, phase))
+                                      a.passes[p].shift, a.passes[p].bits, a.hist, barrier))
             return;
     }
 }
@@ -367,8 +372,12 @@ __global__ __launch_bounds__(kEpiThreads, kEpiPerSm) void k_finish_hsps(const __
     extern __shared__ __align__(16) unsigned char epi_smem[];
     EpiSmem& S = *reinterpret_cast<EpiSmem*>(epi_smem);
     const uint32_t n = min(*a.n_dev, a.n_cap), nb = epi_blocks(n);
+    if (*a.sort_gave_up) {
+        if (blockIdx.x == 0 && threadIdx.x == 0) *a.gave_up = 1;
+        return;
+    }
     if (blockIdx.x >= nb) return;
-    uint32_t phase = 0;
+    GridBarrier barrier(a.bar, a.gave_up, a.polls);
     uint32_t beg, end;
     epi_range(n, nb, blockIdx.x, beg, end);
     // Kept HSPs of the block's range, and of the ranges before it.
@@ -378,7 +387,7 @@ __global__ __launch_bounds__(kEpiThreads, kEpiPerSm) void k_finish_hsps(const __
     uint32_t base = 0, m = S.total;
     if (nb > 1) {
         if (threadIdx.x == 0) a.hist[blockIdx.x] = S.total;
-        if (!grid_barrier(a.bar, nb, phase, &S.ok)) return;
+        if (!barrier.wait(nb, &S.ok)) return;
         uint32_t c0 = 0, c1 = 0;
         for (uint32_t b = threadIdx.x; b < nb; b += kEpiThreads) {
             const uint32_t c = __ldcg(a.hist + b);
@@ -409,7 +418,7 @@ __global__ __launch_bounds__(kEpiThreads, kEpiPerSm) void k_finish_hsps(const __
         __syncthreads();
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) *a.n_hsps = m;
-    if (!grid_barrier(a.bar, nb, phase, &S.ok)) return;
+    if (!barrier.wait(nb, &S.ok)) return;
     Hsp* hsp = a.hsp0;
     uint32_t* unit = a.unit0;
     const uint32_t stride = nb * kEpiThreads, first = blockIdx.x * kEpiThreads + threadIdx.x;
@@ -418,8 +427,8 @@ __global__ __launch_bounds__(kEpiThreads, kEpiPerSm) void k_finish_hsps(const __
         for (int p = 0; p < a.npass; p++) {
             const bool odd = p & 1;
             if (!epi_radix_pass<uint32_t>(S, odd ? a.key1 : a.key0, odd ? a.perm1 : a.perm0, odd ? a.key0 : a.key1,
-                                          odd ? a.perm0 : a.perm1, m, nb, a.passes[p].shift, a.passes[p].bits, a.hist, a.bar,
-                                          phase))
+                                          odd ? a.perm0 : a.perm1, m, nb, a.passes[p].shift, a.passes[p].bits, a.hist,
+                                          barrier))
                 return;
         }
         const uint32_t* perm = (a.npass & 1) ? a.perm1 : a.perm0;
@@ -430,13 +439,13 @@ __global__ __launch_bounds__(kEpiThreads, kEpiPerSm) void k_finish_hsps(const __
         }
         hsp = a.hsp1;
         unit = a.unit1;
-        if (!grid_barrier(a.bar, nb, phase, &S.ok)) return;
+        if (!barrier.wait(nb, &S.ok)) return;
     }
     // Run heads from the unmodified array, then one thread per run sorts it;
     // runs are short and almost always in order already.
     for (uint32_t i = first; i < m; i += stride)
         a.head[i] = (i == 0 || unit[i - 1] != unit[i] || diag_of(hsp[i - 1]) != diag_of(hsp[i])) ? 1 : 0;
-    if (!grid_barrier(a.bar, nb, phase, &S.ok)) return;
+    if (!barrier.wait(nb, &S.ok)) return;
     for (uint32_t i = first; i < m; i += stride) {
         if (!a.head[i]) continue;
         uint32_t e = i + 1;

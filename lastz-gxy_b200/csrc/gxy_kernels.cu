@@ -1331,7 +1331,7 @@ __device__ bool entropy_gate_warp(const SeqView& T, uint32_t ts, uint32_t te, in
 template <int WARPS>
 __global__ __launch_bounds__(WARPS * 32) void k_walk(const __grid_constant__ WalkArgs a) {
     const uint32_t n = min(*a.n_dev, a.n_cap), n_blocks = live_blocks(n, 32);
-    if (blockIdx.x >= n_blocks) return;
+    if (blockIdx.x >= n_blocks || *a.gave_up) return;
     __shared__ int32_t s_lut[16];
     __shared__ WarpStage s_stage[WARPS];
     if (threadIdx.x < 16) s_lut[threadIdx.x] = a.sc.sub[threadIdx.x];
@@ -1495,7 +1495,8 @@ __device__ __forceinline__ uint64_t shl64(uint64_t x, int s) { return s >= 64 ? 
 
 __global__ void k_record_keys(const Hsp* hsp, const uint32_t* unit, const Place* place, const uint32_t* perm,
                               const uint32_t* n_dev, uint32_t n_cap, int mode, int sh_g, int sh_t, int sh_q,
-                              uint64_t* key, uint32_t* val) {
+                              uint64_t* key, uint32_t* val, const uint32_t* gave_up) {
+    if (*gave_up) return;
     const uint32_t n = min(*n_dev, n_cap);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         const uint32_t p = perm ? perm[i] : i;
@@ -1516,9 +1517,10 @@ __global__ void k_record_keys(const Hsp* hsp, const uint32_t* unit, const Place*
 
 void launch_record_keys(const Hsp* hsp, const uint32_t* unit, const Place* place, const uint32_t* perm,
                         const uint32_t* n_dev, uint32_t n_cap, int mode, int sh_g, int sh_t, int sh_q, uint64_t* key,
-                        uint32_t* val, int blocks, cudaStream_t st) {
+                        uint32_t* val, const uint32_t* gave_up, int blocks, cudaStream_t st) {
     count_launch();
-    k_record_keys<<<blocks, 256, 0, st>>>(hsp, unit, place, perm, n_dev, n_cap, mode, sh_g, sh_t, sh_q, key, val);
+    k_record_keys<<<blocks, 256, 0, st>>>(hsp, unit, place, perm, n_dev, n_cap, mode, sh_g, sh_t, sh_q, key, val,
+                                            gave_up);
 }
 
 __device__ __forceinline__ Record make_record(const Hsp* hsp, const uint32_t* unit, const Place* place,
@@ -1537,7 +1539,8 @@ __device__ __forceinline__ Record make_record(const Hsp* hsp, const uint32_t* un
 }
 
 __global__ void k_record_heads(const Hsp* hsp, const uint32_t* unit, const Place* place, const uint32_t* perm,
-                               const uint32_t* n_dev, uint32_t n_cap, uint8_t* flag) {
+                               const uint32_t* n_dev, uint32_t n_cap, uint8_t* flag, const uint32_t* gave_up) {
+    if (*gave_up) return;
     const uint32_t n = min(*n_dev, n_cap);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
         uint8_t head = 1;
@@ -1551,14 +1554,16 @@ __global__ void k_record_heads(const Hsp* hsp, const uint32_t* unit, const Place
 }
 
 void launch_record_heads(const Hsp* hsp, const uint32_t* unit, const Place* place, const uint32_t* perm,
-                         const uint32_t* n_dev, uint32_t n_cap, uint8_t* flag, int blocks, cudaStream_t st) {
+                         const uint32_t* n_dev, uint32_t n_cap, uint8_t* flag, const uint32_t* gave_up, int blocks,
+                         cudaStream_t st) {
     count_launch();
-    k_record_heads<<<blocks, 256, 0, st>>>(hsp, unit, place, perm, n_dev, n_cap, flag);
+    k_record_heads<<<blocks, 256, 0, st>>>(hsp, unit, place, perm, n_dev, n_cap, flag, gave_up);
 }
 
 __global__ void k_record_emit(const Hsp* hsp, const uint32_t* unit, const Place* place, const uint32_t* perm,
                               const uint8_t* flag, const uint32_t* offsets, const uint32_t* n_dev, uint32_t n_cap,
-                              Record* out) {
+                              Record* out, const uint32_t* gave_up) {
+    if (*gave_up) return;
     const uint32_t n = min(*n_dev, n_cap);
     for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x)
         if (flag[i]) out[offsets[i]] = make_record(hsp, unit, place, perm[i]);
@@ -1566,9 +1571,10 @@ __global__ void k_record_emit(const Hsp* hsp, const uint32_t* unit, const Place*
 
 void launch_record_emit(const Hsp* hsp, const uint32_t* unit, const Place* place, const uint32_t* perm,
                         const uint8_t* flag, const uint32_t* offsets, const uint32_t* n_dev, uint32_t n_cap,
-                        Record* out, int blocks, cudaStream_t st) {
+                        Record* out, const uint32_t* gave_up, int blocks, cudaStream_t st) {
     count_launch();
-    k_record_emit<<<blocks, 256, 0, st>>>(hsp, unit, place, perm, flag, offsets, n_dev, n_cap, out);
+    k_record_emit<<<blocks, 256, 0, st>>>(hsp, unit, place, perm, flag, offsets, n_dev, n_cap, out,
+                                            gave_up);
 }
 
 // ---------------------------------------------------------------------------

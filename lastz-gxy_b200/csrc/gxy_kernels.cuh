@@ -107,14 +107,15 @@ constexpr uint32_t kNoUnit = 0xffffffffu;
 //    [kCRedoN + 0/1] redo-list lengths, u64 [kCMaxFail] largest tile that
 //    did not fit the hit buffer, flags [kCSurvOver] and [kCRedoOver],
 //    [kCWorkPasses] passes that found raw hits, [kCWalk] walk cursor, then the
-//    epilogue's barriers [kCBar + 0, 2, 4] and their error flags [kCBar + 1, 3, 5];
+//    sort's and the finish's barriers [kCBar + 0, 2], [kCSortGaveUp] and
+//    [kCFinishGaveUp] (a wait there ran out of polls);
 //  - per pass (reset by k_pass_reset): u64 [kCHits] raw hits, u64 [kCSurv]
 //    survivors, [kCHitNext] screen cursor, [kCFiltNext] filter cursor,
 //    [kCRedoTake] redo-list cursor, [kCStop] the hit buffer is full.
 constexpr uint32_t kCTile = 0, kCHsps = 2, kCRecs = 4, kCStats = 8, kCPass = 128, kCStop = 160, kCRedoN = 192,
                    kCMaxFail = 224, kCSurvOver = 256, kCRedoOver = 288, kCWorkPasses = 320, kCCand = 1024,
                    kCHitNext = 2048, kCRedoTake = 2560, kCHits = 3072, kCSurv = 3328, kCWalk = 3584,
-                   kCFiltNext = 3840, kCBar = kCWalk + 8;
+                   kCFiltNext = 3840, kCBar = kCWalk + 8, kCSortGaveUp = kCBar + 1, kCFinishGaveUp = kCBar + 3;
 constexpr uint32_t kCounterWords = 4096;
 // Tiles a pass can hand to the next one (two lists of this many).
 constexpr uint32_t kRedoCap = 1u << 16;
@@ -217,6 +218,7 @@ struct WalkArgs {
     Hsp* out_hsp;              // per sorted position
     uint32_t* chunk_next;      // work counter: chunks of 32 sorted positions (zeroed by the caller)
     uint32_t n_units;          // units of the launch (one unit: every segment is walked in one pass)
+    const uint32_t* gave_up;   // nothing is read when this is set: the sort did not finish
 };
 // Diagonal suppression (src/diag_hash.rs:34-53 as used at
 // src/seed_search.rs:92-116) over the candidates sorted by (diagonal, t),
@@ -224,8 +226,11 @@ struct WalkArgs {
 void launch_walk(const WalkArgs& a, int warps_per_block, int blocks, cudaStream_t st);
 
 // The launch's epilogue kernels (gxy_epilogue.cu): cooperative launches that
-// use as many of their blocks as the device-side count needs.  bar: two words,
-// zero before the launch; bar[1] is set when a grid barrier gave up.
+// use as many of their blocks as the device-side count needs.  bar: the barrier's
+// arrivals, zero before the launch.  A block whose wait takes more than `polls`
+// sets *gave_up and returns, the outputs unfinished: what follows on the stream
+// looks at *gave_up before it reads them, and the host ends the call.
+constexpr uint32_t kBarrierPolls = 1u << 24;   // some seconds
 struct EpiSort {
     uint64_t *k0, *k1;         // keys and values, ping-ponged: the result is in 0 when npass is even
     uint32_t *v0, *v1;
@@ -236,6 +241,8 @@ struct EpiSort {
     int npass;
     uint32_t* hist;            // 256 words per block
     uint32_t* bar;
+    uint32_t* gave_up;
+    uint32_t polls;
 };
 // Sort of (key, value) pairs.
 cudaError_t launch_sort_candidates(const EpiSort& a, int sm_count, cudaStream_t st);
@@ -259,6 +266,9 @@ struct EpiFinish {
     uint32_t* n_hsps;
     uint32_t* hist;
     uint32_t* bar;
+    const uint32_t* sort_gave_up;   // then this launch has given up too
+    uint32_t* gave_up;
+    uint32_t polls;
 };
 // The flagged HSPs, grouped by unit, each (unit, diagonal) run ordered by
 // (t_start, length, score).
@@ -285,18 +295,20 @@ struct Record {
 // Sort keys of the records.  mode 0: (group, t, q, span) packed into one u64
 // with the given shifts (span at bit 0); mode 1: (q << 32) | span; mode 2:
 // (group << 32) | t.  t = t_start + the unit's t_offset.  HSP i is
-// hsp[perm[i]] (perm may be null: the identity); val[i] = that index.
+// hsp[perm[i]] (perm may be null: the identity); val[i] = that index.  None of the
+// record kernels reads anything when *gave_up is set.
 void launch_record_keys(const Hsp* hsp, const uint32_t* unit, const Place* place, const uint32_t* perm,
                         const uint32_t* n_dev, uint32_t n_cap, int mode, int sh_g, int sh_t, int sh_q, uint64_t* key,
-                        uint32_t* val, int blocks, cudaStream_t st);
+                        uint32_t* val, const uint32_t* gave_up, int blocks, cudaStream_t st);
 // flag[i] = 1 when record perm[i] differs from record perm[i-1] in (group,
 // t, q, span) (dedup_by, src/driver.rs:381-387, keeps the first).
 void launch_record_heads(const Hsp* hsp, const uint32_t* unit, const Place* place, const uint32_t* perm,
-                         const uint32_t* n_dev, uint32_t n_cap, uint8_t* flag, int blocks, cudaStream_t st);
+                         const uint32_t* n_dev, uint32_t n_cap, uint8_t* flag, const uint32_t* gave_up, int blocks,
+                         cudaStream_t st);
 // out[offsets[i]] = the record of perm[i] for every flagged i.
 void launch_record_emit(const Hsp* hsp, const uint32_t* unit, const Place* place, const uint32_t* perm,
                         const uint8_t* flag, const uint32_t* offsets, const uint32_t* n_dev, uint32_t n_cap,
-                        Record* out, int blocks, cudaStream_t st);
+                        Record* out, const uint32_t* gave_up, int blocks, cudaStream_t st);
 
 // --- x-drop of given hits (test entry) ---------------------------------------
 void launch_extend_hits(SeqView T, SeqView Q, Score sc, const uint32_t* tpos, const uint32_t* qpos, uint64_t n,
