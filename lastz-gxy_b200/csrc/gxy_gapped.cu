@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(32) k_gapped_sides(const __grid_constant__ Gap
         target_load(0);
         __syncwarp();
         int32_t best = 0, thr = -a.ydrop;    // the best score of the rows so far, their threshold
-        I bi = 0;                            // the best's row
+        I bi = 0, be = 0;                    // the best's row, the end of that row's chunks
         uint32_t flags = 0;
         // The pool block being filled: kRows rows and kRows units of kCols cells at
         // most; blocks of the chain in order, n_blk of them for this side.
@@ -529,7 +529,10 @@ __global__ void __launch_bounds__(32) k_gapped_sides(const __grid_constant__ Gap
             }
             // Only an M can exceed the best: Y stays below an M of its row, X
             // below an M of an earlier one.
-            if (rv > best) bi = i;
+            if (rv > best) {
+                bi = i;
+                be = e_new;
+            }
             best = max(best, rv);
             thr = best - a.ydrop;
             e_prev = e_new;
@@ -659,6 +662,7 @@ __global__ void __launch_bounds__(32) k_gapped_sides(const __grid_constant__ Gap
             }
             blk_rows += (int32_t)(i - i0);
             if (i != i0) e_prev = cb + kCols;
+            if (bi > i0) be = cb + kCols;
 #pragma unroll
             for (int p = 0; p < S / 4; p++) {
                 rH[p * nblk + b] = make_int4(H[4 * p], H[4 * p + 1], H[4 * p + 2], H[4 * p + 3]);
@@ -699,7 +703,9 @@ __global__ void __launch_bounds__(32) k_gapped_sides(const __grid_constant__ Gap
                 if (h_at((int64_t)bi, (int64_t)mt.y + rel, b, b0) == best) at = mt.y + rel;
             bj = (int64_t)__reduce_min_sync(kFull, at);
         } else if (bi) {
-            bj = (int64_t)min(m, e_prev);   // a bound: the second pass finds the column
+            // A bound that the second pass reserves runs by: the column is in one of its
+            // row's chunks.  (A later row's can all lie to the left of it.)
+            bj = (int64_t)min(m, be);
         }
         res.score = best;
         res.t_span = (uint32_t)bi;

@@ -237,6 +237,32 @@ def test_gapped_second_pass(gxy):
     assert g2 == w and st2["second_pass_sides"] == 0
 
 
+@pytest.mark.parametrize("side", ["right", "left"])
+@pytest.mark.parametrize("seed,nsub", [(3, 185), (5, 180), (7, 184)])
+def test_gapped_second_pass_best_right_of_the_last_rows(gxy, side, seed, nsub):
+    # Target rows 1-352 match query columns 291-642 with nsub transitions, rows
+    # 270-371 columns 0-101: the best cell is near (352, 642) and its last gap ends
+    # before that of the other alignment, so that the last rows' cells lie in columns
+    # 96-607.  The second pass reserves for the best cell's column all the same.
+    rng = np.random.default_rng(seed)
+    bases = np.frombuffer(b"ACGT", np.uint8)
+    t, q = np.full(1000, ord("N"), np.uint8), np.full(760, ord("N"), np.uint8)
+    t[:372] = bases[rng.integers(0, 4, 372)]
+    q[:102] = t[270:372]
+    seg = t[1:353].copy()
+    at = rng.choice(352, nsub, replace=False)
+    seg[at] = bases[(np.searchsorted(bases, seg[at]) + 2) % 4]
+    q[291:643] = seg
+    t, q, anchor = t.tobytes(), q.tobytes(), (0, 0)
+    if side == "left":
+        t, q, anchor = t[::-1], q[::-1], (999, 759)
+    c = gxy.Context(0)
+    c.set_tuning(gapped_pool_blocks=8)
+    g, w, st = both(gxy, c, t, q, [anchor], thr=-10 ** 6)
+    assert g == w and st["second_pass_sides"] == 1
+    assert w[0][3] > 608   # (the best cell is right of the last rows' chunk)
+
+
 def test_gapped_rejects(gxy, ctx):
     dT = gxy.PackedSeq.from_ascii(b"ACGTACGTAC").to_device(ctx)
     m = gxy.ScoringMatrix.hoxd70()
