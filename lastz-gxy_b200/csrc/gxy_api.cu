@@ -147,6 +147,13 @@ gxy_status build_tables(gxy_ctx* ctx, const gxy_dseq* seq, uint32_t n, const uin
         set_error(std::string("table allocation: ") + cudaGetErrorString(e));
         return GXY_ENOMEM;
     }
+    // What only makes searches faster is left out where it does not fit.
+    auto optional = [&](void** p, size_t bytes) {
+        if (dev_alloc(p, bytes, st) == cudaSuccess) return true;
+        cudaGetLastError();
+        *p = nullptr;
+        return false;
+    };
     // The window records of the sequence words the views cover.
     {
         uint64_t lo_min = UINT64_MAX, hi_max = 0;
@@ -157,24 +164,30 @@ gxy_status build_tables(gxy_ctx* ctx, const gxy_dseq* seq, uint32_t n, const uin
         // (One word of margin: the filter's left windows start up to 32 before a view.)
         mem->rec_first = (kPad + lo_min) / 32 - 1;
         const uint64_t n_rec = (kPad + hi_max) / 32 + 1 - mem->rec_first;
-        e = dev_alloc((void**)&mem->rec, (size_t)n_rec * 32, st);
-        if (e != cudaSuccess) {
-            set_error(std::string("table allocation: ") + cudaGetErrorString(e));
-            return GXY_ENOMEM;
-        }
-        launch_window_records(seq->codes, seq->valid, mem->rec_first, n_rec, mem->rec, st);
+        if (optional((void**)&mem->rec, (size_t)n_rec * 32))
+            launch_window_records(seq->codes, seq->valid, mem->rec_first, n_rec, mem->rec, st);
     }
     std::vector<uint32_t> first((size_t)n + 1);
-    const bool masks = total >= kNbrMinWindows * n && pat.weight >= kNbrMinWeight && pat.weight <= kNbrMaxWeight;
-    if (masks) {
-        e = dev_alloc((void**)&mem->nbr, (size_t)G * 2, st);
-        if (e == cudaSuccess) e = dev_alloc((void**)&mem->packed, (size_t)G, st);
-        if (e != cudaSuccess) {
-            set_error(std::string("table allocation: ") + cudaGetErrorString(e));
-            return GXY_ENOMEM;
-        }
+    bool masks = total >= kNbrMinWindows * n && pat.weight >= kNbrMinWeight && pat.weight <= kNbrMaxWeight;
+    if (masks && !(optional((void**)&mem->packed, (size_t)G) && optional((void**)&mem->nbr, (size_t)G * 2))) {
+        dev_free(mem->packed);
+        mem->packed = nullptr;
+        masks = false;
     }
-    API_TRY(atomic_build_views(seq, n, lo, hi, pat, step, mem->starts, mem->positions, mem->occ, mem->packed, first.data(), W));
+    auto build = [&]() {
+        return atomic_build_views(seq, n, lo, hi, pat, step, mem->starts, mem->positions, mem->occ, mem->packed, first.data(), W);
+    };
+    gxy_status built = build();
+    if (built == GXY_ENOMEM && (masks || mem->rec)) {   // the build's own buffers come first
+        for (void* p : {(void*)mem->packed, (void*)mem->nbr, (void*)mem->rec}) dev_free(p);
+        mem->packed = nullptr;
+        mem->nbr = nullptr;
+        mem->rec = nullptr;
+        masks = false;
+        cudaGetLastError();
+        built = build();
+    }
+    API_TRY(built);
     if (masks) launch_neighbours(mem->occ, n, pat.weight, mem->nbr, st);
     std::vector<gxy_table*> made;
     auto fail = [&](gxy_status s) {

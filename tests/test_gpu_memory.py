@@ -1,0 +1,48 @@
+"""A table is built where only what it cannot do without fits the device's memory."""
+import os
+import subprocess
+import sys
+
+import pytest
+
+pytestmark = pytest.mark.gpu
+HERE = os.path.dirname(os.path.abspath(__file__))
+
+# (A process of its own: the memory that earlier calls' pools keep would do.)
+PROGRAM = """
+import sys
+sys.path.insert(0, {here!r})
+import conftest, torch, numpy as np
+gxy = sys.modules["lastz_gxy_b200"]
+length, pattern, room = {length}, {pattern!r}, {room} << 20
+rng = np.random.default_rng(4)
+bases = np.frombuffer(b"ACGT", np.uint8)[rng.integers(0, 4, length)].tobytes()
+c = gxy.Context(0)
+ds = gxy.DeviceSeq.from_ascii(bases, c)
+torch.cuda.mem_get_info()
+ballast = torch.empty(torch.cuda.mem_get_info()[0] - room, dtype=torch.uint8, device="cuda:0")
+few = gxy.PosTable.build_view(ds, 0, length, pattern, 1)
+del ballast
+torch.cuda.empty_cache()
+many = gxy.PosTable.build_view(ds, 0, length, pattern, 1)
+for x, y in zip(few.arrays(), many.arrays()):
+    assert np.array_equal(x, y)
+q = gxy.DeviceSeq.from_ascii(bases[1000:40_000], c)
+m = gxy.ScoringMatrix.hoxd70()
+for transitions in {transitions}:
+    sp = gxy.SearchParams(transitions=transitions)
+    a, b = gxy.search_device(few, q, m, sp), gxy.search_device(many, q, m, sp)
+    assert len(a) and a.tobytes() == b.tobytes()
+print("ok")
+"""
+
+
+@pytest.mark.parametrize("length,pattern,room,transitions", [
+    # 256 MB of bucket starts; neighbour masks and packed bounds would be 192 MB more.
+    (600_000, "1" * 13, 356, (0, 1, 2)),
+])
+def test_table_in_the_memory_that_is_left(length, pattern, room, transitions):
+    code = PROGRAM.format(here=HERE, length=length, pattern=pattern, room=room, transitions=transitions)
+    r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, CUDA_MODULE_LOADING="EAGER"))
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
