@@ -532,10 +532,11 @@ gxy_status atomic_build_views(const gxy_dseq* seq, uint32_t n_views, const uint6
     uint32_t* ctr = W->tv1.as<uint32_t>();   // [0] big buckets, [1] huge buckets, [2] mid buckets
     uint32_t* first = ctr + 16;
     GXY_CK(cudaMemsetAsync(ctr, 0, 12, st));
-    if (nw >= kPartBuckets && nw / kPartBuckets <= kMaxParts) {
-        const uint32_t ppv = (uint32_t)(nw / kPartBuckets), per_group = kMaxParts / ppv;
-        std::vector<PartView> spans(n_views);
-        for (uint32_t v = 0; v < n_views; v++) spans[v] = PartView{kPad + lo[v], nwin[v], 0};
+    bool by_partition = nw >= kPartBuckets && nw / kPartBuckets <= kMaxParts;
+    uint32_t ppv = 1, per_group = 1, max_blocks = 1;
+    if (by_partition) {
+        ppv = (uint32_t)(nw / kPartBuckets);
+        per_group = kMaxParts / ppv;
         uint64_t most = 0;   // windows of a group
         for (uint32_t v0 = 0; v0 < n_views; v0 += per_group) {
             uint64_t t = 0;
@@ -543,10 +544,21 @@ gxy_status atomic_build_views(const gxy_dseq* seq, uint32_t n_views, const uint6
             most = std::max(most, t);
         }
         // A block's share is 2,048 windows at least: below that its counts outweigh them.
-        const uint32_t max_blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(148, most / 2048));
+        max_blocks = (uint32_t)std::max<uint64_t>(1, std::min<uint64_t>(148, most / 2048));
         const uint32_t max_parts = std::min(n_views, per_group) * ppv;
-        GXY_CK(W->tk0.ensure(n_views * sizeof(PartView) + ((uint64_t)max_blocks * max_parts + max_parts + 8) * 4));
-        GXY_CK(W->tk1.ensure(most * 8 + 64));
+        // Eight bytes a window: where they do not fit, the table is built bucket by
+        // bucket, from four bytes a bucket.
+        by_partition = W->tk0.ensure(n_views * sizeof(PartView) + ((uint64_t)max_blocks * max_parts + max_parts + 8) * 4) ==
+                           cudaSuccess &&
+                       W->tk1.ensure(most * 8 + 64) == cudaSuccess;
+        if (!by_partition) {
+            cudaGetLastError();
+            W->tk1.release();
+        }
+    }
+    if (by_partition) {
+        std::vector<PartView> spans(n_views);
+        for (uint32_t v = 0; v < n_views; v++) spans[v] = PartView{kPad + lo[v], nwin[v], 0};
         PartView* dspans = W->tk0.as<PartView>();
         uint32_t* part_start = reinterpret_cast<uint32_t*>(dspans + n_views);   // (16-byte aligned)
         GXY_CK(cudaMemcpyAsync(dspans, spans.data(), n_views * sizeof(PartView), cudaMemcpyHostToDevice, st));

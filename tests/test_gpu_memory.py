@@ -40,6 +40,8 @@ print("ok")
 @pytest.mark.parametrize("length,pattern,room,transitions", [
     # 256 MB of bucket starts; neighbour masks and packed bounds would be 192 MB more.
     (600_000, "1" * 13, 356, (0, 1, 2)),
+    # 153 MB of positions, 88 MB of bucket lists; the partitions' windows would be 306 MB more.
+    (40_000_000, "1" * 8, 310, ()),
 ])
 def test_table_in_the_memory_that_is_left(length, pattern, room, transitions):
     code = PROGRAM.format(here=HERE, length=length, pattern=pattern, room=room, transitions=transitions)
