@@ -236,6 +236,8 @@ struct CopyPiece {
 };
 cudaError_t host_copy(gxy_ctx* ctx, const CopyPiece* pieces, int n, bool to_host, cudaStream_t st,
                       const std::function<void(size_t, size_t)>& seen = {});
+// Makes what copies of so many bytes use, if any: before requests that wait.
+void host_copy_warm(gxy_ctx* ctx, uint64_t bytes);
 // Frees in stream order on st: for sequences only st has used.
 void dseq_destroy_async(gxy_dseq* s, cudaStream_t st);
 gxy_status dseq_fill_host(gxy_dseq* d, const gxy_packed_seq* h, cudaStream_t st);

@@ -11,7 +11,7 @@
 // touched for the first time: 1.1 ms by the driver, 0.3 ms this way.
 //
 // The pinned memory (8 MB), streams, events and helper threads belong to the
-// context, are made at its first such copy and given back with it; a second copy at
+// context, are made at its first such copy (or by host_copy_warm) and given back with it; a second copy at
 // the same time takes the driver's path, as do smaller ones and memory that is
 // pinned already.
 #include <algorithm>
@@ -113,6 +113,12 @@ void HostCopy::destroy() {
     }
     if (pinned) cudaFreeHost(pinned);
     pinned = nullptr;
+}
+
+void host_copy_warm(gxy_ctx* ctx, uint64_t bytes) {
+    if (bytes < kStagedFrom) return;
+    std::lock_guard<std::mutex> hold(ctx->copy.mu);
+    prepare(ctx->copy, ctx->device);   // (without it copies take the driver's path)
 }
 
 cudaError_t host_copy(gxy_ctx* ctx, const CopyPiece* pieces, int n, bool to_host, cudaStream_t st,

@@ -400,6 +400,7 @@ gxy_status gxy_server_create(gxy_ctx* ctx, uint32_t n_tables, const gxy_table* c
     if (!o.big_bases) o.big_bases = 1ull << 20;
     if (!o.max_big_inflight) o.max_big_inflight = 1;
     s->opts = o;
+    if (o.warm_bases) host_copy_warm(ctx, o.warm_bases / 2);   // a query's codes, valid and mask bits
     for (uint32_t i = 0; i < o.max_streams; i++) s->threads.emplace_back(dispatcher, s);
     s->monitor = std::thread(memory_monitor, s);
     if (o.warm_bases) {

@@ -107,6 +107,26 @@ def test_warm_buffers_and_stats(gxy, setup):
         assert ref[i][0].tobytes() == warm[i][0].tobytes() and ref[i][1].tobytes() == warm[i][1].tobytes()
 
 
+def test_warm_server_makes_its_copy_threads_at_creation(gxy):
+    # The first query of 4 Mbp and more is copied by several threads through pinned
+    # memory: with warm_bases they are there before it comes.
+    import os
+    rng = np.random.default_rng(77)
+    t = rand_ascii(rng, 100_000, b"ACGT")
+    c = gxy.Context(0)
+    tab = gxy.PosTable.build(gxy.PackedSeq.from_ascii(t), P12, 1, ctx=c)
+    q = gxy.PackedSeq.from_ascii(t[:50_000] + b"N" * 5_000_000)
+    srv = gxy.Server([tab], gxy.ScoringMatrix.hoxd70(), gxy.SearchParams(), warm_bases=len(q))
+    try:
+        small = srv.submit(0, gxy.PackedSeq.from_ascii(t[:20_000]))
+        assert len(srv.wait(small)[0])
+        before = len(os.listdir("/proc/self/task"))
+        plus, _, _ = srv.wait(srv.submit(0, q))
+        assert len(plus) and len(os.listdir("/proc/self/task")) == before
+    finally:
+        srv.close()
+
+
 def test_wait_timeout_and_unknown_id(gxy, setup):
     _, tables, reqs = setup
     srv = gxy.Server(tables, gxy.ScoringMatrix.hoxd70(), gxy.SearchParams())
