@@ -654,6 +654,15 @@ gxy_status gxy_search(gxy_ctx* ctx, const gxy_table* table, const gxy_packed_seq
     WorkerLease L(ctx);
     if (!L.w) return L.err;
     Worker* W = L.w;
+    // Copies from pinned memory go on after host_copy's return: a return before the
+    // search's own synchronisation waits for them.
+    struct Settle {
+        cudaStream_t st;
+        bool done = false;
+        ~Settle() {
+            if (!done) cudaStreamSynchronize(st);
+        }
+    } settle{W->st};
     SeqView T = table_view(table);
     if (!same_host_seq(table, target)) {
         if (target->len != table->hi - table->lo) {
@@ -675,7 +684,9 @@ gxy_status gxy_search(gxy_ctx* ctx, const gxy_table* table, const gxy_packed_seq
     }
     API_TRY(dseq_fill_host(W->qstage, query, W->st));
     const SeqView Q = view_of(W->qstage, 0, query->len);
-    return search_impl(ctx, W, table, T, Q, params, out, stats);
+    const gxy_status s = search_impl(ctx, W, table, T, Q, params, out, stats);
+    settle.done = s == GXY_OK && n_windows(Q.len, table->pat.len, params->step) > 0;
+    return s;
 }
 
 gxy_status gxy_search_dseq(gxy_ctx* ctx, const gxy_table* table, const gxy_dseq* query,

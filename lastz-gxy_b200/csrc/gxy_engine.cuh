@@ -226,8 +226,8 @@ struct SeqLayout {
 };
 SeqLayout seq_layout(uint64_t len);
 // Copies pieces after what st holds; to the host it is done on return, to the
-// device the host memory is read (or staged by the driver) on return and st's later
-// work comes after it.  seen(lo, hi), if given, is called for the ranges of a
+// device pageable host memory is read (or staged by the driver) on return, pinned
+// memory when st is done with what it held then; st's later work comes after it.  seen(lo, hi), if given, is called for the ranges of a
 // single piece to the device, in no order and from several threads.
 struct CopyPiece {
     void* host;

@@ -164,3 +164,26 @@ def test_fasta_tiles(gxy, ctx, n):
             buf = bytearray(b">first\n" + short.replace(b"A>", b"A\n>") + b"\nACGT")
         data = bytes(buf)
         same(gxy, gxy.parse_fasta(data, ctx), O.parse_fasta(data))
+
+
+def test_search_that_returns_early_has_read_its_pinned_query(gxy):
+    # 256 MB of pinned arrays take 5 ms to the device: a search that is refused before
+    # it launches anything, or has no windows, leaves no copy running.
+    import time
+    import torch
+    c = gxy.Context(0)
+    tab = gxy.PosTable.build(gxy.PackedSeq.from_ascii(b"ACGT" * 5000), "1" * 12, 1, ctx=c)
+    t = gxy.PackedSeq.from_ascii(b"ACGT" * 5000)
+    n = 1 << 29
+    pinned = [torch.zeros(k, dtype=torch.uint8).pin_memory() for k in (n // 4, n // 8, n // 8)]
+    q = gxy.PackedSeq(*(x.numpy() for x in pinned), n)
+    assert q.codes.ctypes.data == pinned[0].data_ptr()
+    m = gxy.ScoringMatrix.hoxd70()
+    gxy.search(tab, t, gxy.PackedSeq.from_ascii(b"ACGT" * 5000), m, gxy.SearchParams())
+    for _ in range(3):
+        with pytest.raises(gxy.GxyError):
+            gxy.search(tab, t, q, m, gxy.SearchParams(step=0))
+        c.mark(0)
+        t0 = time.perf_counter()
+        c.elapsed_ms(0, 0)   # (waits for what the stream holds)
+        assert time.perf_counter() - t0 < 1e-3
