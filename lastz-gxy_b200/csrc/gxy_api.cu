@@ -75,15 +75,11 @@ gxy_status prune_table(gxy_table* t, uint32_t limit, Worker* W) {
     }
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) {
-        dev_free(new_starts);
-        dev_free(newpos);
+        dev_free({new_starts, newpos});
         set_error(std::string("table prune: ") + cudaGetErrorString(e));
         return GXY_ECUDA;
     }
-    if (t->own_arrays) {
-        dev_free(t->starts);
-        dev_free(t->positions);
-    }
+    if (t->own_arrays) dev_free({t->starts, t->positions});
     t->starts = new_starts;
     t->positions = newpos;
     t->pos_base = 0;
@@ -105,12 +101,7 @@ gxy_status prune_table(gxy_table* t, uint32_t limit, Worker* W) {
 
 TableMem::~TableMem() {
     cudaSetDevice(device);
-    dev_free(starts);
-    dev_free(positions);
-    dev_free(occ);
-    dev_free(nbr);
-    dev_free(packed);
-    dev_free(rec);
+    dev_free({starts, positions, occ, nbr, packed, rec});
 }
 
 namespace {
@@ -179,7 +170,7 @@ gxy_status build_tables(gxy_ctx* ctx, const gxy_dseq* seq, uint32_t n, const uin
     };
     gxy_status built = build();
     if (built == GXY_ENOMEM && (masks || mem->rec)) {   // the build's own buffers come first
-        for (void* p : {(void*)mem->packed, (void*)mem->nbr, (void*)mem->rec}) dev_free(p);
+        dev_free({mem->packed, mem->nbr, mem->rec});
         mem->packed = nullptr;
         mem->nbr = nullptr;
         mem->rec = nullptr;
@@ -192,10 +183,7 @@ gxy_status build_tables(gxy_ctx* ctx, const gxy_dseq* seq, uint32_t n, const uin
     std::vector<gxy_table*> made;
     auto fail = [&](gxy_status s) {
         for (gxy_table* t : made) {
-            if (t->own_arrays) {
-                dev_free(t->starts);
-                dev_free(t->positions);
-            }
+            if (t->own_arrays) dev_free({t->starts, t->positions});
             delete t;
         }
         return s;
@@ -634,10 +622,7 @@ gxy_status gxy_table_download(const gxy_table* t, uint32_t* starts, uint32_t* po
 gxy_status gxy_table_free(gxy_table* t) {
     if (!t) return GXY_OK;
     cudaSetDevice(t->device);
-    if (t->own_arrays) {
-        dev_free(t->starts);
-        dev_free(t->positions);
-    }
+    if (t->own_arrays) dev_free({t->starts, t->positions});
     t->mem.reset();
     dseq_destroy(t->owned);
     delete t;

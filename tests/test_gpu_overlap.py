@@ -46,3 +46,23 @@ def test_search_started_during_a_long_walk(gxy):
     beside = min(second(alone / 3) for _ in range(7))
     assert len(set(found)) == 1 and found[0]
     assert beside < 1.3 * alone, (alone, beside)
+
+
+def test_free_of_a_table_with_masks(gxy):
+    # A free waits for the device, which other threads' streams feel as well: once a
+    # table, however many arrays it has (one wait for each of six took 24 us, 17
+    # without the masks and packed bounds; 7 now).
+    c = gxy.Context(0)
+    t = gxy.DeviceSeq.from_ascii(rand_ascii(np.random.default_rng(8), 1_000_000, b"ACGT"), c)
+
+    def free_time(n):
+        times = []
+        for _ in range(300):
+            tab = gxy.PosTable.build_view(t, 0, n, P12, 1)
+            t0 = time.perf_counter()
+            tab.free()
+            times.append(time.perf_counter() - t0)
+        return sorted(times)[150]
+    plain = min(free_time(30_000) for _ in range(2))
+    masks = min(free_time(1_000_000) for _ in range(2))
+    assert masks < 1.25 * plain, (masks, plain)
