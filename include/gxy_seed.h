@@ -425,7 +425,7 @@ typedef struct {
     uint32_t warps_per_side;       /* warps that run one side */
     uint64_t max_side_rows;        /* rows of the longest side (sides run in parallel; rows are sequential) */
     uint64_t second_pass_sides;    /* sides run again with exactly sized traceback storage */
-    uint32_t cells_per_thread;     /* gapped_cells of the call (4 or 8) */
+    uint32_t cells_per_thread;     /* cells of a DP row one thread holds (4, 8 or 16) */
     uint32_t pad_;
     uint64_t second_pass_cells;    /* DP cells computed again by the second pass (not in cells) */
 } gxy_gapped_stats;

@@ -1312,7 +1312,7 @@ gxy_status gxy_gapped_extend(gxy_ctx* ctx, const gxy_dseq* target, uint64_t t_lo
         stats->second_pass_sides = pass2_sides;
         stats->second_pass_cells = pass2_cells;
         stats->warps_per_side = 1;
-        stats->cells_per_thread = (uint32_t)Sc;
+        stats->cells_per_thread = (uint32_t)plan.S;
         stats->max_side_rows = ctr[kCtrMaxRows];
     }
     return GXY_OK;

@@ -220,6 +220,18 @@ def test_gapped_eight_cells_per_thread(gxy):
         assert g == w, case
 
 
+@pytest.mark.parametrize("ydrop,cells,want", [(9400, 4, 16), (5000, 4, 8), (2000, 4, 4), (9400, 8, 8), (70000, 8, 16)])
+def test_gapped_statistics_name_the_cells_a_thread_held(gxy, ydrop, cells, want):
+    # By the band (301, 154 and 54 columns to a side), by the setting, and where rows
+    # are kept in 32 bits 16 whatever it is.
+    c = gxy.Context(0)
+    c.set_tuning(gapped_cells=cells)
+    rng = np.random.default_rng(5)
+    t = rand_ascii(rng, 600, b"ACGT")
+    g, w, st = both(gxy, c, t, t, [(300, 300)], ge=300 if ydrop > 65535 else 30, ydrop=ydrop)
+    assert g == w and st["cells_per_thread"] == want
+
+
 def test_gapped_second_pass(gxy):
     # A first pass with room for only a few traceback blocks: the sides that
     # ran out are extended again with exactly sized storage, and every result
