@@ -109,6 +109,18 @@ struct HitSum {
     }
     __host__ __device__ __forceinline__ uint64_t total() const { return ((uint64_t)hi << 16) + lo; }
 };
+// The windows that start in positions [p0, p0 + span), counted from p0: first, first +
+// stride .. below stop.  Windows start at multiples of step up to `last`, which is
+// not below p0.  (A stride of a whole span ends the loop; step itself could wrap.)
+struct SpanWindows {
+    uint32_t first, stop, stride;
+    __host__ __device__ __forceinline__ SpanWindows(uint64_t p0, uint64_t last, uint32_t step, uint32_t span) {
+        const uint64_t f = step == 1 ? 0 : (p0 + step - 1) / step * step - p0, n = last - p0 + 1;
+        first = f < span ? (uint32_t)f : span;
+        stop = n < span ? (uint32_t)n : span;
+        stride = step < span ? step : span;
+    }
+};
 // Whether slots [base, base + hits) lie in a buffer of cap slots.
 __host__ __device__ __forceinline__ bool hits_fit(uint64_t base, uint64_t hits, uint64_t cap) {
     return hits <= cap && base <= cap - hits;

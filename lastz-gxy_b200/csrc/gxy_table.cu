@@ -231,15 +231,13 @@ __device__ __forceinline__ void for_windows(const PartArgs& a, F f) {
         const uint64_t beg = min(spans, per * blockIdx.x), end = min(spans, beg + per);
         for (uint64_t x = beg + threadIdx.x; x < end; x += kPartThreads) {
             const uint64_t p0 = x * kSpan, g = view.base + p0;
-            // The first window at or after p0, counted from there.
-            const uint32_t first = a.step == 1 ? 0u : (uint32_t)(((p0 + a.step - 1) / a.step) * a.step - p0);
-            if (first >= kSpan) continue;
-            const uint32_t stop = (uint32_t)min((uint64_t)kSpan, last - p0 + 1);
+            const SpanWindows at(p0, last, a.step, kSpan);
+            if (at.first >= kSpan) continue;
             const uint64_t hi = rev_pairs64(load_codes32(a.codes, g)), lo = rev_pairs64(load_codes32(a.codes, g + 32));
             const uint32_t ok0 = load_bits32(a.valid, g) & ~load_bits32(a.mask, g);
             const uint32_t ok1 = load_bits32(a.valid, g + 32) & ~load_bits32(a.mask, g + 32);
 #pragma unroll 4
-            for (uint32_t j = first; j < stop; j += a.step) {
+            for (uint32_t j = at.first; j < at.stop; j += at.stride) {
                 if ((__funnelshift_r(ok0, ok1, j) & a.pat.care_mask) != a.pat.care_mask) continue;
                 const uint32_t w = word_of_reversed(a.pat, j ? hi << (2 * j) | lo >> (64 - 2 * j) : hi);
                 f(v * a.parts_per_view + w / kPartBuckets, w % kPartBuckets, (uint32_t)p0 + j);

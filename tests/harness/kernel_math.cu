@@ -41,6 +41,25 @@ int main() {
             }
     }
     if (hits_fit(~0ull - 1, 5, 4096)) return fail("reservation past 2^64", 1, 0);
+    // The windows of every span of 16 positions, against the multiples of the step.
+    for (uint64_t step : {1ull, 2ull, 3ull, 7ull, 15ull, 16ull, 17ull, 100ull, 65536ull, 0x80000000ull, 0xfffffff0ull,
+                          0xfffffff8ull, 0xfffffff9ull, 0xffffffffull}) {
+        for (uint64_t windows : {1ull, 2ull, 3ull, 50ull}) {
+            const uint64_t last = (windows - 1) * step;
+            if (last > 0xffffffffull) continue;
+            std::vector<uint64_t> got;
+            for (uint64_t w = 0; w < windows; w++)   // the spans that hold one, and their neighbours
+                for (int64_t x = (int64_t)(w * step / 16) - 1; x <= (int64_t)(w * step / 16) + 1; x++) {
+                    if (x < 0 || (uint64_t)x > last / 16 || (got.size() && got.back() / 16 >= (uint64_t)x)) continue;
+                    const SpanWindows at((uint64_t)x * 16, last, (uint32_t)step, 16);
+                    if (at.first < 16)
+                        for (uint32_t j = at.first; j < at.stop; j += at.stride) got.push_back((uint64_t)x * 16 + j);
+                }
+            if (got.size() != windows) return fail("windows of a span", got.size(), windows);
+            for (uint64_t w = 0; w < windows; w++)
+                if (got[w] != w * step) return fail("window", got[w], w * step);
+        }
+    }
     printf("ok\n");
     return 0;
 }
