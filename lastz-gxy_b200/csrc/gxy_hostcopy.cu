@@ -30,14 +30,23 @@ constexpr size_t kStagedFrom = 2u << 20, kHugePage = 2u << 20;
 
 cudaError_t prepare(HostCopy& h, int device) {
     if (h.pinned) return cudaSuccess;
-    cudaError_t e = cudaHostAlloc(reinterpret_cast<void**>(&h.pinned), 2 * kCopyThreads * kChunk, cudaHostAllocPortable);
+    void* pinned = nullptr;
+    cudaError_t e = cudaHostAlloc(&pinned, 2 * kCopyThreads * kChunk, cudaHostAllocPortable);
+    // (A call that fails may leave anything in its handle: kept only when it succeeds.)
+    if (e == cudaSuccess) h.pinned = static_cast<char*>(pinned);
     for (int i = 0; i < kCopyThreads && e == cudaSuccess; i++) {
-        e = cudaStreamCreateWithFlags(&h.st[i], cudaStreamNonBlocking);
-        for (int k = 0; k < 2 && e == cudaSuccess; k++) e = cudaEventCreateWithFlags(&h.ev[i][k], cudaEventDisableTiming);
+        cudaStream_t st;
+        e = cudaStreamCreateWithFlags(&st, cudaStreamNonBlocking);
+        if (e == cudaSuccess) h.st[i] = st;
+        for (int k = 0; k < 2 && e == cudaSuccess; k++) {
+            cudaEvent_t ev;
+            e = cudaEventCreateWithFlags(&ev, cudaEventDisableTiming);
+            if (e == cudaSuccess) h.ev[i][k] = ev;
+        }
     }
     if (e != cudaSuccess) {
-        cudaGetLastError();
         h.destroy();
+        cudaGetLastError();
         return e;
     }
     const int want = (int)std::min<unsigned>(kCopyThreads, std::max(1u, std::thread::hardware_concurrency())) - 1;

@@ -48,3 +48,42 @@ def test_table_in_the_memory_that_is_left(length, pattern, room, transitions):
     r = subprocess.run([sys.executable, "-c", code], capture_output=True, text=True, timeout=300,
                        env=dict(os.environ, CUDA_MODULE_LOADING="EAGER"))
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
+
+
+TWOBIT = """
+import sys
+sys.path.insert(0, {here!r})
+import conftest, struct, torch, numpy as np
+gxy = sys.modules["lastz_gxy_b200"]
+rng = np.random.default_rng(6)
+n, records = 25_000_000, 8
+names = [b"r%d" % k for k in range(records)]
+index, body, at = b"", [], 16 + sum(5 + len(x) for x in names)
+for x in names:
+    body.append(struct.pack("<4I", n, 0, 0, 0) + rng.integers(0, 256, n // 4, np.uint8).tobytes())
+    index += struct.pack("<B", len(x)) + x + struct.pack("<I", at)
+    at += len(body[-1])
+data = struct.pack("<4I", 0x1A412743, 0, records, 0) + index + b"".join(body)
+c = gxy.Context(0)
+torch.cuda.mem_get_info()
+ballast = torch.empty(torch.cuda.mem_get_info()[0] - ({room} << 20), dtype=torch.uint8, device="cuda:0")
+few = gxy.parse_2bit(data, c)
+del ballast
+torch.cuda.empty_cache()
+many = gxy.parse_2bit(data, c)
+for (a, x), (b, y) in zip(few, many):
+    x, y = x.to_host(), y.to_host()
+    assert a == b and len(x) == n
+    assert np.array_equal(x.codes, y.codes) and np.array_equal(x.valid, y.valid) and np.array_equal(x.mask, y.mask)
+print("ok")
+"""
+
+
+@pytest.mark.parametrize("room", [
+    # 95 MB of sequences, 48 of packed bases: none is left for the copies' streams.
+    130,
+])
+def test_2bit_in_the_memory_that_is_left(room):
+    r = subprocess.run([sys.executable, "-c", TWOBIT.format(here=HERE, room=room)], capture_output=True, text=True,
+                       timeout=300, env=dict(os.environ, CUDA_MODULE_LOADING="EAGER"))
+    assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
