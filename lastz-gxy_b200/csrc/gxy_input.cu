@@ -520,24 +520,41 @@ gxy_status gxy_parse_2bit(gxy_ctx* ctx, const uint8_t* bytes, uint64_t n, gxy_se
     if (recs.empty()) return cudaStreamSynchronize(st) == cudaSuccess ? GXY_OK : fail_set(out, "2bit decode", GXY_ECUDA);
     uint8_t* dpk = nullptr;
     uint32_t* drng = nullptr;
-    cudaError_t e = cudaMallocAsync((void**)&dpk, pk_bytes, st);
-    if (e == cudaSuccess) e = cudaMallocAsync((void**)&drng, (rng.size() + 2) * 4, st);
-    std::vector<CopyPiece> pieces;
-    for (const Rec& x : recs) pieces.push_back({const_cast<uint8_t*>(x.packed), dpk + x.pk_at, x.pb});
-    if (e == cudaSuccess) e = host_copy(ctx, pieces.data(), (int)pieces.size(), false, st);
+    cudaError_t e = cudaMallocAsync((void**)&drng, (rng.size() + 2) * 4, st);
     if (e == cudaSuccess && !rng.empty()) e = cudaMemcpyAsync(drng, rng.data(), rng.size() * 4, cudaMemcpyHostToDevice, st);
-    for (const Rec& x : recs) {
-        if (e != cudaSuccess) break;
-        gxy_dseq* d = out->seqs[x.i];
-        const uint64_t nw = (d->len + 31) / 32;
-        count_launch();
-        k_2bit_decode<<<(unsigned)std::min<uint64_t>((nw + 255) / 256, (uint64_t)ctx->sm_count * 16), 256, 0, st>>>(
-            dpk + x.pk_at, d->len, drng + x.rng_at, (uint32_t)(x.nn / 2), drng + x.rng_at + x.nn, (uint32_t)(x.nm / 2),
-            d->codes, d->valid, d->mask);
+    // All records at once, or as many at a time as the device has room for.
+    uint64_t room = pk_bytes;
+    for (size_t k0 = 0; e == cudaSuccess && k0 < recs.size();) {
+        const uint64_t at0 = recs[k0].pk_at;
+        size_t k1 = k0 + 1;
+        while (k1 < recs.size() && recs[k1].pk_at + recs[k1].pb - at0 <= room) k1++;
+        const uint64_t bytes_n = recs[k1 - 1].pk_at + recs[k1 - 1].pb - at0;
+        e = cudaMallocAsync((void**)&dpk, bytes_n, st);
+        if (e == cudaErrorMemoryAllocation && k1 - k0 > 1) {
+            e = cudaSuccess;
+            cudaGetLastError();
+            room = bytes_n / 2;
+            continue;
+        }
+        std::vector<CopyPiece> pieces;
+        for (size_t k = k0; k < k1; k++)
+            pieces.push_back({const_cast<uint8_t*>(recs[k].packed), dpk + (recs[k].pk_at - at0), recs[k].pb});
+        if (e == cudaSuccess) e = host_copy(ctx, pieces.data(), (int)pieces.size(), false, st);
+        for (size_t k = k0; e == cudaSuccess && k < k1; k++) {
+            const Rec& x = recs[k];
+            gxy_dseq* d = out->seqs[x.i];
+            const uint64_t nw = (d->len + 31) / 32;
+            count_launch();
+            k_2bit_decode<<<(unsigned)std::min<uint64_t>((nw + 255) / 256, (uint64_t)ctx->sm_count * 16), 256, 0, st>>>(
+                dpk + (x.pk_at - at0), d->len, drng + x.rng_at, (uint32_t)(x.nn / 2), drng + x.rng_at + x.nn,
+                (uint32_t)(x.nm / 2), d->codes, d->valid, d->mask);
+        }
+        if (dpk) cudaFreeAsync(dpk, st);
+        dpk = nullptr;
+        k0 = k1;
     }
     const cudaError_t synced = cudaStreamSynchronize(st);   // the host buffers die here
     if (e == cudaSuccess) e = synced;
-    if (dpk) cudaFreeAsync(dpk, st);
     if (drng) cudaFreeAsync(drng, st);
     if (e == cudaSuccess) e = cudaGetLastError();
     if (e != cudaSuccess) return fail_set(out, std::string("2bit decode: ") + cudaGetErrorString(e), GXY_ECUDA);

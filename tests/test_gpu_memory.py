@@ -82,6 +82,8 @@ print("ok")
 @pytest.mark.parametrize("room", [
     # 95 MB of sequences, 48 of packed bases: none is left for the copies' streams.
     130,
+    # Nor for the packed bases of all eight records at once.
+    112,
 ])
 def test_2bit_in_the_memory_that_is_left(room):
     r = subprocess.run([sys.executable, "-c", TWOBIT.format(here=HERE, room=room)], capture_output=True, text=True,
