@@ -8,7 +8,8 @@
 // one bucket space, view v's word w being bucket g = v * 4^w + w:
 //
 // Weights 6 to 13 (kPartBuckets and more words, at most kMaxParts partitions of
-// kPartBuckets a view) are built by partition, a group of views at a time:
+// kPartBuckets a view), from kMinParts partitions in all on, are built by
+// partition, a group of views at a time:
 //
 //  1. k_part_count: every block counts its share of the windows by partition, in
 //     shared memory;  k_part_prefix and a scan turn the counts into every block's
@@ -25,7 +26,7 @@
 // and a copy of them), an all but empty one 95 us against 63.  Three and four
 // blocks an SM instead of two spill step 3's registers: 103 and 117 us.
 //
-// The other weights, bucket by bucket:
+// The others, bucket by bucket:
 //
 //  1. k_count_words counts the windows of every bucket (atomics on an array
 //     that stays in L2 for a chromosome-sized view);
@@ -190,6 +191,11 @@ __global__ void k_sort_small_buckets(const uint32_t* __restrict__ starts, uint64
 // ---- The build by partition ------------------------------------------------
 constexpr uint32_t kPartBuckets = 4096;
 constexpr uint32_t kMaxParts = 16384;      // partitions of a group of views: their counts fit a block's shared memory
+// Fewer partitions than this leave step 3 too few blocks.  By partition and by bucket,
+// ms: weight 6, 2 Mbp (1 partition) 1.91 and 0.39; weight 8, 10 Mbp (16) 1.87 and 1.50;
+// weight 9, 40 Mbp (64) 6.12 and 5.76, 2 Mbp 0.16 and 0.17; 40 views of 100 kbp at
+// weight 7 (160) 0.43 and 0.63; weight 10, 2 Mbp (256) 0.12 and 0.18.
+constexpr uint32_t kMinParts = 128;
 constexpr int kPartThreads = 1024;
 constexpr int kBuildThreads = 512;
 constexpr uint32_t kStagedPositions = 7936;
@@ -530,11 +536,14 @@ gxy_status atomic_build_views(const gxy_dseq* seq, uint32_t n_views, const uint6
     uint32_t* ctr = W->tv1.as<uint32_t>();   // [0] big buckets, [1] huge buckets, [2] mid buckets
     uint32_t* first = ctr + 16;
     GXY_CK(cudaMemsetAsync(ctr, 0, 12, st));
-    bool by_partition = nw >= kPartBuckets && nw / kPartBuckets <= kMaxParts;
     uint32_t ppv = 1, per_group = 1, max_blocks = 1;
+    bool by_partition = nw >= kPartBuckets && nw / kPartBuckets <= kMaxParts;
     if (by_partition) {
         ppv = (uint32_t)(nw / kPartBuckets);
         per_group = kMaxParts / ppv;
+        by_partition = (uint64_t)std::min(n_views, per_group) * ppv >= kMinParts;
+    }
+    if (by_partition) {
         uint64_t most = 0;   // windows of a group
         for (uint32_t v0 = 0; v0 < n_views; v0 += per_group) {
             uint64_t t = 0;

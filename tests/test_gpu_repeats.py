@@ -4,7 +4,7 @@ import time
 import numpy as np
 import pytest
 
-from helpers import oracle_search
+from helpers import oracle_search, rand_ascii
 
 pytestmark = pytest.mark.gpu
 P12 = "1110100110010101111"
@@ -40,3 +40,32 @@ def test_search_of_a_satellite_uses_the_device(gxy, ctx):
     want, _ = oracle_search(t, q, P12, m, sp)
     assert len(want) > 100 and found[0] == found[1] == want.tobytes()
     assert best[0] < 1.5 * best[1], best
+
+
+def test_table_of_few_words_uses_the_device(gxy, ctx):
+    # 2 Mbp at weight 6: four times the buckets of weight 5, and not slower (one
+    # partition of buckets kept one block busy for 1.9 ms, weight 5 took 0.65).
+    seq = gxy.DeviceSeq.from_ascii(rand_ascii(np.random.default_rng(6), 2_000_000, b"ACGT"), ctx)
+
+    def build(weight):
+        times = []
+        for _ in range(12):
+            t0 = time.perf_counter()
+            gxy.PosTable.build_view(seq, 0, len(seq), "1" * weight, 1).free()
+            times.append(time.perf_counter() - t0)
+        return min(times)
+    assert build(6) < 1.2 * build(5)
+
+
+@pytest.mark.parametrize("pattern,views", [("111111", 1), ("111111", 127), ("111111", 128), ("11011011", 31),
+                                           ("11011011", 32), ("11110111", 31), ("1" * 8, 7), ("1" * 8, 8),
+                                           ("1" * 9, 1), ("1" * 9, 2), ("1" * 10, 1)])
+def test_tables_around_the_fewest_partitions(gxy, ctx, orc, pattern, views):
+    # 128 partitions of 4,096 buckets in all: from there on by partition, below by bucket.
+    bases = rand_ascii(np.random.default_rng(views), 400 * views + 3000, b"ACGTACGTACGTN")
+    seq = gxy.DeviceSeq.from_ascii(bases, ctx)
+    ranges = [(400 * k, 400 * k + 700 + 3 * (k % 50)) for k in range(views)]
+    for (lo, hi), tab in zip(ranges, gxy.PosTable.build_views(seq, ranges, pattern, 1)):
+        starts, positions = tab.arrays()
+        want = orc.Table(orc.pack_ascii(bases[lo:hi]), pattern, 1)
+        assert np.array_equal(starts, want.starts()) and np.array_equal(positions, want.positions())
