@@ -69,3 +69,51 @@ def test_tables_around_the_fewest_partitions(gxy, ctx, orc, pattern, views):
         starts, positions = tab.arrays()
         want = orc.Table(orc.pack_ascii(bases[lo:hi]), pattern, 1)
         assert np.array_equal(starts, want.starts()) and np.array_equal(positions, want.positions())
+
+
+def test_enumeration_of_a_run_of_one_base(gxy, ctx):
+    # Five runs of 60 A against 3,000 of them in 10 Mbp: 29 M hits, most of them in
+    # buckets of 126,000 positions that one warp copies.  The exact screen of all these
+    # hits takes 2.1 ms, their enumeration 7 (15 with a loop the compiler unrolled, 35
+    # with one read at a time).
+    rng = np.random.default_rng(5)
+
+    def runs(n, k):
+        s = np.frombuffer(rand_ascii(rng, n, b"ACGT"), np.uint8).copy()
+        for p in rng.integers(0, n - 60, k):
+            s[p:p + 60] = ord("A")
+        return gxy.DeviceSeq.from_ascii(s.tobytes(), ctx)
+    t, q = runs(10_000_000, 3000), runs(30_000, 5)
+    tab = gxy.PosTable.build_view(t, 0, len(t), P12, 1)
+    ratios = []
+    for _ in range(5):
+        st = {}
+        gxy.search_device(tab, q, gxy.ScoringMatrix.hoxd70(), gxy.SearchParams(), stats=st)
+        ratios.append(st["enum_ms"] / st["screen_ms"])
+    assert st["raw_hits"] > 10_000_000 and min(ratios) < 5, ratios
+
+
+@pytest.mark.parametrize("masks", [False, True])
+@pytest.mark.parametrize("transitions", [0, 1, 2])
+@pytest.mark.parametrize("units", [1, 2])
+def test_buckets_around_the_copy_of_large_ones(gxy, ctx, orc, masks, transitions, units):
+    # One window of 19 A against runs of A whose bucket has so many positions (six
+    # reads of 32 at a time, the rest singly).
+    rng = np.random.default_rng(40)
+    m, sp = gxy.ScoringMatrix.hoxd70(), gxy.SearchParams(transitions=transitions)
+    q = rand_ascii(rng, 300, b"CT") + b"A" * 19 + rand_ascii(rng, 300, b"CT")
+    pad = rand_ascii(rng, 550_000 if masks else 500, b"ACGT")
+    for size in (16, 17, 18, 33, 192, 193, 194, 384, 385, 386, 500):
+        t = rand_ascii(rng, 200, b"CT") + b"A" * (size + 18) + pad
+        tab = gxy.PosTable.build(gxy.PackedSeq.from_ascii(t), P12, 1, ctx=ctx)
+        dq = gxy.DeviceSeq.from_ascii(q, ctx)
+        st = {}
+        got = gxy.batch_search([tab], [dq], [(0, 0, s) for s in range(units)], m, sp, stats=st, ctx=ctx)
+        T, Q = orc.pack_ascii(t), orc.pack_ascii(q)
+        raw = 0
+        for s in range(units):
+            strand = Q if s == 0 else orc.reverse_complement(Q)
+            want, ost = orc.search(orc.Table(T, P12, 1), T, strand, orc.params(transitions=transitions))
+            assert got[s].tobytes() == want.tobytes(), (size, s)
+            raw += ost["raw_hits"]
+        assert st["raw_hits"] == raw, size
