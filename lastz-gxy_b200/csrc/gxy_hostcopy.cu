@@ -133,15 +133,15 @@ void host_copy_warm(gxy_ctx* ctx, uint64_t bytes) {
 cudaError_t host_copy(gxy_ctx* ctx, const CopyPiece* pieces, int n, bool to_host, cudaStream_t st,
                       const std::function<void(size_t, size_t)>& seen) {
     size_t total = 0;
-    bool staged = true;
-    for (int i = 0; i < n; i++) {
-        total += pieces[i].bytes;
-        staged = staged && (!pieces[i].bytes || pageable(pieces[i].host));
-    }
-    const int threads = (int)std::min<size_t>({(size_t)kCopyThreads, std::max<size_t>(1, std::thread::hardware_concurrency()),
-                                         total >> 19});
+    for (int i = 0; i < n; i++) total += pieces[i].bytes;
+    // (Only for copies of a size: asking what the memory and the host are takes 3 us.)
+    int threads = 0;
     std::unique_lock<std::mutex> hold(ctx->copy.mu, std::defer_lock);
-    if (total < kStagedFrom || threads < 2 || !staged || !hold.try_lock() || prepare(ctx->copy, ctx->device) != cudaSuccess) {
+    if (total >= kStagedFrom &&
+        std::all_of(pieces, pieces + n, [](const CopyPiece& p) { return !p.bytes || pageable(p.host); }))
+        threads = (int)std::min<size_t>({(size_t)kCopyThreads, std::max<size_t>(1, std::thread::hardware_concurrency()),
+                                         total >> 19});
+    if (threads < 2 || !hold.try_lock() || prepare(ctx->copy, ctx->device) != cudaSuccess) {
         for (int i = 0; i < n; i++) {
             if (!pieces[i].bytes) continue;
             const cudaError_t e = to_host ? cudaMemcpyAsync(pieces[i].host, pieces[i].dev, pieces[i].bytes, cudaMemcpyDeviceToHost, st)
