@@ -130,48 +130,20 @@ void host_copy_warm(gxy_ctx* ctx, uint64_t bytes) {
     prepare(ctx->copy, ctx->device);   // (without it copies take the driver's path)
 }
 
-cudaError_t host_copy(gxy_ctx* ctx, const CopyPiece* pieces, int n, bool to_host, cudaStream_t st,
-                      const std::function<void(size_t, size_t)>& seen) {
-    size_t total = 0;
-    for (int i = 0; i < n; i++) total += pieces[i].bytes;
-    // (Only for copies of a size: asking what the memory and the host are takes 3 us.)
-    int threads = 0;
-    std::unique_lock<std::mutex> hold(ctx->copy.mu, std::defer_lock);
-    if (total >= kStagedFrom &&
-        std::all_of(pieces, pieces + n, [](const CopyPiece& p) { return !p.bytes || pageable(p.host); }))
-        threads = (int)std::min<size_t>({(size_t)kCopyThreads, std::max<size_t>(1, std::thread::hardware_concurrency()),
-                                         total >> 19});
-    if (threads < 2 || !hold.try_lock() || prepare(ctx->copy, ctx->device) != cudaSuccess) {
-        for (int i = 0; i < n; i++) {
-            if (!pieces[i].bytes) continue;
-            const cudaError_t e = to_host ? cudaMemcpyAsync(pieces[i].host, pieces[i].dev, pieces[i].bytes, cudaMemcpyDeviceToHost, st)
-                                          : cudaMemcpyAsync(pieces[i].dev, pieces[i].host, pieces[i].bytes, cudaMemcpyHostToDevice, st);
-            if (e != cudaSuccess) return e;
-            if (seen) seen(0, pieces[i].bytes);
-        }
-        return to_host ? cudaStreamSynchronize(st) : cudaSuccess;
-    }
-    // What st holds (the allocation, what fills it) comes first.
-    cudaError_t e = cudaStreamSynchronize(st);
-    if (e != cudaSuccess) return e;
-    struct Chunk {
-        int piece;
-        size_t at, bytes, turn;   // turn: its place in its huge page
-    };
-    std::vector<Chunk> chunks;
-    for (int i = 0; i < n; i++) {
-        const size_t into = reinterpret_cast<uintptr_t>(pieces[i].host) % kHugePage;
-        for (size_t o = 0; o < pieces[i].bytes;) {
-            const size_t b = std::min(kChunk - (into + o) % kChunk, pieces[i].bytes - o);
-            chunks.push_back({i, o, b, (into + o) % kHugePage / kChunk});
-            o += b;
-        }
-    }
-    std::stable_sort(chunks.begin(), chunks.end(), [](const Chunk& x, const Chunk& y) { return x.turn < y.turn; });
+namespace {
+
+struct Chunk {
+    int piece;
+    size_t at, bytes, turn;   // turn: its place in its huge page
+};
+
+// Through the pinned halves, by `threads` threads; the caller holds ctx->copy.mu.
+cudaError_t staged_copy(gxy_ctx* ctx, const CopyPiece* pieces, const std::vector<Chunk>& chunks, int threads, bool to_host,
+                        const std::function<void(size_t, size_t)>& seen) {
     std::atomic<size_t> next{0};
     std::atomic<int> failed{0};
     HostCopy& h = ctx->copy;
-    const std::function<void(int)> work = [&](int me) {
+    auto copies = [&](int me) {
         char* half[2] = {h.pinned + 2 * me * kChunk, h.pinned + (2 * me + 1) * kChunk};
         char* dst[2] = {nullptr, nullptr};   // a half that waits to be emptied
         size_t len[2] = {0, 0};
@@ -219,8 +191,52 @@ cudaError_t host_copy(gxy_ctx* ctx, const CopyPiece* pieces, int n, bool to_host
             failed.compare_exchange_strong(none, (int)r);
         }
     };
-    h.run(work, threads);
+    h.run(std::ref(copies), threads);   // (by reference: nothing is allocated)
     return (cudaError_t)failed.load();
+}
+
+}  // namespace
+
+cudaError_t host_copy(gxy_ctx* ctx, const CopyPiece* pieces, int n, bool to_host, cudaStream_t st,
+                      const std::function<void(size_t, size_t)>& seen) {
+    size_t total = 0;
+    for (int i = 0; i < n; i++) total += pieces[i].bytes;
+    // (Only for copies of a size: asking what the memory and the host are takes 3 us.)
+    std::unique_lock<std::mutex> hold(ctx->copy.mu, std::defer_lock);
+    if (total >= kStagedFrom &&
+        std::all_of(pieces, pieces + n, [](const CopyPiece& p) { return !p.bytes || pageable(p.host); })) {
+        const int threads = (int)std::min<size_t>({(size_t)kCopyThreads, std::max<size_t>(1, std::thread::hardware_concurrency()),
+                                                   total >> 19});
+        if (threads >= 2 && hold.try_lock() && prepare(ctx->copy, ctx->device) == cudaSuccess) {
+            std::vector<Chunk> chunks;
+            try {
+                for (int i = 0; i < n; i++) {
+                    const size_t into = reinterpret_cast<uintptr_t>(pieces[i].host) % kHugePage;
+                    for (size_t o = 0; o < pieces[i].bytes;) {
+                        const size_t b = std::min(kChunk - (into + o) % kChunk, pieces[i].bytes - o);
+                        chunks.push_back({i, o, b, (into + o) % kHugePage / kChunk});
+                        o += b;
+                    }
+                }
+                std::stable_sort(chunks.begin(), chunks.end(), [](const Chunk& x, const Chunk& y) { return x.turn < y.turn; });
+            } catch (const std::bad_alloc&) {   // the driver's path needs nothing of the host
+                chunks.clear();
+            }
+            if (!chunks.empty()) {
+                // What st holds (the allocation, what fills it) comes first.
+                const cudaError_t e = cudaStreamSynchronize(st);
+                return e != cudaSuccess ? e : staged_copy(ctx, pieces, chunks, threads, to_host, seen);
+            }
+        }
+    }
+    for (int i = 0; i < n; i++) {
+        if (!pieces[i].bytes) continue;
+        const cudaError_t e = to_host ? cudaMemcpyAsync(pieces[i].host, pieces[i].dev, pieces[i].bytes, cudaMemcpyDeviceToHost, st)
+                                      : cudaMemcpyAsync(pieces[i].dev, pieces[i].host, pieces[i].bytes, cudaMemcpyHostToDevice, st);
+        if (e != cudaSuccess) return e;
+        if (seen) seen(0, pieces[i].bytes);
+    }
+    return to_host ? cudaStreamSynchronize(st) : cudaSuccess;
 }
 
 }  // namespace gxy
