@@ -249,7 +249,7 @@ __global__ void __launch_bounds__(32) k_gapped_sides(const __grid_constant__ Gap
         target_load(0);
         __syncwarp();
         int32_t best = 0, thr = -a.ydrop;    // the best score of the rows so far, their threshold
-        I bi = 0, be = 0;                    // the best's row, the end of that row's chunks
+        I bi = 0;                            // the best's row
         uint32_t flags = 0;
         // The pool block being filled: kRows rows and kRows units of kCols cells at
         // most; blocks of the chain in order, n_blk of them for this side.
@@ -529,10 +529,7 @@ __global__ void __launch_bounds__(32) k_gapped_sides(const __grid_constant__ Gap
             }
             // Only an M can exceed the best: Y stays below an M of its row, X
             // below an M of an earlier one.
-            if (rv > best) {
-                bi = i;
-                be = e_new;
-            }
+            if (rv > best) bi = i;
             best = max(best, rv);
             thr = best - a.ydrop;
             e_prev = e_new;
@@ -662,7 +659,6 @@ __global__ void __launch_bounds__(32) k_gapped_sides(const __grid_constant__ Gap
             }
             blk_rows += (int32_t)(i - i0);
             if (i != i0) e_prev = cb + kCols;
-            if (bi > i0) be = cb + kCols;
 #pragma unroll
             for (int p = 0; p < S / 4; p++) {
                 rH[p * nblk + b] = make_int4(H[4 * p], H[4 * p + 1], H[4 * p + 2], H[4 * p + 3]);
@@ -703,9 +699,11 @@ __global__ void __launch_bounds__(32) k_gapped_sides(const __grid_constant__ Gap
                 if (h_at((int64_t)bi, (int64_t)mt.y + rel, b, b0) == best) at = mt.y + rel;
             bj = (int64_t)__reduce_min_sync(kFull, at);
         } else if (bi) {
-            // A bound that the second pass reserves runs by: the column is in one of its
-            // row's chunks.  (A later row's can all lie to the left of it.)
-            bj = (int64_t)min(m, be);
+            // An estimate: the second pass finds the column, and its host makes room for
+            // the runs of one further right (the last row's cells can all lie to the left
+            // of it).  Kept exactly, the end of the best row's chunks took 1 to 2 % of
+            // every call's time.
+            bj = (int64_t)min(m, e_prev);
         }
         res.score = best;
         res.t_span = (uint32_t)bi;
@@ -723,7 +721,8 @@ __global__ void __launch_bounds__(32) k_gapped_sides(const __grid_constant__ Gap
         //  - else it is Y, in the same way along the row.
         // The first pass walks into its scratch and reserves exactly the runs
         // written; the second pass reserves best_i + best_j words (the longest
-        // possible script) and writes in place.
+        // possible script) and writes in place, if they fit: the counter has the
+        // reservations of all sides in any case.
         int64_t ti = (int64_t)bi, tj = bj;
         int32_t v = best;
         uint32_t op = 3, cnt = 0, nr = 0;
@@ -1226,7 +1225,8 @@ gxy_status gxy_gapped_extend(gxy_ctx* ctx, const gxy_dseq* target, uint64_t t_lo
         std::vector<uint64_t> base(list.size());
         uint64_t k0 = 0;
         unsigned long long c2[kCtrWords] = {};
-        bool first_group = true;
+        uint64_t reserved = 0;   // run words of the groups done
+        bool more_room = false;
         while (e == cudaSuccess && k0 < list.size()) {
             uint64_t k1 = k0, used = 0;
             while (k1 < list.size() && used + need[k1] <= group_blocks) {
@@ -1240,13 +1240,27 @@ gxy_status gxy_gapped_extend(gxy_ctx* ctx, const gxy_dseq* target, uint64_t t_lo
             e = cudaMemcpyAsync(dl + k0, list.data() + k0, (k1 - k0) * 4, cudaMemcpyHostToDevice, st);
             if (e == cudaSuccess)
                 e = cudaMemcpyAsync(dbase + k0, base.data() + k0, (k1 - k0) * 8, cudaMemcpyHostToDevice, st);
-            // The task cursor restarts; the run counter keeps counting across groups.
+            // The task cursor restarts; the run counter goes on from the groups done.
             if (e == cudaSuccess) e = cudaMemsetAsync(B.ctr + kCtrTask, 0, 8, st);
-            if (e == cudaSuccess && first_group) e = cudaMemsetAsync(B.ctr + kCtrRuns, 0, 8, st);
+            if (e == cudaSuccess) e = cudaMemcpyAsync(B.ctr + kCtrRuns, &reserved, 8, cudaMemcpyHostToDevice, st);
             // Rows and cells count this group's sides only.
             if (e == cudaSuccess) e = cudaMemsetAsync(B.ctr + kCtrRows, 0, 16, st);
             if (e == cudaSuccess) e = cudaMemsetAsync(B.ctr + kCtrFlags, 0, 8, st);
             if (e == cudaSuccess) e = launch(B, c2);
+            if (e == cudaSuccess && !(c2[kCtrFlags] & (kFlagPool | kFlagState)) && (c2[kCtrFlags] & kFlagRuns) && !more_room) {
+                // The columns were estimates; now all that this group's sides need is
+                // known.  The groups done keep their runs.
+                uint32_t* bigger = nullptr;
+                B.runs_cap += c2[kCtrRuns] - reserved;
+                e = cudaMallocAsync((void**)&bigger, B.runs_cap * 4, st);
+                if (e == cudaSuccess && reserved) e = cudaMemcpyAsync(bigger, d_runs2, reserved * 4, cudaMemcpyDeviceToDevice, st);
+                if (e == cudaSuccess) std::swap(d_runs2, bigger);
+                if (bigger) cudaFreeAsync(bigger, st);
+                B.runs = d_runs2;
+                more_room = true;
+                pass2_cells += c2[kCtrCells];
+                continue;
+            }
             if (e == cudaSuccess && (c2[kCtrFlags] & (kFlagPool | kFlagRuns | kFlagState))) {
                 cudaFreeAsync(d_pool2, st);
                 cudaFreeAsync(d_runs2, st);
@@ -1256,7 +1270,8 @@ gxy_status gxy_gapped_extend(gxy_ctx* ctx, const gxy_dseq* target, uint64_t t_lo
                 return fail(GXY_ECUDA, "gapped extension: the exactly sized second pass fell short");
             }
             pass2_cells += c2[kCtrCells];
-            first_group = false;
+            reserved = c2[kCtrRuns];
+            more_room = false;
             k0 = k1;
         }
         A.runs2 = d_runs2;

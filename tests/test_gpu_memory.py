@@ -89,3 +89,40 @@ def test_2bit_in_the_memory_that_is_left(room):
     r = subprocess.run([sys.executable, "-c", TWOBIT.format(here=HERE, room=room)], capture_output=True, text=True,
                        timeout=300, env=dict(os.environ, CUDA_MODULE_LOADING="EAGER"))
     assert r.returncode == 0 and r.stdout.strip() == "ok", r.stdout + r.stderr
+
+
+GAPPED = """
+import sys
+sys.path.insert(0, {here!r})
+import conftest, torch, numpy as np
+gxy = sys.modules["lastz_gxy_b200"]
+from test_gpu_gapped import both
+rng = np.random.default_rng(3)
+bases = np.frombuffer(b"ACGT", np.uint8)
+t, q = np.full(1000, ord("N"), np.uint8), np.full(760, ord("N"), np.uint8)
+t[:372] = bases[rng.integers(0, 4, 372)]
+q[:102] = t[270:372]
+seg = t[1:353].copy()
+at = rng.choice(352, 185, replace=False)
+seg[at] = bases[(np.searchsorted(bases, seg[at]) + 2) % 4]
+q[291:643] = seg
+c = gxy.Context(0)
+c.set_tuning(gapped_pool_blocks=8)
+torch.cuda.mem_get_info()
+ballast = torch.empty(torch.cuda.mem_get_info()[0] - (640 << 20), dtype=torch.uint8, device="cuda:0")
+g, w, st = both(gxy, c, t.tobytes(), q.tobytes(), [(0, 0)] * 400, thr=-10 ** 6)
+assert g == w and st["second_pass_sides"] == 400
+# (every side once, and the groups that were short of run words again)
+one = st["cells"] // 400
+print("ok", st["second_pass_cells"] // one)
+"""
+
+
+def test_gapped_second_pass_in_groups_short_of_runs():
+    # 400 sides of the shape of test_gapped_second_pass_best_right_of_the_last_rows, in
+    # groups that fit half of what is left: run words reserved by the last rows' ends
+    # last for the first groups, a later one makes room and runs again.
+    r = subprocess.run([sys.executable, "-c", GAPPED.format(here=HERE)], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, CUDA_MODULE_LOADING="EAGER"))
+    assert r.returncode == 0 and r.stdout.startswith("ok "), r.stdout + r.stderr
+    assert 400 < int(r.stdout.split()[1]) < 800, r.stdout
