@@ -392,7 +392,7 @@ __device__ __forceinline__ void store_hit(const ScreenArgs& a, uint64_t i, uint3
 
 constexpr int kEnumWarps = 8, kEnumBlocks = 4;   // 31 KB of shared memory a block, 35 with a lane a byte
 constexpr uint32_t kWordBits = (1u << 27) - 1;   // of an entry; the lane above
-constexpr uint32_t kBigReads = 6;               // of a lane in a large bucket
+constexpr uint32_t kBigReads = 5;               // of a lane in a large bucket
 
 // kMode 0: the words themselves only; 1: neighbour masks; 2: masks formed from
 // the occupancy bitmap (tables without neighbour masks).
@@ -675,8 +675,9 @@ __global__ __launch_bounds__(kEnumWarps * 32, kEnumBlocks) void k_enumerate(cons
                         }
                         // Several reads on their way at a time: a run of one base (or another
                         // short unit) in the query is one warp's millions of hits (29 M hits of
-                        // runs of A: 7.1 ms; one read at a time 34.5; four 7.1, eight 5.8 but
-                        // with spills that the ordinary tiles pay for).
+                        // runs of A: 7.5 ms, one read at a time 34.5; four 7.1, six 7.1 and
+                        // eight 5.8, but with spills that ordinary tiles pay for, 1 % with six;
+                        // in a function of its own 12 %).
                         const uint32_t* from = U->positions + bb + 1 + lane;
                         uint32_t* to = a.hits + more + lane;
                         uint32_t left = cc - 1;
@@ -755,8 +756,8 @@ void launch_pass_reset(uint32_t* ctl, uint64_t surv_cap, cudaStream_t st) {
 
 void launch_enumerate(const ScreenArgs& a, int sm_count, cudaStream_t st) {
     count_launch();
-    // A warp per item at most: the idle warps of a full grid took 30 us to claim
-    // nothing on a 30 kbp query (938 tiles).
+    // A warp per item at most (those that claim first take several): the idle warps
+    // of a full grid took 30 us to claim nothing on a 30 kbp query (938 tiles).
     const int blocks = (int)std::max<uint64_t>(1, umin64(((uint64_t)a.n_items + kEnumWarps - 1) / kEnumWarps, (uint64_t)sm_count * kEnumBlocks));
     if (a.enum_mode == 0) k_enumerate<0><<<blocks, kEnumWarps * 32, 0, st>>>(a);
     else if (a.enum_mode == 1) k_enumerate<1><<<blocks, kEnumWarps * 32, 0, st>>>(a);
