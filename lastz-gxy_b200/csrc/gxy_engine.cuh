@@ -89,8 +89,7 @@ struct UnitPlan {
 
 // Candidate arrays are sized up front at one candidate per this many
 // estimated raw hits (the estimate carries a 1.5x margin; about 3 % of raw
-// hits become candidates), up to a bound.  Larger arrays also widen the
-// capacity-sized sort and scan grids of every later launch on the worker.
+// hits become candidates), up to a bound.
 constexpr uint64_t kHitsPerCandidate = 32;
 // With the upper-bound filter the hit buffer is sized at one slot per this
 // many estimated raw hits (survivors are a few percent of the raw hits).

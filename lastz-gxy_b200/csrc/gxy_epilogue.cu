@@ -4,11 +4,11 @@
 //
 // The element counts are only known on the device (the screen's candidates,
 // the walk's HSPs) and range from a handful to tens of millions.  Both kernels
-// are cooperative launches that use as many of their blocks as the count
-// needs -- one, without any grid barrier, up to a tile -- so a small search
-// pays for neither the empty launches (a three-kernel pass per digit took 60 us
-// for a few hundred candidates) nor grids sized by capacity, and a large one
-// crosses the device a few times per digit.
+// are cooperative launches of a block an SM that use as many of their blocks as
+// the count needs -- one, without any grid barrier, up to 512 candidates (the
+// sort) or a tile of 4,096 (the finish) -- so a small search does not pay for
+// empty launches (a three-kernel pass per digit took 60 us for a few hundred
+// candidates), and a large one crosses the device a few times per digit.
 //
 // What bounds them: barriers and launch latency for small counts; for large
 // ones the scatter's read and write of 12 B an item and digit.

@@ -422,7 +422,8 @@ __global__ void k_neighbours(const uint32_t* __restrict__ occ, uint64_t n_words,
                 else r[v] = __ldg(occ + view + (x ^ (1u << (bit - 5))));
             }
         }
-        // Both 16 x 16 halves at once.
+        // Both 16 x 16 halves at once, by the recursive block swap of Warren, Hacker's
+        // Delight, section 7-3.
         uint32_t m = 0x00ff00ffu;
 #pragma unroll
         for (int j = 8; j; j >>= 1, m ^= m << j) {
